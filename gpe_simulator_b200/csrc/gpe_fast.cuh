@@ -373,6 +373,74 @@ __device__ __forceinline__ float expm1_series(float x) {
   }
 }
 
+// complex128: the same factors in FP64, as f - 1 applied by v + v*(f - 1).  Taylor
+// series on |x| <= 1/2: sin to x^15 (first omitted term x^17/17! < 3e-20 of x), cos - 1
+// to x^16 (x^18/18! < 7e-22), exp - 1 to x^15 (x^16/16! < 8e-19); library functions,
+// out of line, beyond.  Steps in use keep V dt/2 far inside the range; with the library
+// sincos and exp inlined per half-step, and two of them per fused z sweep, that sweep was
+// bound by FP64 issue.  Box and absorber at 256^3, 4 steps: 3260 -> 2634 us together with
+// the single rotation of the fused sweep (half_all).
+static __device__ __noinline__ void sin_cosm1_far(double x, double* s, double* cm1) {
+  double sh, ch;
+  sincos(0.5 * x, &sh, &ch);
+  *cm1 = -2.0 * sh * sh;
+  *s = 2.0 * sh * ch;
+}
+static __device__ __noinline__ double exp_far(double x) { return exp(x); }
+__device__ __forceinline__ void sin_cosm1_d(double x, double& s, double& cm1) {
+  if (fabs(x) <= 0.5) {
+    const double z = x * x;
+    double a = -1.0 / 1307674368000.0, b = 1.0 / 20922789888000.0;
+    a = fma(a, z, 1.0 / 6227020800.0);
+    b = fma(b, z, -1.0 / 87178291200.0);
+    a = fma(a, z, -1.0 / 39916800.0);
+    b = fma(b, z, 1.0 / 479001600.0);
+    a = fma(a, z, 1.0 / 362880.0);
+    b = fma(b, z, -1.0 / 3628800.0);
+    a = fma(a, z, -1.0 / 5040.0);
+    b = fma(b, z, 1.0 / 40320.0);
+    a = fma(a, z, 1.0 / 120.0);
+    b = fma(b, z, -1.0 / 720.0);
+    a = fma(a, z, -1.0 / 6.0);
+    b = fma(b, z, 1.0 / 24.0);
+    b = fma(b, z, -0.5);
+    s = fma(a * z, x, x);
+    cm1 = b * z;
+  } else {
+    sin_cosm1_far(x, &s, &cm1);
+  }
+}
+// v * exp(x): v + v*(exp(x) - 1) in the series' range, the product with exp itself beyond
+// (where exp - 1 would lose the relative accuracy of a small factor).
+__device__ __forceinline__ double2 mul_exp_d(double2 v, double x) {
+  if (fabs(x) <= 0.5) {
+    double a = 1.0 / 1307674368000.0;
+    a = fma(a, x, 1.0 / 87178291200.0);
+    a = fma(a, x, 1.0 / 6227020800.0);
+    a = fma(a, x, 1.0 / 479001600.0);
+    a = fma(a, x, 1.0 / 39916800.0);
+    a = fma(a, x, 1.0 / 3628800.0);
+    a = fma(a, x, 1.0 / 362880.0);
+    a = fma(a, x, 1.0 / 40320.0);
+    a = fma(a, x, 1.0 / 5040.0);
+    a = fma(a, x, 1.0 / 720.0);
+    a = fma(a, x, 1.0 / 120.0);
+    a = fma(a, x, 1.0 / 24.0);
+    a = fma(a, x, 1.0 / 6.0);
+    a = fma(a, x, 0.5);
+    a = fma(a * x, x, x);
+    return make_double2(fma(v.x, a, v.x), fma(v.y, a, v.y));
+  }
+  const double f = exp_far(x);
+  return make_double2(v.x * f, v.y * f);
+}
+// v * exp(-i x)
+__device__ __forceinline__ double2 rotate_d(double2 v, double x) {
+  double sn, cm1;
+  sin_cosm1_d(x, sn, cm1);
+  return make_double2(fma(v.x, cm1, fma(v.y, sn, v.x)), fma(v.y, cm1, fma(-v.x, sn, v.y)));
+}
+
 // Per-tile tables in shared memory.
 template <typename R>
 struct FastTables {
@@ -387,7 +455,7 @@ struct FastTables {
 };
 
 // two: the tables of the fused z sweep (c2, c12 at the second half-step's time).
-// pre (real time, two half-steps as one rotation, no potential arrays): vz and
+// pre (real time, two half-steps as one rotation): vz and
 // c12 are stored already multiplied by dt (vz by dt, c12 by dt/2), so that the
 // phase (2 vz + c12 + 2 beta |psi|^2) dt/2 is one add and one fma per point.
 template <int N, typename R>
@@ -482,6 +550,15 @@ __device__ __forceinline__ void kin_all(typename Cx<R>::T (&v)[EPT], const Phys&
   }
 }
 
+// (1 + exp(2 g))/2: the mean density factor of two consecutive half-steps with gain or
+// loss g each (1 without an absorber)
+template <bool ARR> __device__ __forceinline__ float two_density(float g) {
+  return ARR ? (g == 0.0f ? 1.0f : fmaf(0.5f, expm1f(g + g), 1.0f)) : 1.0f;
+}
+template <bool ARR> __device__ __forceinline__ double two_density(double g) {
+  return ARR ? (g == 0.0 ? 1.0 : 0.5 + 0.5 * exp_far(g + g)) : 1.0;
+}
+
 // One local half-step over all registers (layout LANES x VALS, element m = lane +
 // LANES*a, Z tiles: m = z index), potential vz[m] + ctab[l] (+ arrays).  complex64:
 // each element whose phase is within the short series' range (|phase| <= 1/8,
@@ -492,7 +569,10 @@ __device__ __forceinline__ void kin_all(typename Cx<R>::T (&v)[EPT], const Phys&
 // keeps the fused sweeps within their register budget.
 // TWO: two consecutive real-time half-steps at one point as one rotation by
 // (2 vz[m] + ctab[l] + 2 beta |psi|^2) dt/2 with ctab = c1 + c2; exact because
-// the first rotation leaves |psi| unchanged.  The tables come prescaled (vz[m]
+// the first rotation leaves |psi| unchanged.  With an absorber the first half-step
+// leaves |psi|^2 exp(2 g), g = Im V dt/2, so the density term is
+// beta |psi|^2 (1 + exp(2 g)) dt/2 and the amplitude exp(2 g): still one rotation, the
+// array potentials read once.  The tables come prescaled (vz[m]
 // by dt, ctab by dt/2, see z_tables) and callers pass beta as 2 beta dt/2.
 template <int N, int AX, typename R, int LANES, int VALS, int SLOTS, int EPT, bool REAL, bool ARR,
           bool TWO = false>
@@ -517,20 +597,20 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
       R V = tb.vz[m] + c;
       R g = (R)0;
       if (ARR) {
-        V += ph.vre ? ((const R*)ph.vre)[row + m] : (R)0;
+        const R va = ph.vre ? ((const R*)ph.vre)[row + m] : (R)0;
+        V = TWO ? fma(va, h + h, V) : V + va;
         g = ph.vim ? ((const R*)ph.vim)[row + m] * h : (R)0;
       }
       const typename Cx<R>::T x = v[e];
-      const R phs = TWO ? fma(beta, x.x * x.x + x.y * x.y, V) : (V + beta * (x.x * x.x + x.y * x.y)) * h;
-      if (sizeof(R) == 8) {
+      const R phs = TWO ? fma(beta * two_density<ARR>(g), x.x * x.x + x.y * x.y, V)
+                        : (V + beta * (x.x * x.x + x.y * x.y)) * h;
+      if constexpr (sizeof(R) == 8) {
         if (!REAL) {
-          const double f = exp(-(double)phs);
-          v[e] = mk((R)(x.x * f), (R)(x.y * f));
+          v[e] = mul_exp_d(x, -phs);
         } else {
-          double sd, cd;
-          sincos((double)phs, &sd, &cd);
-          if (ARR) { const double am = exp((double)g); sd *= am; cd *= am; }
-          v[e] = mk((R)(x.x * cd + x.y * sd), (R)(x.y * cd - x.x * sd));
+          v[e] = rotate_d(x, phs);
+          // (g is zero away from the absorbers: whole warps skip its exponential)
+          if (ARR) { if (g != 0.0) v[e] = mul_exp_d(v[e], TWO ? 2.0 * g : g); }
         }
       } else if (fabs(phs) <= (R)0.125) {
         if (!REAL) {
@@ -539,7 +619,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
         } else {
           float sn, cm1;
           sin_cosm1_tiny((float)phs, sn, cm1);
-          if (ARR) { const float am = expm1f((float)g); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
+          if (ARR) { const float am = expm1f((float)(TWO ? g + g : g)); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
           v[e] = mk(fma(x.x, (R)cm1, fma(x.y, (R)sn, x.x)), fma(x.y, (R)cm1, fma(-x.x, (R)sn, x.y)));
         }
       } else {
@@ -564,11 +644,13 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
       R V = tb.vz[m] + c;
       R g = (R)0;
       if (ARR) {
-        V += ph.vre ? ((const R*)ph.vre)[row + m] : (R)0;
+        const R va = ph.vre ? ((const R*)ph.vre)[row + m] : (R)0;
+        V = TWO ? fma(va, h + h, V) : V + va;
         g = ph.vim ? ((const R*)ph.vim)[row + m] * h : (R)0;
       }
       const typename Cx<R>::T x = v[e];
-      const float p = (float)(TWO ? fma(beta, x.x * x.x + x.y * x.y, V) : (V + beta * (x.x * x.x + x.y * x.y)) * h);
+      const float p = (float)(TWO ? fma(beta * two_density<ARR>(g), x.x * x.x + x.y * x.y, V)
+                                  : (V + beta * (x.x * x.x + x.y * x.y)) * h);
       if (!REAL) {
         const float em = fabsf(p) <= 0.5f ? expm1_series(-p) : expm1f(-p);
         v[e] = mk(fma(x.x, (R)em, x.x), fma(x.y, (R)em, x.y));
@@ -581,7 +663,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
           sincosf(0.5f * p, &sh, &ch);
           cm1 = -2.0f * sh * sh; sn = 2.0f * sh * ch;
         }
-        if (ARR) { const float am = expm1f((float)g); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
+        if (ARR) { const float am = expm1f((float)(TWO ? g + g : g)); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
         v[e] = mk(fma(x.x, (R)cm1, fma(x.y, (R)sn, x.x)), fma(x.y, (R)cm1, fma(-x.x, (R)sn, x.y)));
       }
     }
@@ -689,7 +771,10 @@ __device__ __forceinline__ void fast_pointwise(typename Cx<R>::T (&v)[EPT], cons
     if (op.scale) {
       if (sizeof(R) == 8) {
 #pragma unroll
-        for (int e = 0; e < EPT; ++e) { v[e].x = (R)((double)v[e].x / cx.sc_div); v[e].y = (R)((double)v[e].y / cx.sc_div); }
+        for (int e = 0; e < EPT; ++e) {
+          v[e].x = (R)div_by((double)v[e].x, cx.sc_div, cx.sc_rcp);
+          v[e].y = (R)div_by((double)v[e].y, cx.sc_div, cx.sc_rcp);
+        }
       } else {
         scale_all(v, cx.sc_mul);
       }
@@ -698,14 +783,16 @@ __device__ __forceinline__ void fast_pointwise(typename Cx<R>::T (&v)[EPT], cons
     return;
   }
   // (1/M was applied with the kinetic factor in the x sweep)
-  if (MODE == FM_Z21 && ph.kind == 1 && ph.vre == nullptr && ph.vim == nullptr) {
-    // real time, potential from tables: the two half-steps as one rotation
-    const R h = (R)(ph.dt * 0.5);
-    half_all<N, AX, R, LANES, VALS, SLOTS, EPT, true, false, true>(v, tl, ph, tb, tb.c12, (R)(2.0 * ph.beta) * h, h);
+  if (MODE == FM_Z21) {
+    // (real time only) the two half-steps as one rotation
+    const R h = (R)(ph.dt * 0.5), b2 = (R)(2.0 * ph.beta) * h;
+    if (ph.vre == nullptr && ph.vim == nullptr)
+      half_all<N, AX, R, LANES, VALS, SLOTS, EPT, true, false, true>(v, tl, ph, tb, tb.c12, b2, h);
+    else
+      half_all<N, AX, R, LANES, VALS, SLOTS, EPT, true, true, true>(v, tl, ph, tb, tb.c12, b2, h);
     return;
   }
   half_dispatch<N, AX, R, LANES, VALS, SLOTS, EPT>(v, tl, ph, tb, tb.c1);
-  if (MODE == FM_Z21) half_dispatch<N, AX, R, LANES, VALS, SLOTS, EPT>(v, tl, ph, tb, tb.c2);
   if (MODE == FM_Z2 && op.norm) {
     // a thread's few values summed in plain FP64 (fixed order), the thread sums
     // then combined with compensation across the block and the grid
@@ -840,8 +927,7 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
       }
     }
     if (ZM || (MODE == FM_DIAGR && ph.ltab))
-      z_tables<N, R>(ph, sw, tl.a0, tb, MODE == FM_Z21,
-                     MODE == FM_Z21 && ph.kind == 1 && ph.vre == nullptr && ph.vim == nullptr);
+      z_tables<N, R>(ph, sw, tl.a0, tb, MODE == FM_Z21, MODE == FM_Z21);
     if (MODE == FM_XKIN) x_tables<N, R>(ph, tl.a0, tl.b0, tb);
     // diagnostic x sweep: the shell histogram takes the tables region
     if (MODE == FM_DIAGK && sw.hist)
@@ -857,7 +943,8 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
   cx.sc_mul = (R)1;
   if (MODE == FM_Z1 && op.scale) {
     cx.sc_div = __ldcg(sw.scale);
-    cx.sc_mul = (R)__ldcg(sw.scale + 1);
+    cx.sc_rcp = __ldcg(sw.scale + 1);
+    cx.sc_mul = (R)cx.sc_rcp;
   }
   if (MODE == FM_DIAGR) {
     cx.t1 = sw.t1;

@@ -99,6 +99,18 @@ struct LineSlots {
 };
 
 // ---------------------------------------------------------------- helpers
+// a / d for d's correctly rounded reciprocal r: one Newton correction of a*r by its exact
+// remainder gives the correctly rounded quotient (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990) in three operations instead of
+// a division per component.  A reciprocal that is zero or not finite (a norm that is
+// not) takes the division itself, which then gives what it always gave.
+static __device__ __noinline__ double div_far(double a, double d) { return a / d; }
+__device__ __forceinline__ double div_by(double a, double d, double r) {
+  if (!(fabs(r) > 0.0 && fabs(r) <= 1.7976931348623157e308)) return div_far(a, d);
+  const double q = a * r;
+  return fma(fma(-q, d, a), r, q);
+}
+
 __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
   s = a + b;
   double bb = s - a;
@@ -351,7 +363,7 @@ struct PwCtx {
   double t1, t2;
   double b1x, b1y, b2x, b2y;  // beam centres at t1, t2
   R sc_mul;                   // 1/sqrt(N) (float path)
-  double sc_div;              // sqrt(N) (double path)
+  double sc_div, sc_rcp;      // sqrt(N) and its rounded reciprocal (double path)
   Acc acc[4];                 // norm / diag accumulators
   double* hist;               // shared-memory shell histogram (PW_DIAG_K)
   int nbins;

@@ -376,9 +376,9 @@ __device__ __forceinline__ void scale_state(typename Cx<R>::T* psi, long long co
 #pragma unroll
     for (int q = 0; q < 4; ++q) { v[q].x *= f; v[q].y *= f; }
   } else {
-    const double d = __ldcg(scale);
+    const double d = __ldcg(scale), r = __ldcg(scale + 1);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) { v[q].x = (R)((double)v[q].x / d); v[q].y = (R)((double)v[q].y / d); }
+    for (int q = 0; q < 4; ++q) { v[q].x = (R)div_by((double)v[q].x, d, r); v[q].y = (R)div_by((double)v[q].y, d, r); }
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
