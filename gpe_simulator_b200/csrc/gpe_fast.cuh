@@ -86,6 +86,9 @@ struct FastOps {
   int invm;         // FM_PLAIN: multiply by 1/M
   int scale;        // FM_Z1: apply the pending renormalisation
   int norm;         // FM_Z2: norm partials and renormalisation scale
+  int tr;           // host: 0 step, 1 transform or reduction (radices of the Stockham passes in
+                    // complex64, whose rounding such results keep), 2 the same on the
+                    // run-time-length sweeps whatever the side
   int pdl;          // host: launch as a programmatic dependent of the previous sweep
   int pf;           // tiles ahead whose lines a block prefetches into L2 (0 = none): the
                     // tile the block that follows it on the SM will process

@@ -271,14 +271,14 @@ template <int B, int E> struct SFor {
 };
 
 // R = R1*R2 from two smaller DFTs with compile-time twiddles W_R^(n2 k1).
-template <int R1, int R2> struct DftSplitG {
+template <int R1, int R2, typename D1 = Dft<R1>, typename D2 = Dft<R2>> struct DftSplitG {
   template <typename C> __device__ __forceinline__ static void run(C* v, const C* tw, const C* twl, int unused) {
     C y[R2][R1];
     SFor<0, R2>::run([&](auto n2c) {
       constexpr int n2 = decltype(n2c)::value;
 #pragma unroll
       for (int n1 = 0; n1 < R1; ++n1) y[n2][n1] = v[R2 * n1 + n2];
-      Dft<R1>::run(y[n2], tw, twl, unused);
+      D1::run(y[n2], tw, twl, unused);
       SFor<1, R1>::run([&](auto k1c) {
         constexpr int k1 = decltype(k1c)::value;
         y[n2][k1] = mul_root<R1 * R2, n2 * k1>(y[n2][k1]);
@@ -289,7 +289,7 @@ template <int R1, int R2> struct DftSplitG {
       C z[R2];
 #pragma unroll
       for (int n2 = 0; n2 < R2; ++n2) z[n2] = y[n2][k1];
-      Dft<R2>::run(z, tw, twl, unused);
+      D2::run(z, tw, twl, unused);
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) v[k1 + R1 * k2] = z[k2];
     }
@@ -303,8 +303,47 @@ template <> struct Dft<10> : DftSplitG<5, 2> {};
 template <> struct Dft<12> : DftSplitG<4, 3> {};
 template <> struct Dft<32> : DftSplitG<4, 8> {};
 
-// Generic odd prime radix (7, 11, 13): direct O(R^2) DFT, W_R^e read from the
-// length-n twiddle table (tw[j] = W_n^j) at stride n/R.
+// Odd prime radix: sums and differences of the conjugate pairs, v[j] +- v[R-j], against
+// cosines and sines (compile-time constants, split hi + lo for complex64):
+//   X[k], X[R-k] = v[0] + sum_j a_j cos(2 pi j k/R) -+ i sum_j b_j sin(2 pi j k/R)
+template <int R> struct DftPrime {
+  template <typename C> __device__ __forceinline__ static void run(C* v, const C*, const C*, int) {
+    using Rl = decltype(v[0].x);
+    constexpr int H = (R - 1) / 2;
+    C a[H + 1], b[H + 1];
+    const C x0 = v[0];
+    C sum = x0;
+#pragma unroll
+    for (int j = 1; j <= H; ++j) {
+      a[j] = cadd(v[j], v[R - j]);
+      b[j] = csub(v[j], v[R - j]);
+      sum = cadd(sum, a[j]);
+    }
+    v[0] = sum;
+    SFor<1, H + 1>::run([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      C p = x0, q = mk(Rl(0), Rl(0)), pl = mk(Rl(0), Rl(0)), ql = mk(Rl(0), Rl(0));
+      SFor<1, H + 1>::run([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        constexpr CxCS w = cx_root((j * k) % R, R);
+        constexpr Rl c = (Rl)w.c, s = (Rl)w.s;
+        p = mk(fma(a[j].x, c, p.x), fma(a[j].y, c, p.y));
+        q = mk(fma(b[j].x, s, q.x), fma(b[j].y, s, q.y));
+        if constexpr (sizeof(Rl) == 4) {
+          constexpr Rl cl = (Rl)(w.c - (double)c), sl = (Rl)(w.s - (double)s);
+          pl = mk(fma(a[j].x, cl, pl.x), fma(a[j].y, cl, pl.y));
+          ql = mk(fma(b[j].x, sl, ql.x), fma(b[j].y, sl, ql.y));
+        }
+      });
+      if constexpr (sizeof(Rl) == 4) { p = cadd(p, pl); q = cadd(q, ql); }
+      q = cmi(q);
+      v[k] = cadd(p, q);
+      v[R - k] = csub(p, q);
+    });
+  }
+};
+// Generic odd prime radix (7, 11, 13) of the Stockham passes: direct O(R^2) DFT, W_R^e
+// read from the length-n twiddle table (tw[j] = W_n^j) at stride n/R.
 template <int R> struct DftDirect {
   template <typename C> __device__ __forceinline__ static void run(C* v, const C* tw, const C* twl, int n_over_r) {
     C w[R], wl[R];
@@ -325,6 +364,8 @@ template <int R> struct DftDirect {
 template <> struct Dft<7>  : DftDirect<7> {};
 template <> struct Dft<11> : DftDirect<11> {};
 template <> struct Dft<13> : DftDirect<13> {};
+template <> struct Dft<9>  : DftSplitG<3, 3> {};
+template <> struct Dft<15> : DftSplitG<5, 3> {};
 
 // ---------------------------------------------------------------- one pass
 template <int R, int EPT, typename C>

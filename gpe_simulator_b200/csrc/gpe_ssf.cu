@@ -3,6 +3,7 @@
 #include "../../include/gpe_ssf.h"
 #include "gpe_sweep.h"
 #include "gpe_fast.cuh"
+#include "gpe_line.cuh"
 
 namespace gpe {
 cudaError_t launch_fast_tma(int n, int ax, const Phys& ph, const Sweep& sw, const FastOps& op,
@@ -554,7 +555,13 @@ struct gpe_plan {
   Phys ph{};
   int lt_z = 1, lt_yx = 16;
   bool gen = false;                // grid size needs the odd-prime radices 7/11/13
-  bool fast = false;               // register-resident sweeps exist for this n
+  bool fast = false;               // register-resident sweeps (of this side, or with the side at run time)
+  bool line = false;               // run-time-length sweeps exist for this n: two radices or more
+  bool fixed = false;              // sweeps compiled for this side exist
+  // their geometry, tiles and tables: [0] steps, [1] transforms and reductions (complex64:
+  // the radices of the Stockham passes, so that these results keep their rounding)
+  struct LineSet { LineGeo geo{}; LineShape z{}, p{}; bool ok = false; void* d_tw = nullptr; void* d_bf = nullptr; };
+  LineSet ls[2];
   bool plane = false;              // y and z sweeps fused per x-plane (opt-in; complex64, n = 128, 256)
   bool tma = false;                // plain y/x sweeps stage their pencils by TMA (opt-in; complex64, n = 128, 256)
   // tensor maps of recently swept arrays: base address -> maps of y and x tiles
@@ -804,9 +811,16 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   o.pdl = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
   p->pdl_prev = p->pdl_chain;
   const CUtensorMap* map = p->tma && o.mode == FM_PLAIN && fax != FZ ? tma_maps(p, sw.src, fax) : nullptr;
-  const cudaError_t e = map ? launch_fast_tma(p->n, fax, p->ph, sw, o, *map, st)
-                        : p->dtype == GPE_C64 ? launch_fast<float>(p->n, fax, p->ph, sw, o, st)
-                                              : launch_fast<double>(p->n, fax, p->ph, sw, o, st);
+  const bool line = !p->fixed || o.mode == FM_LZ;
+  const gpe_plan::LineSet& ls = p->ls[o.tr];
+  const LineShape& shape = fax == FZ ? ls.z : ls.p;
+  const size_t smem = line ? line_smem(ls.geo, shape, (int)p->csize, fax == FZ, sw.hist ? sw.nbins : 0) : 0;
+  const cudaError_t e =
+      line ? (p->dtype == GPE_C64 ? launch_line<float>(fax, p->ph, sw, o, ls.geo, shape, smem, st)
+                                  : launch_line<double>(fax, p->ph, sw, o, ls.geo, shape, smem, st))
+      : map ? launch_fast_tma(p->n, fax, p->ph, sw, o, *map, st)
+      : p->dtype == GPE_C64 ? launch_fast<float>(p->n, fax, p->ph, sw, o, st)
+                            : launch_fast<double>(p->n, fax, p->ph, sw, o, st);
   if (e != cudaSuccess) return fail(GPE_ERR_CUDA, std::string("fast sweep: ") + cudaGetErrorString(e));
   ++p->launches;
   if (p->prof) {
@@ -861,7 +875,14 @@ int psweep(gpe_plan* p, void* psi, int mz, const FastOps* ops, int nstage, int z
 
 FastOps mk_ops(int mode, int inv1 = 0, int invm = 0, int scale = 0, int norm = 0) {
   FastOps o;
-  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.pdl = 0; o.pf = 0;
+  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.pf = 0;
+  return o;
+}
+
+// the same for a sweep of a transform or reduction
+FastOps tr_ops(int mode, int inv1 = 0, int invm = 0) {
+  FastOps o = mk_ops(mode, inv1, invm);
+  o.tr = 1;
   return o;
 }
 
@@ -954,15 +975,31 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
   for (int q = 0; q < p->pp.npass; ++q)
     if (p->pp.radix[q] > 5 && p->pp.radix[q] != 8 && p->pp.radix[q] != 16) p->gen = true;
   p->ept = p->gen ? 8 : 16;
-  // register-resident sweeps: n = 32, 48, 64, 96, 128, 160, 256; potentials from tables (no per-point program)
+  // register-resident sweeps: compiled for n = 32, 48, 64, 96, 128, 160, 256 (512 in complex64), with the
+  // side at run time for every other n of two radices or more; potentials from tables (no per-point program)
   // (complex64 plans that evaluate the local factor in FP64 use the generic sweeps,
   // which carry that variant; keeping it out of the register-resident kernels keeps
   // their register budget)
   // a dynamic potential stays on them when none of its terms depends on z (line form)
   const bool line_ok = d->dynamic_g_len == 0 || dynamic_line_form(p->prog_dyn, p->prog_line, p->slot_progs);
-  p->fast = (n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 160 || n == 256 ||
-             (n == 512 && d->dtype == GPE_C64)) &&
-            d->generic_only != 1 && line_ok && !(d->local_fp64 && d->dtype == GPE_C64) &&
+  p->fixed = n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 160 || n == 256 ||
+             (n == 512 && d->dtype == GPE_C64);
+  {
+    std::vector<int> merged;
+    const std::vector<int> passes(p->pp.radix, p->pp.radix + p->pp.npass);
+    line_radices(n, merged);
+    for (int q = 0; q < 2; ++q) {
+      gpe_plan::LineSet& s = p->ls[q];
+      s.ok = line_geometry(n, q == 1 && d->dtype == GPE_C64 ? passes : merged, s.geo);
+      if (!s.ok) continue;
+      s.geo.direct = q == 1 && d->dtype == GPE_C64;
+      s.z = line_shape_z(s.geo, (int)p->csize);
+      s.p = line_shape_p(s.geo, (int)p->csize);
+    }
+    // (a side of one radix has no exchange: the Stockham sweeps take it)
+    p->line = p->ls[0].ok && p->ls[1].ok;
+  }
+  p->fast = (p->fixed || p->line) && d->generic_only != 1 && line_ok && !(d->local_fp64 && d->dtype == GPE_C64) &&
             !d->exact_local;
   if (!p->fast) { p->prog_line.clear(); p->slot_progs.clear(); }
   p->plane = p->fast && d->dtype == GPE_C64 && (n == 128 || n == 256) && d->generic_only == 3;
@@ -989,6 +1026,8 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
         p->counts[std::min(s, p->nbins - 1)]++;
       }
   p->max_tiles = std::max(tiles_of(p, AX_Z), tiles_of(p, AX_X));
+  for (const auto& s : p->ls)
+    if (s.ok) p->max_tiles = std::max(p->max_tiles, std::max(s.z.tiles, s.p.tiles));
   return GPE_OK;
 }
 
@@ -1009,6 +1048,43 @@ int upload_tables(gpe_plan* p, const gpe_desc* d) {
   CU(cudaMalloc(&p->d_tw, 2 * n * sizeof(tw[0])));
   CU(cudaMemcpy(p->d_tw, tw.data(), n * sizeof(tw[0]), cudaMemcpyHostToDevice));
   CU(cudaMemcpy((char*)p->d_tw + n * sizeof(tw[0]), twl.data(), n * sizeof(tw[0]), cudaMemcpyHostToDevice));
+  // run-time-length sweeps: twiddles in the order of each phase's lanes, butterfly tables
+  for (auto& ls : p->ls) {
+    if (!ls.ok) continue;
+    LineGeo& g = ls.geo;
+    std::vector<typename TwE<R>::T> lt;
+    std::vector<int> lb, bf;
+    size_t tw0[LINE_PMAX] = {}, twi0[LINE_PMAX] = {}, bf0[LINE_PMAX] = {};
+    auto push = [&](int e) {
+      if constexpr (sizeof(R) == 4) lt.push_back(make_float4(tw[e].x, tw[e].y, twl[e].x, twl[e].y));
+      else lt.push_back(tw[e]);
+    };
+    for (int q = 0; q < g.P; ++q) {
+      if (q > 0) {
+        bf0[q] = lb.size();
+        line_butterflies(g, q, bf);
+        lb.insert(lb.end(), bf.begin(), bf.end());
+        twi0[q] = lt.size();
+        for (int a = 1; a < g.r[q]; ++a)
+          for (int c = 0; c < g.np[q]; ++c) push(g.nl[q] * a * c);
+      }
+      if (q < g.P - 1) {
+        tw0[q] = lt.size();
+        for (int k = 1; k < g.r[q]; ++k)
+          for (int c = 0; c < g.nl[q]; ++c) push(g.np[q] * k * c);
+      }
+    }
+    CU(cudaMalloc(&ls.d_tw, lt.size() * sizeof(lt[0])));
+    CU(cudaMemcpy(ls.d_tw, lt.data(), lt.size() * sizeof(lt[0]), cudaMemcpyHostToDevice));
+    CU(cudaMalloc(&ls.d_bf, lb.size() * sizeof(int)));
+    CU(cudaMemcpy(ls.d_bf, lb.data(), lb.size() * sizeof(int), cudaMemcpyHostToDevice));
+    for (int q = 0; q < g.P; ++q) {
+      g.tw[q] = (const char*)ls.d_tw + tw0[q] * sizeof(lt[0]);
+      g.twi[q] = (const char*)ls.d_tw + twi0[q] * sizeof(lt[0]);
+      g.bf[q] = (const char*)ls.d_bf + bf0[q] * sizeof(int);
+    }
+    g.w = p->d_tw;
+  }
   // static axis potentials
   std::vector<R> vax(3 * n, (R)0);
   const double* ap[] = {d->static_x, d->static_y, d->static_z};
@@ -1054,7 +1130,7 @@ void free_plan(gpe_plan* p) {
   for (auto e : p->pool) cudaEventDestroy(e);
   void* bufs[] = {p->d_x, p->d_k, p->d_kin, p->d_kth, p->d_vax, p->d_vre, p->d_vim, p->d_prog_g, p->d_dyn, p->d_line, p->d_ltab,
                   p->d_tw, p->d_partial, p->d_ticket, p->d_scale, p->d_status, p->d_hist, p->d_out,
-                  p->d_work, p->d_plane, p->d_proj};
+                  p->d_work, p->d_plane, p->d_proj, p->ls[0].d_tw, p->ls[0].d_bf, p->ls[1].d_tw, p->ls[1].d_bf};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete p;
@@ -1206,15 +1282,15 @@ int fft3d(gpe_plan* p, const void* in, void* out, bool inverse, cudaStream_t st)
   if (p->fast) {
     Sweep s = mk_sweep(in, out);
     if (!inverse) {
-      TRY(fsweep(p, AX_Z, s, mk_ops(FM_PLAIN), st));
+      TRY(fsweep(p, AX_Z, s, tr_ops(FM_PLAIN), st));
       s.src = out;
-      TRY(fsweep(p, AX_Y, s, mk_ops(FM_PLAIN), st));
-      return fsweep(p, AX_X, s, mk_ops(FM_PLAIN), st);
+      TRY(fsweep(p, AX_Y, s, tr_ops(FM_PLAIN), st));
+      return fsweep(p, AX_X, s, tr_ops(FM_PLAIN), st);
     }
-    TRY(fsweep(p, AX_X, s, mk_ops(FM_PLAIN, 1), st));
+    TRY(fsweep(p, AX_X, s, tr_ops(FM_PLAIN, 1), st));
     s.src = out;
-    TRY(fsweep(p, AX_Y, s, mk_ops(FM_PLAIN, 1), st));
-    return fsweep(p, AX_Z, s, mk_ops(FM_PLAIN, 1, 1), st);
+    TRY(fsweep(p, AX_Y, s, tr_ops(FM_PLAIN, 1), st));
+    return fsweep(p, AX_Z, s, tr_ops(FM_PLAIN, 1, 1), st);
   }
   if (!inverse) {
     Sweep s = mk_sweep(in, out);
@@ -1278,7 +1354,10 @@ int finish_diag(gpe_plan* p, int na, int nb, bool hist, std::vector<double>& hos
 // shells in the x sweep); results stay on the device until finish_diag.
 // Tile counts of the diagnostic z and x sweeps (the partials to finish).
 void diag_tiles(const gpe_plan* p, bool fast, int& na, int& nb) {
-  if (fast) {
+  if (fast && !p->fixed) {
+    na = p->ls[1].z.tiles;
+    nb = p->ls[1].p.tiles;
+  } else if (fast) {
     const int lt = fast_lines(p->n, (int)p->csize / 2);
     na = p->n * p->n / lt;
     nb = p->n * (p->n / lt);
@@ -1291,7 +1370,9 @@ void diag_tiles(const gpe_plan* p, bool fast, int& na, int& nb) {
 // The diagnostics run on the register-resident sweeps when the plan has them
 // and the shell histogram (if wanted) fits their shared tables region.
 bool diag_fast(const gpe_plan* p, bool hist) {
-  return p->fast && (!hist || (size_t)p->nbins * sizeof(double) <= fast_tables_bytes_rt(p->n, (int)p->csize / 2));
+  if (!p->fast || !hist) return p->fast;
+  if (p->fixed) return (size_t)p->nbins * sizeof(double) <= fast_tables_bytes_rt(p->n, (int)p->csize / 2);
+  return line_smem(p->ls[1].geo, p->ls[1].p, (int)p->csize, false, p->nbins) <= 96 * 1024;
 }
 
 int diag_launch(gpe_plan* p, const void* psi, double t, bool hist, cudaStream_t st) {
@@ -1299,15 +1380,15 @@ int diag_launch(gpe_plan* p, const void* psi, double t, bool hist, cudaStream_t 
     Sweep s = mk_sweep(psi, p->d_work);
     s.t1 = t;
     s.partial = p->d_partial;
-    TRY(fsweep(p, AX_Z, s, mk_ops(FM_DIAGR), st));
+    TRY(fsweep(p, AX_Z, s, tr_ops(FM_DIAGR), st));
     s = mk_sweep(p->d_work, p->d_work);
-    TRY(fsweep(p, AX_Y, s, mk_ops(FM_PLAIN), st));
+    TRY(fsweep(p, AX_Y, s, tr_ops(FM_PLAIN), st));
     s = mk_sweep(p->d_work, nullptr);
     s.partial = p->d_partial + 4 * (size_t)p->max_tiles;
     s.hist = hist ? p->d_hist : nullptr;
     s.nbins = p->nbins;
     s.shell_w = p->shell_w;
-    return fsweep(p, AX_X, s, mk_ops(FM_DIAGK), st);
+    return fsweep(p, AX_X, s, tr_ops(FM_DIAGK), st);
   }
   Sweep s = mk_sweep(psi, p->d_work);
   s.pre = PW_DIAG_R;
@@ -1868,12 +1949,22 @@ int group_launch(gpe_batch* b, gpe_batch::Group& g, int role, cudaStream_t st) {
       case ROLE_Y1: op = mk_ops(FM_PLAIN); break;
       case ROLE_X: op = mk_ops(FM_XKIN); break;
       case ROLE_Y2: op = mk_ops(FM_PLAIN, 1); break;
-      case ROLE_DZ: op = mk_ops(FM_DIAGR); break;
-      case ROLE_DY: op = mk_ops(FM_PLAIN); break;
-      case ROLE_DX: op = mk_ops(FM_DIAGK); break;
+      case ROLE_DZ: op = tr_ops(FM_DIAGR); break;
+      case ROLE_DY: op = tr_ops(FM_PLAIN); break;
+      case ROLE_DX: op = tr_ops(FM_DIAGK); break;
       default: op = mk_ops(FM_Z2, 0, 0, 0, g.kind == GPE_IMAGINARY ? 1 : 0); break;
     }
-    CU(launch_fast_batch<R>(g.n, fax, g.d_ph, sws, count, op, st));
+    const gpe_plan* p = b->plans[g.members[0]];
+    if (p->fixed) {
+      CU(launch_fast_batch<R>(g.n, fax, g.d_ph, sws, count, op, st));
+    } else {
+      // (the members share the side: the first one's geometry and tables serve all; a change
+      // of membership discards the step graph that holds their addresses)
+      const gpe_plan::LineSet& ls = p->ls[op.tr];
+      const LineShape& shape = fax == FZ ? ls.z : ls.p;
+      const size_t smem = line_smem(ls.geo, shape, (int)p->csize, fax == FZ, 0);
+      CU(launch_line_batch<R>(fax, g.d_ph, sws, count, op, ls.geo, shape, smem, st));
+    }
   } else {
     gpe_plan* p = b->plans[g.members[0]];
     Sweep geo = mk_sweep(nullptr, nullptr);
