@@ -289,6 +289,17 @@ __global__ void k_build_static(int n, const double* x, const double* prog, int l
 
 // Sum per-block diagnostic partials in a fixed order: out[0..3] = sums of pa
 // columns 0..2 and pb column 3 (the shell bins out[4 + b] come from k_finish_hist).
+// Angular momentum: the sums of the x and y sweeps' partials (column 3) into out[0], out[1].
+__global__ void k_finish_lz(const double* px, int nx, const double* py, int ny, double* out) {
+  __shared__ Acc sh[32 * 2];
+  Acc a[2];
+  for (int b = threadIdx.x; b < nx; b += blockDim.x) a[0].add(px[(long long)b * 4 + 3]);
+  for (int b = threadIdx.x; b < ny; b += blockDim.x) a[1].add(py[(long long)b * 4 + 3]);
+  block_merge<2>(a, sh);
+  if (threadIdx.x == 0)
+    for (int v = 0; v < 2; ++v) out[v] = a[v].value();
+}
+
 __global__ void k_finish_diag(const double* pa, int na, const double* pb, int nb, double* out) {
   __shared__ Acc sh[32 * 4];
   Acc a[4];
@@ -391,6 +402,32 @@ __device__ __forceinline__ void scale_state(typename Cx<R>::T* psi, long long co
 template <typename R>
 __global__ void __launch_bounds__(256) k_scale(Sweep sw, long long count) {
   scale_state<R>((typename Cx<R>::T*)sw.dst, count, sw.scale);
+}
+
+// Norm of a state into the plan's scale: a streaming read (8 loads in flight per thread,
+// summed in plain FP64 in a fixed order, then compensated across threads and blocks).
+// Bound by HBM; the no-transform Stockham sweep it replaces staged every element through
+// shared memory with a division for its coordinates: 53 us at 128^3 complex128.
+constexpr int NORM_UNROLL = 8;
+template <typename R>
+__global__ void __launch_bounds__(256) k_norm(Phys ph, Sweep sw, long long count) {
+  __shared__ Acc red[32];
+  using C = typename Cx<R>::T;
+  const C* __restrict__ psi = (const C*)sw.src;
+  Acc a[1];
+  const long long chunk = 256LL * NORM_UNROLL;
+  for (long long e0 = blockIdx.x * chunk + threadIdx.x; e0 < count; e0 += gridDim.x * chunk) {
+    C v[NORM_UNROLL];
+#pragma unroll
+    for (int q = 0; q < NORM_UNROLL; ++q) v[q] = e0 + q * 256 < count ? psi[e0 + q * 256] : mk((R)0, (R)0);
+    double sum = 0.0;
+#pragma unroll
+    for (int q = 0; q < NORM_UNROLL; ++q)
+      sum = fma((double)v[q].x, (double)v[q].x, fma((double)v[q].y, (double)v[q].y, sum));
+    a[0].add(sum);
+  }
+  block_merge<1>(a, red);
+  norm_finish(ph, sw, a[0], red);
 }
 
 // batched: blockIdx.y selects the instance
@@ -810,9 +847,9 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   FastOps o = op;
   o.pdl = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
   p->pdl_prev = p->pdl_chain;
-  const CUtensorMap* map = p->tma && o.mode == FM_PLAIN && fax != FZ ? tma_maps(p, sw.src, fax) : nullptr;
-  const bool line = !p->fixed || o.mode == FM_LZ;
-  const gpe_plan::LineSet& ls = p->ls[o.tr];
+  const CUtensorMap* map = p->tma && o.tr != 2 && o.mode == FM_PLAIN && fax != FZ ? tma_maps(p, sw.src, fax) : nullptr;
+  const bool line = !p->fixed || o.tr == 2;
+  const gpe_plan::LineSet& ls = p->ls[o.tr ? 1 : 0];
   const LineShape& shape = fax == FZ ? ls.z : ls.p;
   const size_t smem = line ? line_smem(ls.geo, shape, (int)p->csize, fax == FZ, sw.hist ? sw.nbins : 0) : 0;
   const cudaError_t e =
@@ -879,10 +916,16 @@ FastOps mk_ops(int mode, int inv1 = 0, int invm = 0, int scale = 0, int norm = 0
   return o;
 }
 
-// the same for a sweep of a transform or reduction
+// the same for a sweep of a transform or reduction; lz_ops: on the run-time-length sweeps
+// whatever the side (they carry the angular-momentum sums)
 FastOps tr_ops(int mode, int inv1 = 0, int invm = 0) {
   FastOps o = mk_ops(mode, inv1, invm);
   o.tr = 1;
+  return o;
+}
+FastOps lz_ops(int mode) {
+  FastOps o = mk_ops(mode);
+  o.tr = 2;
   return o;
 }
 
@@ -907,12 +950,22 @@ Sweep mk_sweep(const void* src, void* dst) {
 double t_mid_host(const gpe_plan* p, long long step) { return (double)step * p->dt + p->dt / 2; }
 
 
-// Norm of psi into d_scale (sqrtN, 1/sqrtN, N) via a no-store sweep.
+// Norm of psi into d_scale (sqrtN, 1/sqrtN, N).
 int norm_sweep(gpe_plan* p, const void* psi, cudaStream_t st) {
   Sweep s = mk_sweep(psi, nullptr);
-  s.post = PW_NORM;
   s.partial = p->d_partial;
-  return sweep(p, AX_Z, s, st);
+  s.ticket = p->d_ticket;
+  s.scale = p->d_scale;
+  s.status = p->d_status;
+  const long long count = (long long)p->n * p->n * p->n;
+  // up to eight blocks per SM (one partial sum each)
+  const long long chunks = (count + 256 * NORM_UNROLL - 1) / (256 * NORM_UNROLL);
+  const unsigned blocks = (unsigned)std::min(chunks, (long long)std::min(8 * 148, p->max_tiles));
+  if (p->dtype == GPE_C64) k_norm<float><<<blocks, 256, 0, st>>>(p->ph, s, count);
+  else k_norm<double><<<blocks, 256, 0, st>>>(p->ph, s, count);
+  CU(cudaGetLastError());
+  ++p->launches;
+  return GPE_OK;
 }
 
 int scale_sweep(gpe_plan* p, void* psi, cudaStream_t st) {
@@ -1408,43 +1461,53 @@ int diag_launch(gpe_plan* p, const void* psi, double t, bool hist, cudaStream_t 
 }
 
 // Lz of psi (reference gpe/helper.py:143-156).  By Parseval along each axis the
-// reference's slab sums become two k-space sums of the z-transformed state F_z:
-//   Lz = dx^3/n^2 [ sum x k_y |FFT_y F_z|^2 - sum y k_x |FFT_x F_z|^2 ],
-// one forward z sweep into the work buffer and two read-only sweeps (x, y) of it;
-// the per-tile partials are summed on the host in tile order (deterministic).
+// reference's slab sums become two k-space sums,
+//   Lz = dx^3/n [ sum x k_y |FFT_y psi|^2 - sum y k_x |FFT_x psi|^2 ],
+// two read-only sweeps of psi.  complex64 sums the z transform of psi instead (one more
+// sweep, into the work buffer, and 1/n^2): a state with little rotation has an Lz far
+// below the terms of its sums, so its complex64 value depends on how the summed values
+// were rounded, and it keeps the one it has.  Plans on the Stockham sweeps (sides of one
+// radix, accuracy modes) take the same route in either precision.
 int angular_momentum(gpe_plan* p, const void* psi, double* lz, cudaStream_t st) {
-  TRY(ensure_work(p));
-  Sweep s = mk_sweep(psi, p->d_work);
+  const bool line = p->fast && p->line, through_z = !line || p->dtype == GPE_C64;
+  double* px = p->d_partial;
+  double* py = p->d_partial + 4 * (size_t)p->max_tiles;
+  int nx = 0, ny = 0;
+  const void* f = psi;
+  if (through_z) {
+    TRY(ensure_work(p));
+    f = p->d_work;
+    Sweep s = mk_sweep(psi, p->d_work);
+    s.fft1 = 1;
+    if (line) TRY(fsweep(p, AX_Z, s, lz_ops(FM_PLAIN), st));
+    else TRY(sweep(p, AX_Z, s, st));
+  }
+  Sweep s = mk_sweep(f, nullptr);
   s.fft1 = 1;
-  TRY(sweep(p, AX_Z, s, st));
-  s = mk_sweep(p->d_work, nullptr);
-  s.fft1 = 1;
-  s.post = PW_LZ_X;
-  s.partial = p->d_partial;
-  TRY(sweep(p, AX_X, s, st));
-  s = mk_sweep(p->d_work, nullptr);
-  s.fft1 = 1;
-  s.post = PW_LZ_Y;
-  s.partial = p->d_partial + 4 * (size_t)p->max_tiles;
-  TRY(sweep(p, AX_Y, s, st));
-  const int nx = tiles_of(p, AX_X), ny = tiles_of(p, AX_Y);
-  std::vector<double> hx(4 * (size_t)nx), hy(4 * (size_t)ny);
-  CU(cudaMemcpyAsync(hx.data(), p->d_partial, hx.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(hy.data(), p->d_partial + 4 * (size_t)p->max_tiles, hy.size() * sizeof(double),
-                     cudaMemcpyDeviceToHost, st));
+  if (line) {
+    nx = ny = p->ls[1].p.tiles;
+    s.partial = px;
+    TRY(fsweep(p, AX_X, s, lz_ops(FM_LZ), st));
+    s.partial = py;
+    TRY(fsweep(p, AX_Y, s, lz_ops(FM_LZ), st));
+  } else {
+    nx = tiles_of(p, AX_X);
+    ny = tiles_of(p, AX_Y);
+    s.post = PW_LZ_X;
+    s.partial = px;
+    TRY(sweep(p, AX_X, s, st));
+    s.post = PW_LZ_Y;
+    s.partial = py;
+    TRY(sweep(p, AX_Y, s, st));
+  }
+  k_finish_lz<<<1, 512, 0, st>>>(px, nx, py, ny, p->d_out);
+  CU(cudaGetLastError());
+  ++p->launches;
+  double h[2];
+  CU(cudaMemcpyAsync(h, p->d_out, sizeof(h), cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
-  // compensated sums in tile order
-  auto csum = [](const std::vector<double>& v, int count) {
-    double sum = 0.0, c = 0.0;
-    for (int b = 0; b < count; ++b) {
-      const double y = v[4 * (size_t)b + 3] - c, t = sum + y;
-      c = (t - sum) - y;
-      sum = t;
-    }
-    return sum;
-  };
-  const double n2 = (double)p->n * p->n;
-  *lz = (csum(hy, ny) - csum(hx, nx)) / n2 * p->ph.dx3;
+  const double scale = through_z ? (double)p->n * p->n : (double)p->n;
+  *lz = (h[1] - h[0]) / scale * p->ph.dx3;
   return GPE_OK;
 }
 
