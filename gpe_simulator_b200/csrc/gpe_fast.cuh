@@ -1044,10 +1044,8 @@ __device__ __forceinline__ void fast_batch_body(const Phys* __restrict__ phs, co
                                                 const FastOps& op) {
   __shared__ Phys ph;
   __shared__ Sweep sw;
-  if (threadIdx.x == 0) {
-    ph = phs[blockIdx.y];
-    sw = sws[blockIdx.y];
-  }
+  copy_words(&ph, phs + blockIdx.y);
+  copy_words(&sw, sws + blockIdx.y);
   __syncthreads();
   if (batch_frozen(sw.live)) return;
   fast_body<N, AX, R, MODE>(ph, sw, op, blockIdx.x, gridDim.x);

@@ -82,13 +82,17 @@ struct Sweep {
                          // launches return at once; null: always advance
 };
 
-// A batched launch's instance is frozen: thread 0 reads the flag (written by an
-// earlier launch on the stream) into shared memory; every thread returns alike.
-__device__ __forceinline__ bool batch_frozen(const int* live) {
-  __shared__ int s_live;
-  if (threadIdx.x == 0) s_live = live ? __ldcg(live) : 1;
-  __syncthreads();
-  return s_live == 0;
+// A batched launch's instance is frozen (the flag was written by an earlier launch on the
+// stream, so every thread reads the same).
+__device__ __forceinline__ bool batch_frozen(const int* live) { return live && __ldcg(live) == 0; }
+
+// A batched launch's instance: its structs copied into shared memory by the whole block,
+// a word per thread (one thread copying them field by field held every block up for the
+// latency of its loads).
+template <typename T> __device__ __forceinline__ void copy_words(T* dst, const T* __restrict__ src) {
+  static_assert(sizeof(T) % 8 == 0, "whole words");
+  for (int q = threadIdx.x; q < (int)(sizeof(T) / 8); q += blockDim.x)
+    ((unsigned long long*)dst)[q] = ((const unsigned long long*)src)[q];
 }
 
 // Values of a line program's slots (its time-dependent subexpressions, FP64,
@@ -598,10 +602,8 @@ __global__ void __launch_bounds__(512, 1) k_sweep_batch(const Phys* __restrict__
                                                          const Sweep* __restrict__ sws) {
   __shared__ Phys ph;
   __shared__ Sweep sw;
-  if (threadIdx.x == 0) {
-    ph = phs[blockIdx.y];
-    sw = sws[blockIdx.y];
-  }
+  copy_words(&ph, phs + blockIdx.y);
+  copy_words(&sw, sws + blockIdx.y);
   __syncthreads();
   if (batch_frozen(sw.live)) return;
   sweep_body<R, AX, EPT, GEN>(ph, sw);

@@ -511,10 +511,8 @@ __global__ void __launch_bounds__(LINE_T, LineBounds<R>::blocks) k_line_batch(co
                                                                             int ax) {
   __shared__ Phys ph;
   __shared__ Sweep sw;
-  if (threadIdx.x == 0) {
-    ph = phs[blockIdx.y];
-    sw = sws[blockIdx.y];
-  }
+  copy_words(&ph, phs + blockIdx.y);
+  copy_words(&sw, sws + blockIdx.y);
   __syncthreads();
   if (batch_frozen(sw.live)) return;
   line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, blockIdx.x, gridDim.x);
