@@ -90,6 +90,7 @@ struct FastOps {
                     // complex64, whose rounding such results keep), 2 the same on the
                     // run-time-length sweeps whatever the side
   int pdl;          // host: launch as a programmatic dependent of the previous sweep
+  int rev;          // tiles in descending order (see tile_of)
   int pf;           // tiles ahead whose lines a block prefetches into L2 (0 = none): the
                     // tile the block that follows it on the SM will process
 };
@@ -461,10 +462,10 @@ struct FastTables {
 // pre (real time, two half-steps as one rotation): vz and
 // c12 are stored already multiplied by dt (vz by dt, c12 by dt/2), so that the
 // phase (2 vz + c12 + 2 beta |psi|^2) dt/2 is one add and one fma per point.
-template <int N, typename R>
+template <int N, typename R, int T = FastCfg<N, R>::T>
 __device__ __forceinline__ void z_tables(const Phys& ph, const Sweep& sw, int a0, FastTables<R>& tb,
                                          bool two, bool pre = false) {
-  constexpr int L = FastCfg<N, R>::L, T = FastCfg<N, R>::T;
+  constexpr int L = FastCfg<N, R>::L;
   const R* vax = (const R*)ph.vax;
   const R h = (R)(ph.dt * 0.5), dt2 = h + h;
   for (int q = threadIdx.x; q < N; q += T) tb.vz[q] = pre ? vax[2 * N + q] * dt2 : vax[2 * N + q];
@@ -493,9 +494,9 @@ __device__ __forceinline__ void z_tables(const Phys& ph, const Sweep& sw, int a0
   }
 }
 
-template <int N, typename R>
+template <int N, typename R, int T = FastCfg<N, R>::T>
 __device__ __forceinline__ void x_tables(const Phys& ph, int j, int k0, FastTables<R>& tb) {
-  constexpr int L = FastCfg<N, R>::L, T = FastCfg<N, R>::T;
+  constexpr int L = FastCfg<N, R>::L;
   for (int q = threadIdx.x; q < N; q += T) {
     tb.kx[q] = ph.kin[q];
     tb.kx2[q] = ph.k[q] * ph.k[q];
@@ -849,10 +850,10 @@ __device__ __forceinline__ void fast_store(const typename Cx<R>::T (&v)[EPT], co
 
 // Prefetch the lines of tile `tn` into L2 (128-byte lines; z tiles are one
 // contiguous block, y/x tiles N rows of L elements).
-template <int N, int AX, typename R>
+template <int N, int AX, typename R, int T = FastCfg<N, R>::T>
 __device__ __forceinline__ void fast_prefetch_l2(const FastTile<N, AX, R>& tn, const void* src) {
   using C = typename Cx<R>::T;
-  constexpr int L = FastCfg<N, R>::L, T = FastCfg<N, R>::T;
+  constexpr int L = FastCfg<N, R>::L;
   const C* base = (const C*)src + tn.base;
   if (AX == FZ) {
     constexpr int LINES = L * N * (int)sizeof(C) / 128;
@@ -965,7 +966,10 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
   // Bring the tile of the next wave's block on this SM into L2 while this one
   // computes: one wave ahead (tile + resident blocks), measured 51.2 -> 46.4 us
   // for the y sweep at 256^3 (two waves ahead was slower).
-  if (!CG && op.pf > 0 && tile + op.pf < ntiles) fast_prefetch_l2<N, AX, R>(FastTile<N, AX, R>(tile + op.pf), sw.src);
+  if (!CG && op.pf > 0) {
+    const int next = op.rev ? tile - op.pf : tile + op.pf;
+    if (next >= 0 && next < ntiles) fast_prefetch_l2<N, AX, R>(FastTile<N, AX, R>(next), sw.src);
+  }
   prologue();
   __syncthreads();  // twiddles and tables visible
   if (MODE == FM_Z1) fast_pointwise<N, AX, R, MODE, 0, N1, N2, S1>(v, tl, ph, tb, op, cx);
@@ -1028,14 +1032,18 @@ template <int N, typename R, int MODE> struct FastBounds {
                                    ? (MODE == FM_DIAGR ? 512 : 1024) / FastCfg<N, R>::T : 0;
 };
 
+__device__ __forceinline__ int tile_of(const FastOps& op) {
+  return op.rev ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+}
+
 template <int N, int AX, typename R, int MODE>
 __global__ void __launch_bounds__(FastCfg<N, R>::T) k_fast(Phys ph, Sweep sw, FastOps op) {
-  fast_body<N, AX, R, MODE>(ph, sw, op, blockIdx.x, gridDim.x);
+  fast_body<N, AX, R, MODE>(ph, sw, op, tile_of(op), gridDim.x);
 }
 
 template <int N, int AX, typename R, int MODE, int B>
 __global__ void __launch_bounds__(FastCfg<N, R>::T, B) k_fast_occ(Phys ph, Sweep sw, FastOps op) {
-  fast_body<N, AX, R, MODE>(ph, sw, op, blockIdx.x, gridDim.x);
+  fast_body<N, AX, R, MODE>(ph, sw, op, tile_of(op), gridDim.x);
 }
 
 // Batched launch: blockIdx.y selects the instance (structs staged in shared memory).
@@ -1048,7 +1056,7 @@ __device__ __forceinline__ void fast_batch_body(const Phys* __restrict__ phs, co
   copy_words(&sw, sws + blockIdx.y);
   __syncthreads();
   if (batch_frozen(sw.live)) return;
-  fast_body<N, AX, R, MODE>(ph, sw, op, blockIdx.x, gridDim.x);
+  fast_body<N, AX, R, MODE>(ph, sw, op, tile_of(op), gridDim.x);
 }
 
 template <int N, int AX, typename R, int MODE>

@@ -266,7 +266,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       const C* p = src + base + (long long)l * lstride + (long long)q * nstride;
       C v[RAD];
 #pragma unroll
-      for (int a = 0; a < RAD; ++a) v[a] = p[a * st];
+      for (int a = 0; a < RAD; ++a) v[a] = __ldcg(p + a * st);   // (past L1, which holds the tables)
       if (conj_in) {
 #pragma unroll
         for (int a = 0; a < RAD; ++a) v[a].y = -v[a].y;
@@ -500,7 +500,7 @@ template <typename R> struct LineBounds { static constexpr int blocks = sizeof(R
 template <typename R, bool ZT, int MODE>
 __global__ void __launch_bounds__(LINE_T, LineBounds<R>::blocks) k_line(Phys ph, Sweep sw, FastOps op, LineGeo g,
                                                                       LineShape sh, int ax) {
-  line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, blockIdx.x, gridDim.x);
+  line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, tile_of(op), gridDim.x);
 }
 
 // Batched launch: blockIdx.y selects the instance (structs staged in shared memory).
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(LINE_T, LineBounds<R>::blocks) k_line_batch(co
   copy_words(&sw, sws + blockIdx.y);
   __syncthreads();
   if (batch_frozen(sw.live)) return;
-  line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, blockIdx.x, gridDim.x);
+  line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, tile_of(op), gridDim.x);
 }
 
 // host: launch one sweep (one translation unit per precision and group of modes)

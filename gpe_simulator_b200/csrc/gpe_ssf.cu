@@ -607,6 +607,7 @@ struct gpe_plan {
   int tma_next = 0;
   bool pdl_chain = false;          // inside a step sequence: sweeps may launch programmatically
   bool pdl_prev = false;           // a sweep of the current sequence has been launched
+  int sweep_dir = 0;               // tile order of its next sweep (1: descending)
   int ept = 16;                    // elements per thread of the sweep family
   int nbins = 0;
   double shell_w = 0;
@@ -845,6 +846,15 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   }
   const int fax = ax == AX_Z ? FZ : ax == AX_Y ? FY : FX;
   FastOps o = op;
+  // A sweep takes its tiles in the order opposite to the sweep before it, so that it starts
+  // on what that one left in L2; only the y sweep after an x sweep keeps the x sweep's
+  // order.  256^3 complex64 (134 MB against 126 MB of L2): 225.9 -> 215.1 us per step; every
+  // order measured within 2% of this one but the plain one.  States that fit in L2 with
+  // room for their successor's writes gain nothing and keep the plain order.
+  if (p->pdl_chain && (size_t)p->n * p->n * p->n * p->csize > ((size_t)48 << 20)) {
+    o.rev = p->sweep_dir;
+    if (ax != AX_X) p->sweep_dir ^= 1;
+  }
   o.pdl = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
   p->pdl_prev = p->pdl_chain;
   const CUtensorMap* map = p->tma && o.tr != 2 && o.mode == FM_PLAIN && fax != FZ ? tma_maps(p, sw.src, fax) : nullptr;
@@ -912,7 +922,7 @@ int psweep(gpe_plan* p, void* psi, int mz, const FastOps* ops, int nstage, int z
 
 FastOps mk_ops(int mode, int inv1 = 0, int invm = 0, int scale = 0, int norm = 0) {
   FastOps o;
-  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.pf = 0;
+  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.rev = 0; o.pf = 0;
   return o;
 }
 
@@ -934,7 +944,7 @@ FastOps lz_ops(int mode) {
 // constants until their grid-dependency wait).
 struct PdlChain {
   gpe_plan* p;
-  explicit PdlChain(gpe_plan* q) : p(q) { p->pdl_chain = true; p->pdl_prev = false; }
+  explicit PdlChain(gpe_plan* q) : p(q) { p->pdl_chain = true; p->pdl_prev = false; p->sweep_dir = 0; }
   ~PdlChain() { p->pdl_chain = false; p->pdl_prev = false; }
 };
 
