@@ -90,6 +90,7 @@ struct FastOps {
                     // complex64, whose rounding such results keep), 2 the same on the
                     // run-time-length sweeps whatever the side
   int pdl;          // host: launch as a programmatic dependent of the previous sweep
+  int vec;          // host: src and dst aligned to 16 bytes (packed sweeps)
   int rev;          // tiles in descending order (see tile_of)
   int pf;           // tiles ahead whose lines a block prefetches into L2 (0 = none): the
                     // tile the block that follows it on the SM will process

@@ -1,22 +1,31 @@
 // gpe_fast_impl.cuh -- launch wrappers of the register-resident sweeps for one precision.
 #pragma once
 #include "gpe_fast.cuh"
+#include "gpe_packed.cuh"
 #include "gpe_sweep.h"
 #include "gpe_tma.cuh"
 
 namespace gpe {
 
-// the kernel of (N, AX, R, MODE): explicit occupancy bounds where measured
-template <int N, int AX, typename R, int MODE> constexpr auto fast_kernel() {
-  constexpr int B = FastBounds<N, R, MODE>::value;
-  if constexpr (B > 0) return &k_fast_occ<N, AX, R, MODE, B>;
-  else return &k_fast<N, AX, R, MODE>;
-}
-template <int N, int AX, typename R, int MODE> constexpr auto fast_batch_kernel() {
-  constexpr int B = FastBounds<N, R, MODE>::value;
-  if constexpr (B > 0) return &k_fast_batch_occ<N, AX, R, MODE, B>;
-  else return &k_fast_batch<N, AX, R, MODE>;
-}
+// the kernel of (N, AX, R, MODE), its threads and shared memory: the 512-point
+// complex64 sweeps take two lines per thread; explicit occupancy bounds where measured
+template <int N, int AX, typename R, int MODE, bool TR> struct FastKernel {
+  static constexpr bool PACK = sizeof(R) == 4 && !TR && pack_sweep(N, MODE);
+  static constexpr int T = PACK ? PackCfg<N>::T : FastCfg<N, R>::T;
+  static constexpr size_t SMEM = PACK ? pack_smem<N, MODE>() : fast_smem_bytes<N, R>();
+  static constexpr auto one() {
+    constexpr int B = FastBounds<N, R, MODE>::value;
+    if constexpr (PACK) return &k_pack<N, AX, MODE>;
+    else if constexpr (B > 0) return &k_fast_occ<N, AX, R, MODE, B>;
+    else return &k_fast<N, AX, R, MODE>;
+  }
+  static constexpr auto batch() {
+    constexpr int B = FastBounds<N, R, MODE>::value;
+    if constexpr (PACK) return &k_pack_batch<N, AX, MODE>;
+    else if constexpr (B > 0) return &k_fast_batch_occ<N, AX, R, MODE, B>;
+    else return &k_fast_batch<N, AX, R, MODE>;
+  }
+};
 
 // Blocks of `kern` resident on the whole device at once (the L2 prefetch
 // distance of a sweep: the tile the next block on an SM will take).
@@ -30,13 +39,14 @@ static cudaError_t resident_blocks(K kern, int threads, size_t smem, int& out) {
   return e;
 }
 
-template <int N, int AX, typename R, int MODE>
+template <int N, int AX, typename R, int MODE, bool TR = false>
 static cudaError_t launch_fast_one(const Phys& ph, const Sweep& sw, const FastOps& op_in, cudaStream_t st) {
   constexpr int L = FastCfg<N, R>::L;
-  constexpr int T = FastCfg<N, R>::T;
+  using FK = FastKernel<N, AX, R, MODE, TR>;
+  constexpr int T = FK::T;
   const int tiles = AX == FZ ? N * N / L : N * (N / L);
-  constexpr size_t smem = fast_smem_bytes<N, R>();
-  constexpr auto kern = fast_kernel<N, AX, R, MODE>();
+  constexpr size_t smem = FK::SMEM;
+  constexpr auto kern = FK::one();
   static int attr_dev = -1, resident = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -76,19 +86,30 @@ cudaError_t launch_fast_n(int ax, const Phys& ph, const Sweep& sw, const FastOps
     case FM_DIAGK: return launch_fast_one<N, FX, R, FM_DIAGK>(ph, sw, op, st);
     default: break;
   }
+  // (transforms and reductions where the steps take other kernels)
+  if constexpr (sizeof(R) == 4 && pack_sweep(N, FM_PLAIN)) {
+    if (op.tr) {
+      if (ax == FZ) return launch_fast_one<N, FZ, R, FM_PLAIN, true>(ph, sw, op, st);
+      if (ax == FY) return launch_fast_one<N, FY, R, FM_PLAIN, true>(ph, sw, op, st);
+      return launch_fast_one<N, FX, R, FM_PLAIN, true>(ph, sw, op, st);
+    }
+    if (ax == FY) return launch_fast_one<N, FY, R, FM_PLAIN>(ph, sw, op, st);
+    return cudaErrorInvalidValue;
+  }
   if (ax == FZ) return launch_fast_one<N, FZ, R, FM_PLAIN>(ph, sw, op, st);
   if (ax == FY) return launch_fast_one<N, FY, R, FM_PLAIN>(ph, sw, op, st);
   return launch_fast_one<N, FX, R, FM_PLAIN>(ph, sw, op, st);
 }
 
-template <int N, int AX, typename R, int MODE>
+template <int N, int AX, typename R, int MODE, bool TR = false>
 static cudaError_t launch_fastb_one(const Phys* phs, const Sweep* sws, int count, const FastOps& op_in,
                                     cudaStream_t st) {
   constexpr int L = FastCfg<N, R>::L;
-  constexpr int T = FastCfg<N, R>::T;
+  using FK = FastKernel<N, AX, R, MODE, TR>;
+  constexpr int T = FK::T;
   const int tiles = AX == FZ ? N * N / L : N * (N / L);
-  constexpr size_t smem = fast_smem_bytes<N, R>();
-  constexpr auto kern = fast_batch_kernel<N, AX, R, MODE>();
+  constexpr size_t smem = FK::SMEM;
+  constexpr auto kern = FK::batch();
   static int attr_dev = -1, resident = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -117,6 +138,9 @@ cudaError_t launch_fastb_n(int ax, const Phys* phs, const Sweep* sws, int count,
     case FM_DIAGR: return launch_fastb_one<N, FZ, R, FM_DIAGR>(phs, sws, count, op, st);
     case FM_DIAGK: return launch_fastb_one<N, FX, R, FM_DIAGK>(phs, sws, count, op, st);
     default: break;
+  }
+  if constexpr (sizeof(R) == 4 && pack_sweep(N, FM_PLAIN)) {
+    if (op.tr) return ax == FY ? launch_fastb_one<N, FY, R, FM_PLAIN, true>(phs, sws, count, op, st) : cudaErrorInvalidValue;
   }
   if (ax == FZ) return launch_fastb_one<N, FZ, R, FM_PLAIN>(phs, sws, count, op, st);
   if (ax == FY) return launch_fastb_one<N, FY, R, FM_PLAIN>(phs, sws, count, op, st);

@@ -63,6 +63,7 @@ struct Sweep {
   void* dst;
   const void* tw;        // [n] forward twiddles W_n^j, precision of the sweep
   const void* tw_lo;     // [n] rounding residuals of tw (complex64), zeros (complex128)
+  const void* twp;       // packed complex64 sweeps: twiddles of both phases in lane order (null: none)
   PassPlan pp;
   int lt;                // lines per tile
   int tiles_per_row;     // y/x tiles: ceil(n/lt)

@@ -625,6 +625,7 @@ struct gpe_plan {
   double* d_line = nullptr;
   void* d_ltab = nullptr;          // [2][n*n] per-line dynamic potential (line form), precision of psi
   void* d_tw = nullptr;
+  void* d_twp = nullptr;         // packed complex64 sweeps (n = 512): twiddles in lane order
   double* d_partial = nullptr;   // 2 areas of 4*max_tiles doubles
   unsigned* d_ticket = nullptr;
   unsigned* d_plane = nullptr;   // plane-fused launches: ticket, finished blocks, per (plane, stage) counts
@@ -659,6 +660,7 @@ int sweep_geometry(const gpe_plan* p, int ax, Sweep& sw, int& tiles, int& thread
   sw.pp = p->pp;
   sw.tw = p->d_tw;
   sw.tw_lo = (const char*)p->d_tw + (size_t)n * sizeof(C);
+  sw.twp = p->d_twp;
   sw.ticket = p->d_ticket;
   sw.scale = p->d_scale;
   sw.status = p->d_status;
@@ -835,6 +837,7 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   sw.pp = p->pp;
   sw.tw = p->d_tw;
   sw.tw_lo = (const char*)p->d_tw + (size_t)p->n * p->csize;
+  sw.twp = p->d_twp;
   sw.ticket = p->d_ticket;
   sw.scale = p->d_scale;
   sw.status = p->d_status;
@@ -846,6 +849,7 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   }
   const int fax = ax == AX_Z ? FZ : ax == AX_Y ? FY : FX;
   FastOps o = op;
+  o.vec = ((uintptr_t)sw.src | (uintptr_t)sw.dst) % 16 == 0;
   // A sweep takes its tiles in the order opposite to the sweep before it, so that it starts
   // on what that one left in L2; only the y sweep after an x sweep keeps the x sweep's
   // order.  256^3 complex64 (134 MB against 126 MB of L2): 225.9 -> 215.1 us per step; every
@@ -922,7 +926,7 @@ int psweep(gpe_plan* p, void* psi, int mz, const FastOps* ops, int nstage, int z
 
 FastOps mk_ops(int mode, int inv1 = 0, int invm = 0, int scale = 0, int norm = 0) {
   FastOps o;
-  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.rev = 0; o.pf = 0;
+  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.vec = 0; o.rev = 0; o.pf = 0;
   return o;
 }
 
@@ -1148,6 +1152,25 @@ int upload_tables(gpe_plan* p, const gpe_desc* d) {
     }
     g.w = p->d_tw;
   }
+  // packed sweeps: entries (hi.x, hi.x, hi.y, hi.y), then the residuals, [value][lane]: the
+  // first phase's W_512^(p k3), then the second's W_64^(p1 k1)
+  if constexpr (sizeof(R) == 4) {
+    if (n == 512) {
+      std::vector<float4> tp;
+      auto table = [&](int lanes, int vals, int stride) {
+        for (int part = 0; part < 2; ++part)
+          for (int k = 0; k < vals; ++k)
+            for (int l = 0; l < lanes; ++l) {
+              const float2 w = (part ? twl : tw)[stride * k * l];
+              tp.push_back(make_float4(w.x, w.x, w.y, w.y));
+            }
+      };
+      table(64, 8, 1);
+      table(8, 8, 8);
+      CU(cudaMalloc(&p->d_twp, tp.size() * sizeof(tp[0])));
+      CU(cudaMemcpy(p->d_twp, tp.data(), tp.size() * sizeof(tp[0]), cudaMemcpyHostToDevice));
+    }
+  }
   // static axis potentials
   std::vector<R> vax(3 * n, (R)0);
   const double* ap[] = {d->static_x, d->static_y, d->static_z};
@@ -1193,7 +1216,7 @@ void free_plan(gpe_plan* p) {
   for (auto e : p->pool) cudaEventDestroy(e);
   void* bufs[] = {p->d_x, p->d_k, p->d_kin, p->d_kth, p->d_vax, p->d_vre, p->d_vim, p->d_prog_g, p->d_dyn, p->d_line, p->d_ltab,
                   p->d_tw, p->d_partial, p->d_ticket, p->d_scale, p->d_status, p->d_hist, p->d_out,
-                  p->d_work, p->d_plane, p->d_proj, p->ls[0].d_tw, p->ls[0].d_bf, p->ls[1].d_tw, p->ls[1].d_bf};
+                  p->d_work, p->d_plane, p->d_proj, p->ls[0].d_tw, p->ls[0].d_bf, p->ls[1].d_tw, p->ls[1].d_bf, p->d_twp};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete p;
@@ -1841,6 +1864,7 @@ struct gpe_batch {
     int priority = 0;           // of `stream`: that of the stream the batch was last bound on
     cudaEvent_t ev = nullptr;
     int uploaded = 0;           // member count the device arrays hold
+    int aligned = 0;            // every member's state is aligned to 16 bytes
     // real time: half-step time and beam centres of every step of the current call,
     // [step][member][6] = {t_mid, cx, cy, t_end, cx, cy}, and each member's position in it
     double* d_times = nullptr;
@@ -2028,6 +2052,7 @@ int group_launch(gpe_batch* b, gpe_batch::Group& g, int role, cudaStream_t st) {
       default: op = mk_ops(FM_Z2, 0, 0, 0, g.kind == GPE_IMAGINARY ? 1 : 0); break;
     }
     const gpe_plan* p = b->plans[g.members[0]];
+    op.vec = g.aligned;
     if (p->fixed) {
       CU(launch_fast_batch<R>(g.n, fax, g.d_ph, sws, count, op, st));
     } else {
@@ -2116,6 +2141,9 @@ int group_upload(gpe_batch* b, gpe_batch::Group& g) {
     CU(cudaMalloc(&g.d_tick, sizeof(int) * m));
     g.times_cap = m;
   }
+  g.aligned = 1;
+  for (int i : g.members)
+    if ((uintptr_t)b->psis[i] % 16) g.aligned = 0;
   std::vector<Phys> hph(m);
   std::vector<Sweep> hsw((size_t)m * ROLE_COUNT);
   for (int q = 0; q < m; ++q) {
