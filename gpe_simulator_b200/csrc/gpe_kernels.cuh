@@ -29,6 +29,10 @@ enum Axis : int { AX_Z = 0, AX_Y = 1, AX_X = 2 };
 constexpr int OP_SQR = 40;
 constexpr int OP_SLOT0 = 64;
 #define GPE_LINE_SLOTS 8
+// point programs: push of row value k, of z value k
+constexpr int OP_ROW0 = 80;
+constexpr int OP_Z0 = 96;
+#define GPE_POINT_TABS 8
 
 // status bits
 enum : int { ST_NONFINITE = 1, ST_TIMEOUT = 2, ST_LAYOUT = 4 };  // ST_LAYOUT: a sweep refused its shared-memory layout
@@ -79,6 +83,8 @@ struct Sweep {
   int nbins;             // diag k-space: number of shells
   double shell_w;        // shell width
   double* hist;          // per-block shell histograms [gridDim][nbins]
+  const void* vd1;       // dynamic potential with z terms: its values at t1 and t2, [n^3] in
+  const void* vd2;       //   precision R (null: none), filled by k_point_table
   const int* live;       // batched imaginary-time instance: 0 = frozen (converged), its
                          // launches return at once; null: always advance
 };

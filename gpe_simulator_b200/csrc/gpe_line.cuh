@@ -119,6 +119,8 @@ struct LineCx {
   const R* c12;           // [L] (line parts at t1 and t2) dt/2 (shared; fused half-steps)
   const double2* kyz;     // [L] kinetic factor of the line, with 1/M (shared)
   const double* kyz2;     // [L] k_y^2 + k_z^2 of the line (shared)
+  const R* vd1;           // dynamic potential with z terms at t1 (t2), per point (global, null: none)
+  const R* vd2;
   long long row0;         // z tiles: global index of line 0
   int n;
 };
@@ -132,8 +134,9 @@ __device__ __forceinline__ typename Cx<R>::T line_half(const Phys& ph, const Lin
   const R rho = x.x * x.x + x.y * x.y;
   R V = TWO ? fma(cx.vz[m], h + h, cx.c12[l]) : cx.vz[m] + cx.c1[l];
   R g = (R)0;
+  const long long e = cx.row0 + (long long)l * cx.n + m;
+  if (cx.vd1) V = TWO ? fma(cx.vd1[e] + cx.vd2[e], h, V) : V + cx.vd1[e];
   if (ph.vre) {
-    const long long e = cx.row0 + (long long)l * cx.n + m;
     const R va = ((const R*)ph.vre)[e];
     V = TWO ? fma(va, h + h, V) : V + va;
     if (ph.vim) g = ((const R*)ph.vim)[e] * h;
@@ -176,6 +179,8 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   lc.vz = (const R*)ph.vax + 2 * n;
   lc.c1 = c1;
   lc.c12 = c12;
+  lc.vd1 = (const R*)sw.vd1;
+  lc.vd2 = (const R*)sw.vd2;
   lc.kyz = kyz;
   lc.kyz2 = kyz2;
   lc.n = n;
@@ -295,6 +300,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
           const double rho = (double)v[a].x * v[a].x + (double)v[a].y * v[a].y;
           R V = lc.vz[m] + c1[l];
           if (ph.vre) V += ((const R*)ph.vre)[lc.row0 + (long long)l * n + m];
+          if (lc.vd1) V += lc.vd1[lc.row0 + (long long)l * n + m];
           n0 += rho;
           n1 = fma((double)V, rho, n1);
           n2 = fma(rho, rho, n2);

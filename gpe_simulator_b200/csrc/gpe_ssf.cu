@@ -209,6 +209,76 @@ bool dynamic_line_form(const std::vector<double>& prog, std::vector<double>& lin
   return (int)line.size() <= GPE_PROGRAM_MAX;
 }
 
+// ---- dynamic potentials with z terms
+// Evaluated per point into a table by k_point_table.  Of the tree, maximal subtrees in t
+// alone become slots (host, per launch), subtrees in x, y (and t) one value per row of the
+// cube, subtrees in z (and t) one value per z; the rest is the residual program, run per
+// point.  Subtrees past a budget stay in the residual program as they are (a time that no
+// slot is left for then comes from a slot holding t itself).
+struct PointForm {
+  std::vector<std::vector<double>> slots, rows, zs;
+  std::vector<double> residual;
+};
+
+// Program of node i for one evaluation site; `site` 0: residual (rows and z values
+// hoisted), 1: inside a row or z program (only slots hoisted).
+void expr_emit_point(const std::vector<ExprNode>& nodes, int i, int site, std::vector<double>& out, PointForm& f) {
+  const ExprNode& nd = nodes[i];
+  auto plain = [&](int q) {
+    std::vector<double> sub;
+    expr_emit_plain(nodes, q, sub);
+    return sub;
+  };
+  if (nd.vars == 0 && nd.op != GPE_OP_CONST) {
+    out.push_back(GPE_OP_CONST);
+    out.push_back(host_eval(plain(i), 0.0, 0.0, 0.0, 0.0));
+    return;
+  }
+  // (the last slot is kept for t itself)
+  if (nd.vars == 8 && nd.op != GPE_OP_T && (int)f.slots.size() < GPE_LINE_SLOTS - 1) {
+    f.slots.push_back(plain(i));
+    out.push_back((double)(OP_SLOT0 + (int)f.slots.size() - 1));
+    return;
+  }
+  if (nd.op == GPE_OP_T) {
+    out.push_back((double)(OP_SLOT0 + GPE_LINE_SLOTS - 1));
+    return;
+  }
+  const bool leaf = nd.a < 0;
+  if (site == 0 && !leaf && nd.vars && !(nd.vars & 4) && (nd.vars & 3) && (int)f.rows.size() < GPE_POINT_TABS) {
+    std::vector<double> sub;
+    expr_emit_point(nodes, i, 1, sub, f);
+    f.rows.push_back(sub);
+    out.push_back((double)(OP_ROW0 + (int)f.rows.size() - 1));
+    return;
+  }
+  if (site == 0 && !leaf && (nd.vars & 4) && !(nd.vars & 3) && (int)f.zs.size() < GPE_POINT_TABS) {
+    std::vector<double> sub;
+    expr_emit_point(nodes, i, 1, sub, f);
+    f.zs.push_back(sub);
+    out.push_back((double)(OP_Z0 + (int)f.zs.size() - 1));
+    return;
+  }
+  if (nd.op == GPE_OP_POW && nodes[nd.b].vars == 0 && host_eval(plain(nd.b), 0.0, 0.0, 0.0, 0.0) == 2.0) {
+    expr_emit_point(nodes, nd.a, site, out, f);
+    out.push_back((double)OP_SQR);
+    return;
+  }
+  if (nd.a >= 0) expr_emit_point(nodes, nd.a, site, out, f);
+  if (nd.b >= 0) expr_emit_point(nodes, nd.b, site, out, f);
+  out.push_back((double)nd.op);
+  if (nd.op == GPE_OP_CONST) out.push_back(nd.val);
+}
+
+bool dynamic_point_form(const std::vector<double>& prog, PointForm& f) {
+  std::vector<ExprNode> nodes;
+  int root = -1;
+  if (!expr_tree(prog, nodes, root)) return false;
+  f = PointForm();
+  expr_emit_point(nodes, root, 0, f.residual, f);
+  return true;
+}
+
 // Validate a program: known opcodes, operands present, stack within bounds, one result.
 bool check_program(const double* p, int len, std::string& why) {
   if (len == 0) return true;
@@ -512,6 +582,97 @@ __global__ void k_fill_int(int* a, int n, int v) {
   if (i < n) a[i] = v;
 }
 
+// ---------------------------------------------------------------- dynamic potentials with z terms
+// Programs of one point form in a device array: rows, z values, residual.
+struct PointProg {
+  const double* base;
+  int nrow, nz;
+  int row_off[GPE_POINT_TABS], row_len[GPE_POINT_TABS];
+  int z_off[GPE_POINT_TABS], z_len[GPE_POINT_TABS];
+  int off, len;
+};
+
+constexpr int POINT_ROWS = 16;     // rows (x, y) of a block
+constexpr int POINT_LANES = 4;     // points a thread evaluates together
+
+// V(x, y, z, t) of every point at up to two times: blockIdx.y picks the time.  A block
+// evaluates its rows' values and the z values once (FP64, in shared memory), then runs the
+// residual program over its rows, four points per thread so that decoding an operation is
+// paid once for four.  Bound by FP64 issue and the residual's operations.  Before, the
+// whole program ran per point and half-step inside the Stockham z sweeps: five steps of a
+// formula moving a plug along z at 105^3 complex128 took 3518 us, now 528 us.
+template <typename R>
+__global__ void __launch_bounds__(128) k_point_table(PointProg pp, const double* __restrict__ x, int n,
+                                                     LineSlots sl, R* tab1, R* tab2) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ double sh[];
+  double* zt = sh;                                  // [nz][n]
+  double* rt = zt + (size_t)pp.nz * n;              // [nrow][POINT_ROWS]
+  double* prog = rt + (size_t)pp.nrow * POINT_ROWS; // residual program
+  const double* slots = blockIdx.y ? sl.s2 : sl.s1;
+  R* tab = blockIdx.y ? tab2 : tab1;
+  const int r0 = blockIdx.x * POINT_ROWS, nr = min(POINT_ROWS, n * n - r0);
+  for (int q = threadIdx.x; q < pp.nz * n; q += blockDim.x) {
+    const int k = q / n, z = q - k * n;
+    zt[q] = eval_program(pp.base + pp.z_off[k], pp.z_len[k], 0.0, 0.0, x[z], 0.0, slots);
+  }
+  for (int q = threadIdx.x; q < pp.nrow * nr; q += blockDim.x) {
+    const int k = q / nr, r = q - k * nr, g = r0 + r;
+    rt[k * POINT_ROWS + r] = eval_program(pp.base + pp.row_off[k], pp.row_len[k], x[g / n], x[g % n], 0.0, 0.0, slots);
+  }
+  for (int q = threadIdx.x; q < pp.len; q += blockDim.x) prog[q] = pp.base[pp.off + q];
+  __syncthreads();
+  // the sweep before may still read the table's previous values
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int per_row = (n + POINT_LANES - 1) / POINT_LANES;
+  for (int q = threadIdx.x; q < nr * per_row; q += blockDim.x) {
+    const int r = q / per_row, zq = q - r * per_row, g = r0 + r;
+    int z[POINT_LANES];                             // lanes a quarter row apart: coalesced stores
+#pragma unroll
+    for (int a = 0; a < POINT_LANES; ++a) z[a] = min(zq + a * per_row, n - 1);
+    double st[33][POINT_LANES];
+    int sp = 0;
+    for (int pc = 0; pc < pp.len;) {
+      const int op = (int)prog[pc++];
+      double* a = st[sp > 0 ? sp - 1 : 0];          // top of the stack
+      const double* b = a;
+      if (op >= 6 && op <= 10) { --sp; a = st[sp - 1]; b = st[sp]; }
+#define GPE_LANES(E) _Pragma("unroll") for (int i = 0; i < POINT_LANES; ++i) { E; }
+      switch (op) {
+        case 1: { const double c = prog[pc++]; GPE_LANES(st[sp][i] = c) ++sp; break; }
+        case 2: { const double c = x[g / n]; GPE_LANES(st[sp][i] = c) ++sp; break; }
+        case 3: { const double c = x[g % n]; GPE_LANES(st[sp][i] = c) ++sp; break; }
+        case 4: GPE_LANES(st[sp][i] = x[z[i]]) ++sp; break;
+        case 6: GPE_LANES(a[i] = a[i] + b[i]) break;
+        case 7: GPE_LANES(a[i] = a[i] - b[i]) break;
+        case 8: GPE_LANES(a[i] = a[i] * b[i]) break;
+        case 9: GPE_LANES(a[i] = a[i] / b[i]) break;
+        case 10: GPE_LANES(a[i] = pow(a[i], b[i])) break;
+        case 11: GPE_LANES(a[i] = -a[i]) break;
+        case 13: GPE_LANES(a[i] = sin(a[i])) break;
+        case 14: GPE_LANES(a[i] = cos(a[i])) break;
+        case 15: GPE_LANES(a[i] = tan(a[i])) break;
+        case 16: GPE_LANES(a[i] = exp(a[i])) break;
+        case 17: GPE_LANES(a[i] = sqrt(a[i])) break;
+        case 18: GPE_LANES(a[i] = tanh(a[i])) break;
+        case 19: GPE_LANES(a[i] = fabs(a[i])) break;
+        case 20: GPE_LANES(a[i] = log(a[i])) break;
+        case OP_SQR: GPE_LANES(a[i] = a[i] * a[i]) break;
+        default:
+          if (op >= OP_Z0) { GPE_LANES(st[sp][i] = zt[(op - OP_Z0) * n + z[i]]) }
+          else if (op >= OP_ROW0) { const double c = rt[(op - OP_ROW0) * POINT_ROWS + r]; GPE_LANES(st[sp][i] = c) }
+          else { const double c = slots[op - OP_SLOT0]; GPE_LANES(st[sp][i] = c) }
+          ++sp;
+          break;
+      }
+#undef GPE_LANES
+    }
+#pragma unroll
+    for (int a = 0; a < POINT_LANES; ++a)
+      if (zq + a * per_row < n) tab[(long long)g * n + zq + a * per_row] = (R)st[0][a];
+  }
+}
+
 // ---------------------------------------------------------------- image projections
 // The image outputs of the reference's save_outputs (gpe/save.py:59-90); out
 // arrays are n x n, row-major, at fftshifted indices for the momentum images.
@@ -622,6 +783,15 @@ struct gpe_plan {
   void* d_vim = nullptr;
   double* d_prog_g = nullptr;
   double* d_dyn = nullptr;
+  // dynamic potential with z terms: its point form, the programs on the device, and its
+  // values [2][n^3] at two times (pt_t; the first pt_n hold within the current call)
+  PointForm point;
+  bool has_point = false;
+  PointProg pprog{};
+  double* d_pprog = nullptr;
+  void* d_ptab = nullptr;
+  double pt_t[2] = {0.0, 0.0};
+  bool pt_ok[2] = {false, false};
   double* d_line = nullptr;
   void* d_ltab = nullptr;          // [2][n*n] per-line dynamic potential (line form), precision of psi
   void* d_tw = nullptr;
@@ -759,6 +929,59 @@ int line_table(gpe_plan* p, double t1, double t2, bool two, cudaStream_t st) {
   return GPE_OK;
 }
 
+// The point tables of the next z sweep: slots of d_ptab with the potential at t1 (and t2),
+// evaluating what the two slots do not hold yet in one launch.  Like the line table, inside
+// a step sequence a programmatic dependent of the sweep before it, and the z sweep after it
+// is one of it.
+int point_tables(gpe_plan* p, double t1, double t2, bool two, Sweep& sw, cudaStream_t st) {
+  auto find = [&](double t) { return p->pt_ok[0] && p->pt_t[0] == t ? 0 : p->pt_ok[1] && p->pt_t[1] == t ? 1 : -1; };
+  int a = find(t1), b = two ? find(t2) : -1;
+  const bool need_a = a < 0, need_b = two && b < 0 && !(t1 == t2);
+  if (need_a) a = b == 0 ? 1 : 0;
+  if (two && t1 == t2) b = a;
+  else if (need_b) b = 1 - a;
+  const size_t bytes = (size_t)p->n * p->n * p->n * (p->dtype == GPE_C64 ? 4 : 8);
+  char* tab = (char*)p->d_ptab;
+  if (need_a || need_b) {
+    LineSlots sl;
+    memset(&sl, 0, sizeof(sl));
+    auto fill = [&](double* s, double t) {
+      for (size_t k = 0; k < p->point.slots.size(); ++k) s[k] = host_eval(p->point.slots[k], 0.0, 0.0, 0.0, t);
+      s[GPE_LINE_SLOTS - 1] = t;
+    };
+    const int first = need_a ? a : b, second = need_a && need_b ? b : first;
+    fill(sl.s1, need_a ? t1 : t2);
+    fill(sl.s2, t2);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((p->n * p->n + POINT_ROWS - 1) / POINT_ROWS), need_a && need_b ? 2 : 1);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes =
+        ((size_t)p->pprog.nz * p->n + (size_t)p->pprog.nrow * POINT_ROWS + p->pprog.len) * sizeof(double);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
+    const cudaError_t e =
+        p->dtype == GPE_C64
+            ? cudaLaunchKernelEx(&cfg, k_point_table<float>, p->pprog, (const double*)p->d_x, p->n, sl,
+                                 (float*)(tab + first * bytes), (float*)(tab + second * bytes))
+            : cudaLaunchKernelEx(&cfg, k_point_table<double>, p->pprog, (const double*)p->d_x, p->n, sl,
+                                 (double*)(tab + first * bytes), (double*)(tab + second * bytes));
+    if (e != cudaSuccess) return fail(GPE_ERR_CUDA, std::string("point table: ") + cudaGetErrorString(e));
+    ++p->launches;
+    p->pdl_prev = p->pdl_chain;
+    if (need_a) { p->pt_t[a] = t1; p->pt_ok[a] = true; }
+    if (need_b) { p->pt_t[b] = t2; p->pt_ok[b] = true; }
+  }
+  // (outside a step sequence nothing is kept for a later call)
+  if (!p->pdl_chain) p->pt_ok[0] = p->pt_ok[1] = false;
+  sw.vd1 = tab + a * bytes;
+  sw.vd2 = two ? tab + b * bytes : sw.vd1;
+  return GPE_OK;
+}
+
 bool needs_lines(int mode) { return mode == FM_Z1 || mode == FM_Z2 || mode == FM_Z21 || mode == FM_DIAGR; }
 
 int sweep(gpe_plan* p, int ax, const Sweep& sw_in, cudaStream_t st) {
@@ -834,6 +1057,8 @@ const CUtensorMap* tma_maps(gpe_plan* p, const void* base, int fax) {
 int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   beam_centres(p, sw);
   if (p->d_ltab && needs_lines(op.mode)) TRY(line_table(p, sw.t1, sw.t2, op.mode == FM_Z21, st));
+  if (p->has_point && needs_lines(op.mode))
+    TRY(point_tables(p, sw.t1, sw.t2, op.mode == FM_Z21 || (op.mode == FM_Z1 && sw.t2 != 0.0), sw, st));
   sw.pp = p->pp;
   sw.tw = p->d_tw;
   sw.tw_lo = (const char*)p->d_tw + (size_t)p->n * p->csize;
@@ -948,8 +1173,8 @@ FastOps lz_ops(int mode) {
 // constants until their grid-dependency wait).
 struct PdlChain {
   gpe_plan* p;
-  explicit PdlChain(gpe_plan* q) : p(q) { p->pdl_chain = true; p->pdl_prev = false; p->sweep_dir = 0; }
-  ~PdlChain() { p->pdl_chain = false; p->pdl_prev = false; }
+  explicit PdlChain(gpe_plan* q) : p(q) { p->pdl_chain = true; p->pdl_prev = false; p->sweep_dir = 0; p->pt_ok[0] = p->pt_ok[1] = false; }
+  ~PdlChain() { p->pdl_chain = false; p->pdl_prev = false; p->pt_ok[0] = p->pt_ok[1] = false; }
 };
 
 Sweep mk_sweep(const void* src, void* dst) {
@@ -1009,6 +1234,21 @@ int ensure_hist(gpe_plan* p) {
   return GPE_OK;
 }
 
+// The point tables' memory: taken when the plan is made (a step then allocates nothing, as
+// under stream capture), and only where it is a small part of what is free; without it
+// the potential is evaluated per point in the Stockham sweeps.
+bool point_memory(gpe_plan* p) {
+  const size_t bytes = 2 * (size_t)p->n * p->n * p->n * (p->dtype == GPE_C64 ? 4 : 8);
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
+      cudaMalloc(&p->d_ptab, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    p->d_ptab = nullptr;
+    return false;
+  }
+  return true;
+}
+
 int fill_plan(gpe_plan* p, const gpe_desc* d) {
   const int n = d->n;
   if (n < 2 || n > 1024) return fail(GPE_ERR_UNSUPPORTED, "n must be in [2, 1024]");
@@ -1048,7 +1288,15 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
   // which carry that variant; keeping it out of the register-resident kernels keeps
   // their register budget)
   // a dynamic potential stays on them when none of its terms depends on z (line form)
-  const bool line_ok = d->dynamic_g_len == 0 || dynamic_line_form(p->prog_dyn, p->prog_line, p->slot_progs);
+  bool line_ok = d->dynamic_g_len == 0 || dynamic_line_form(p->prog_dyn, p->prog_line, p->slot_progs);
+  // ... and one with z terms through tables of its values per point (run-time-length sweeps);
+  // the programs' shared memory bounds the side it is used for
+  if (!line_ok) {
+    p->prog_line.clear();
+    p->slot_progs.clear();
+    p->has_point = dynamic_point_form(p->prog_dyn, p->point) &&
+                   (p->point.zs.size() * n + p->point.rows.size() * 16 + p->point.residual.size()) * 8 <= 48 * 1024;
+  }
   p->fixed = n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 160 || n == 256 ||
              (n == 512 && d->dtype == GPE_C64);
   {
@@ -1066,11 +1314,15 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
     // (a side of one radix has no exchange: the Stockham sweeps take it)
     p->line = p->ls[0].ok && p->ls[1].ok;
   }
+  p->has_point = p->has_point && p->line && d->generic_only != 1 && !(d->local_fp64 && d->dtype == GPE_C64) &&
+                 !d->exact_local;
+  if (p->has_point && point_memory(p)) { line_ok = true; p->fixed = false; }
+  else p->has_point = false;
   p->fast = (p->fixed || p->line) && d->generic_only != 1 && line_ok && !(d->local_fp64 && d->dtype == GPE_C64) &&
             !d->exact_local;
   if (!p->fast) { p->prog_line.clear(); p->slot_progs.clear(); }
-  p->plane = p->fast && d->dtype == GPE_C64 && (n == 128 || n == 256) && d->generic_only == 3;
-  p->tma = p->fast && d->dtype == GPE_C64 && (n == 128 || n == 256) && d->generic_only == 4;
+  p->plane = p->fast && p->fixed && d->dtype == GPE_C64 && (n == 128 || n == 256) && d->generic_only == 3;
+  p->tma = p->fast && p->fixed && d->dtype == GPE_C64 && (n == 128 || n == 256) && d->generic_only == 4;
   const int emax = 512 * p->ept;
   p->lt_yx = std::max(1, std::min(d->dtype == GPE_C64 ? 16 : 8, emax / n));
   p->lt_z = std::max(1, std::min(n * n, std::min(4096, emax) / n));
@@ -1216,7 +1468,7 @@ void free_plan(gpe_plan* p) {
   for (auto e : p->pool) cudaEventDestroy(e);
   void* bufs[] = {p->d_x, p->d_k, p->d_kin, p->d_kth, p->d_vax, p->d_vre, p->d_vim, p->d_prog_g, p->d_dyn, p->d_line, p->d_ltab,
                   p->d_tw, p->d_partial, p->d_ticket, p->d_scale, p->d_status, p->d_hist, p->d_out,
-                  p->d_work, p->d_plane, p->d_proj, p->ls[0].d_tw, p->ls[0].d_bf, p->ls[1].d_tw, p->ls[1].d_bf, p->d_twp};
+                  p->d_work, p->d_plane, p->d_proj, p->ls[0].d_tw, p->ls[0].d_bf, p->ls[1].d_tw, p->ls[1].d_bf, p->d_twp, p->d_pprog, p->d_ptab};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete p;
@@ -1225,7 +1477,7 @@ void free_plan(gpe_plan* p) {
 int create(const gpe_desc* d, gpe_plan** out) {
   gpe_plan* p = new gpe_plan();
   int rc = fill_plan(p, d);
-  if (rc != GPE_OK) { delete p; return rc; }
+  if (rc != GPE_OK) { free_plan(p); return rc; }
   const int n = p->n;
   CU(cudaMalloc(&p->d_x, n * sizeof(double)));
   CU(cudaMemcpy(p->d_x, p->x.data(), n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1254,6 +1506,23 @@ int create(const gpe_desc* d, gpe_plan** out) {
   if (!p->prog_dyn.empty()) {
     CU(cudaMalloc(&p->d_dyn, p->prog_dyn.size() * sizeof(double)));
     CU(cudaMemcpy(p->d_dyn, p->prog_dyn.data(), p->prog_dyn.size() * sizeof(double), cudaMemcpyHostToDevice));
+  }
+  if (p->has_point) {
+    std::vector<double> all;
+    PointProg& q = p->pprog;
+    auto put = [&](const std::vector<double>& v, int& off, int& len) {
+      off = (int)all.size();
+      len = (int)v.size();
+      all.insert(all.end(), v.begin(), v.end());
+    };
+    q.nrow = (int)p->point.rows.size();
+    q.nz = (int)p->point.zs.size();
+    for (int k = 0; k < q.nrow; ++k) put(p->point.rows[k], q.row_off[k], q.row_len[k]);
+    for (int k = 0; k < q.nz; ++k) put(p->point.zs[k], q.z_off[k], q.z_len[k]);
+    put(p->point.residual, q.off, q.len);
+    CU(cudaMalloc(&p->d_pprog, all.size() * sizeof(double)));
+    CU(cudaMemcpy(p->d_pprog, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice));
+    q.base = p->d_pprog;
   }
   if (!p->prog_line.empty()) {
     CU(cudaMalloc(&p->d_line, p->prog_line.size() * sizeof(double)));
@@ -1341,9 +1610,11 @@ int strang_step(gpe_plan* p, void* psi, double t, bool scaled, cudaStream_t st) 
 // Fast path, 5 sweeps: Z(half, fwd) Y(fwd) X(fwd, kin, inv) Y(inv) Z(inv, 1/M, half [, norm]).
 // With `fuse_next`, the last sweep also applies the next step's half-step and
 // forward z transform (real time), so the next step starts at its Y sweep.
-int fast_front(gpe_plan* p, void* psi, double t, bool scaled, cudaStream_t st) {
+// (t_next: the next step's time if the call has one, for the point tables; else 0)
+int fast_front(gpe_plan* p, void* psi, double t, bool scaled, cudaStream_t st, double t_next = 0.0) {
   Sweep s = mk_sweep(psi, psi);
   s.t1 = t;
+  s.t2 = t_next;
   return fsweep(p, AX_Z, s, mk_ops(FM_Z1, 0, 0, scaled ? 1 : 0), st);
 }
 
@@ -1681,7 +1952,8 @@ int gpe_step(gpe_plan* p, void* psi, int nsteps, long long step0, void* stream) 
   }
   if (p->fast && nsteps > 0) {
     // real time fuses each step's last z sweep with the next step's first
-    TRY(fast_front(p, psi, t_mid_host(p, step0), false, st));
+    TRY(fast_front(p, psi, t_mid_host(p, step0), false, st,
+                   p->has_point && nsteps > 1 ? t_mid_host(p, step0 + 1) : 0.0));
     for (int s = 0; s < nsteps; ++s) {
       const double t = t_mid_host(p, step0 + s);
       TRY(fast_middle(p, psi, st));
