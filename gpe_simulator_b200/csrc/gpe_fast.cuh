@@ -64,8 +64,10 @@ template <int N, typename R> struct FastCfg {
   static constexpr bool THREE = N == 512;
   static constexpr int P1 = L * N1, P2 = THREE ? P1 : L * N2;
   static constexpr bool POW2 = (N & (N - 1)) == 0 && N <= 512;
-  // power-of-two sizes: 16 values per thread; other sizes: one slot per thread per phase
-  static constexpr int T0 = POW2 ? L * N / 16 : cdiv(P1 > P2 ? P1 : P2, 32) * 32;
+  // power-of-two sizes from 128: 16 values per thread; other sizes: one slot per thread per
+  // phase (small grids have few warps, and a thread's values are its serial work: 64^3
+  // complex128 ran 16 values on 3.5 warps per SM)
+  static constexpr int T0 = POW2 && N >= 128 ? L * N / 16 : cdiv(P1 > P2 ? P1 : P2, 32) * 32;
   static constexpr int T = T0 < 32 ? 32 : T0;
   static constexpr int Q1 = cdiv(P1, T), Q2 = cdiv(P2, T);
   // registers (complex) per thread
@@ -384,7 +386,7 @@ __device__ __forceinline__ float expm1_series(float x) {
 // out of line, beyond.  Steps in use keep V dt/2 far inside the range; with the library
 // sincos and exp inlined per half-step, and two of them per fused z sweep, that sweep was
 // bound by FP64 issue.  Box and absorber at 256^3, 4 steps: 3260 -> 2634 us together with
-// the single rotation of the fused sweep (half_all).
+// the single rotation of the fused sweep (half_all), 2138 us with local_block.
 static __device__ __noinline__ void sin_cosm1_far(double x, double* s, double* cm1) {
   double sh, ch;
   sincos(0.5 * x, &sh, &ch);
@@ -392,48 +394,51 @@ static __device__ __noinline__ void sin_cosm1_far(double x, double* s, double* c
   *s = 2.0 * sh * ch;
 }
 static __device__ __noinline__ double exp_far(double x) { return exp(x); }
+__device__ __forceinline__ void sin_cosm1_near(double x, double& s, double& cm1) {   // |x| <= 1/2
+  const double z = x * x;
+  double a = -1.0 / 1307674368000.0, b = 1.0 / 20922789888000.0;
+  a = fma(a, z, 1.0 / 6227020800.0);
+  b = fma(b, z, -1.0 / 87178291200.0);
+  a = fma(a, z, -1.0 / 39916800.0);
+  b = fma(b, z, 1.0 / 479001600.0);
+  a = fma(a, z, 1.0 / 362880.0);
+  b = fma(b, z, -1.0 / 3628800.0);
+  a = fma(a, z, -1.0 / 5040.0);
+  b = fma(b, z, 1.0 / 40320.0);
+  a = fma(a, z, 1.0 / 120.0);
+  b = fma(b, z, -1.0 / 720.0);
+  a = fma(a, z, -1.0 / 6.0);
+  b = fma(b, z, 1.0 / 24.0);
+  b = fma(b, z, -0.5);
+  s = fma(a * z, x, x);
+  cm1 = b * z;
+}
 __device__ __forceinline__ void sin_cosm1_d(double x, double& s, double& cm1) {
-  if (fabs(x) <= 0.5) {
-    const double z = x * x;
-    double a = -1.0 / 1307674368000.0, b = 1.0 / 20922789888000.0;
-    a = fma(a, z, 1.0 / 6227020800.0);
-    b = fma(b, z, -1.0 / 87178291200.0);
-    a = fma(a, z, -1.0 / 39916800.0);
-    b = fma(b, z, 1.0 / 479001600.0);
-    a = fma(a, z, 1.0 / 362880.0);
-    b = fma(b, z, -1.0 / 3628800.0);
-    a = fma(a, z, -1.0 / 5040.0);
-    b = fma(b, z, 1.0 / 40320.0);
-    a = fma(a, z, 1.0 / 120.0);
-    b = fma(b, z, -1.0 / 720.0);
-    a = fma(a, z, -1.0 / 6.0);
-    b = fma(b, z, 1.0 / 24.0);
-    b = fma(b, z, -0.5);
-    s = fma(a * z, x, x);
-    cm1 = b * z;
-  } else {
-    sin_cosm1_far(x, &s, &cm1);
-  }
+  if (fabs(x) <= 0.5) sin_cosm1_near(x, s, cm1);
+  else sin_cosm1_far(x, &s, &cm1);
+}
+__device__ __forceinline__ double expm1_d(double x) {   // |x| <= 1/2
+  double a = 1.0 / 1307674368000.0;
+  a = fma(a, x, 1.0 / 87178291200.0);
+  a = fma(a, x, 1.0 / 6227020800.0);
+  a = fma(a, x, 1.0 / 479001600.0);
+  a = fma(a, x, 1.0 / 39916800.0);
+  a = fma(a, x, 1.0 / 3628800.0);
+  a = fma(a, x, 1.0 / 362880.0);
+  a = fma(a, x, 1.0 / 40320.0);
+  a = fma(a, x, 1.0 / 5040.0);
+  a = fma(a, x, 1.0 / 720.0);
+  a = fma(a, x, 1.0 / 120.0);
+  a = fma(a, x, 1.0 / 24.0);
+  a = fma(a, x, 1.0 / 6.0);
+  a = fma(a, x, 0.5);
+  return fma(a * x, x, x);
 }
 // v * exp(x): v + v*(exp(x) - 1) in the series' range, the product with exp itself beyond
 // (where exp - 1 would lose the relative accuracy of a small factor).
 __device__ __forceinline__ double2 mul_exp_d(double2 v, double x) {
   if (fabs(x) <= 0.5) {
-    double a = 1.0 / 1307674368000.0;
-    a = fma(a, x, 1.0 / 87178291200.0);
-    a = fma(a, x, 1.0 / 6227020800.0);
-    a = fma(a, x, 1.0 / 479001600.0);
-    a = fma(a, x, 1.0 / 39916800.0);
-    a = fma(a, x, 1.0 / 3628800.0);
-    a = fma(a, x, 1.0 / 362880.0);
-    a = fma(a, x, 1.0 / 40320.0);
-    a = fma(a, x, 1.0 / 5040.0);
-    a = fma(a, x, 1.0 / 720.0);
-    a = fma(a, x, 1.0 / 120.0);
-    a = fma(a, x, 1.0 / 24.0);
-    a = fma(a, x, 1.0 / 6.0);
-    a = fma(a, x, 0.5);
-    a = fma(a * x, x, x);
+    const double a = expm1_d(x);
     return make_double2(fma(v.x, a, v.x), fma(v.y, a, v.y));
   }
   const double f = exp_far(x);
@@ -564,6 +569,111 @@ template <bool ARR> __device__ __forceinline__ double two_density(double g) {
   return ARR ? (g == 0.0 ? 1.0 : 0.5 + 0.5 * exp_far(g + g)) : 1.0;
 }
 
+// Values in the reach of the short series, and those series, by precision.
+__device__ __forceinline__ bool in_reach(double x) { return fabs(x) <= 0.5; }
+__device__ __forceinline__ bool in_reach(float x) { return fabsf(x) <= 0.125f; }
+__device__ __forceinline__ void sin_cosm1_reach(double x, double& s, double& c) { sin_cosm1_near(x, s, c); }
+__device__ __forceinline__ void sin_cosm1_reach(float x, float& s, float& c) { sin_cosm1_tiny(x, s, c); }
+__device__ __forceinline__ double expm1_reach(double x) { return expm1_d(x); }
+__device__ __forceinline__ float expm1_reach(float x) { return expm1_tiny(x); }
+// one element beyond them: v exp(-i p), v exp(p)
+__device__ __forceinline__ double2 rotate_by(double2 x, double p) { return rotate_d(x, p); }
+__device__ __forceinline__ double2 decay_by(double2 x, double p) { return mul_exp_d(x, p); }
+static __device__ __noinline__ float2 rotate_far(float2 x, float p) {
+  float sn, cm1;
+  if (fabsf(p) <= 0.78539816f) {
+    sin_cosm1_series(p, sn, cm1);
+  } else {
+    float sh, ch;
+    sincosf(0.5f * p, &sh, &ch);
+    cm1 = -2.0f * sh * sh;
+    sn = 2.0f * sh * ch;
+  }
+  return make_float2(fmaf(x.x, cm1, fmaf(x.y, sn, x.x)), fmaf(x.y, cm1, fmaf(-x.x, sn, x.y)));
+}
+static __device__ __noinline__ float2 decay_far(float2 x, float p) {
+  const float em = fabsf(p) <= 0.5f ? expm1_series(p) : expm1f(p);
+  return make_float2(fmaf(x.x, em, x.x), fmaf(x.y, em, x.y));
+}
+__device__ __forceinline__ float2 rotate_by(float2 x, float p) {
+  if (!in_reach(p)) return rotate_far(x, p);
+  float sn, cm1;
+  sin_cosm1_tiny(p, sn, cm1);
+  return make_float2(fmaf(x.x, cm1, fmaf(x.y, sn, x.x)), fmaf(x.y, cm1, fmaf(-x.x, sn, x.y)));
+}
+__device__ __forceinline__ float2 decay_by(float2 x, float p) {
+  if (!in_reach(p)) return decay_far(x, p);
+  const float em = expm1_tiny(p);
+  return make_float2(fmaf(x.x, em, x.x), fmaf(x.y, em, x.y));
+}
+
+// The local half-step of U elements with potentials V and gain/loss g (ARR), TWO as below.
+// One test of the phases for all of them, then straight code: the U series run interleaved,
+// where a test per element ran them one after the other, each a chain of a dozen dependent
+// operations, and kept the loads of array potentials from being issued together.  Box and
+// absorber at 256^3 complex128, 4 steps: 2662 -> 2138 us; 64^3 complex128 imaginary time,
+// with one slot of 8 values per thread (FastCfg), 50 steps: 2143 -> 1518 us.
+template <typename R, bool ARR, bool TWO, int U>
+__device__ __forceinline__ void local_block(typename Cx<R>::T* v, const R (&V)[U], const R (&g)[U], bool real, R beta,
+                                            R h) {
+  using C = typename Cx<R>::T;
+  R p[U], em[U], rho[U];
+  // (complex64: the short series are short, and its sweeps run at twice the warps with half
+  // the registers: one element after the other)
+  bool near = sizeof(R) == 8, lossy = false;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    rho[u] = v[u].x * v[u].x + v[u].y * v[u].y;
+    em[u] = (R)0;
+    if (ARR && sizeof(R) == 8) {
+      lossy = lossy || g[u] != (R)0;
+      near = near && in_reach(TWO ? g[u] + g[u] : g[u]);
+    }
+  }
+  if (ARR && lossy && near) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) em[u] = expm1_reach(TWO ? g[u] + g[u] : g[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    p[u] = TWO ? fma(ARR ? fma((R)0.5 * em[u], beta, beta) : beta, rho[u], V[u]) : (V[u] + beta * rho[u]) * h;
+    near = near && in_reach(p[u]);
+  }
+  if (sizeof(R) == 8 && near) {
+    if (real) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const C x = v[u];
+        R sn, cm1;
+        sin_cosm1_reach(p[u], sn, cm1);
+        v[u] = mk(fma(x.x, cm1, fma(x.y, sn, x.x)), fma(x.y, cm1, fma(-x.x, sn, x.y)));
+      }
+      if (ARR && lossy) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = mk(fma(v[u].x, em[u], v[u].x), fma(v[u].y, em[u], v[u].y));
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const R e = expm1_reach(-p[u]);
+        v[u] = mk(fma(v[u].x, e, v[u].x), fma(v[u].y, e, v[u].y));
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (!real) { v[u] = decay_by(v[u], -(V[u] + beta * rho[u]) * h); continue; }
+    const R q = TWO ? fma(ARR && g[u] != (R)0 ? beta * two_density<ARR>(g[u]) : beta, rho[u], V[u])
+                    : (V[u] + beta * rho[u]) * h;
+    v[u] = rotate_by(v[u], q);
+    if (ARR) { if (g[u] != (R)0) v[u] = decay_by(v[u], TWO ? g[u] + g[u] : g[u]); }
+  }
+}
+
+// elements per local_block: the largest of 5, 4, 3, 2 that divides n (1: none does)
+constexpr int local_unroll(int n) { return n % 4 == 0 ? 4 : n % 5 == 0 ? 5 : n % 3 == 0 ? 3 : n % 2 == 0 ? 2 : 1; }
+
 // One local half-step over all registers (layout LANES x VALS, element m = lane +
 // LANES*a, Z tiles: m = z index), potential vz[m] + ctab[l] (+ arrays).  complex64:
 // each element whose phase is within the short series' range (|phase| <= 1/8,
@@ -585,6 +695,34 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
                                          const Phys& ph, const FastTables<R>& tb, const R* ctab,
                                          R beta, R h) {
   constexpr int L = FastCfg<N, R>::L, T = FastCfg<N, R>::T;
+  if constexpr (sizeof(R) == 8) {
+    constexpr int U = local_unroll(VALS);
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      if (!slot_ok<N, R, LANES, SLOTS>(s)) break;
+      int l, lane;
+      slot<AX, L, T>(threadIdx.x + s * T, LANES, l, lane);
+      const long long row = tl.base + (long long)l * tl.lstride;
+      const R c = ctab[l];
+#pragma unroll
+      for (int a0 = 0; a0 < VALS; a0 += U) {
+        R V[U], g[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int m = lane + LANES * (a0 + u);
+          V[u] = tb.vz[m] + c;
+          g[u] = (R)0;
+          if (ARR) {
+            const R va = ph.vre ? ((const R*)ph.vre)[row + m] : (R)0;
+            V[u] = TWO ? fma(va, h + h, V[u]) : V[u] + va;
+            g[u] = ph.vim ? ((const R*)ph.vim)[row + m] * h : (R)0;
+          }
+        }
+        local_block<R, ARR, TWO, U>(v + s * VALS + a0, V, g, REAL, beta, h);
+      }
+    }
+    return;
+  }
   static_assert(SLOTS * VALS <= 64, "pending mask");
   // complex64: elements whose phase exceeds the short series' range
   using Mask = typename std::conditional<(SLOTS * VALS <= 32), unsigned, unsigned long long>::type;
@@ -609,15 +747,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
       const typename Cx<R>::T x = v[e];
       const R phs = TWO ? fma(beta * two_density<ARR>(g), x.x * x.x + x.y * x.y, V)
                         : (V + beta * (x.x * x.x + x.y * x.y)) * h;
-      if constexpr (sizeof(R) == 8) {
-        if (!REAL) {
-          v[e] = mul_exp_d(x, -phs);
-        } else {
-          v[e] = rotate_d(x, phs);
-          // (g is zero away from the absorbers: whole warps skip its exponential)
-          if (ARR) { if (g != 0.0) v[e] = mul_exp_d(v[e], TWO ? 2.0 * g : g); }
-        }
-      } else if (fabs(phs) <= (R)0.125) {
+      if (fabs(phs) <= (R)0.125) {
         if (!REAL) {
           const float em = expm1_tiny((float)-phs);
           v[e] = mk(fma(x.x, (R)em, x.x), fma(x.y, (R)em, x.y));
@@ -632,7 +762,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
       }
     }
   }
-  if (sizeof(R) == 8 || !__any_sync(0xffffffffu, pend != 0)) return;
+  if (!__any_sync(0xffffffffu, pend != 0)) return;
   // second pass over the elements left unrotated: full series up to pi/4 (1/2 in
   // imaginary time), library functions beyond
 #pragma unroll

@@ -490,6 +490,7 @@ static __device__ void norm_finish_n(const Phys& ph, const Sweep& sw, Acc total,
   if (!last) return;
   __threadfence();
   Acc a[1];
+#pragma unroll 8
   for (int b = threadIdx.x; b < count; b += blockDim.x) a[0].add(__ldcg(sw.partial + b));
   block_merge<1>(a, sh);
   if (threadIdx.x == 0) {

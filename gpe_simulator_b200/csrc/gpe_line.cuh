@@ -27,7 +27,7 @@
 // Against the Stockham sweeps these replace (run-time strides and divisions per element,
 // every stage through shared memory, five sweeps per step instead of four): 200^3
 // complex64, 6 imaginary-time steps 7343 -> 1472 us; 512^3 complex128, one stirred step
-// 24.6 -> 6.78 ms; 294^3 complex64 with array potentials, 2 steps 14.0 -> 1.84 ms.  Bound
+// 24.6 -> 6.09 ms; 294^3 complex64 with array potentials, 2 steps 14.0 -> 1.84 ms.  Bound
 // by the latency of the loads and barriers at 16 (complex128) and 32 (complex64) warps per
 // SM and, in complex64, by issue.
 #pragma once
@@ -79,38 +79,6 @@ template <int RAD, bool DIRECT, typename C> __device__ __forceinline__ void line
 }
 
 // ---------------------------------------------------------------- pointwise physics
-// Rotations and decays beyond the short series (rare), out of line.
-static __device__ __noinline__ float2 rotate_far(float2 x, float p) {
-  float sn, cm1;
-  if (fabsf(p) <= 0.78539816f) {
-    sin_cosm1_series(p, sn, cm1);
-  } else {
-    float sh, ch;
-    sincosf(0.5f * p, &sh, &ch);
-    cm1 = -2.0f * sh * sh;
-    sn = 2.0f * sh * ch;
-  }
-  return make_float2(fmaf(x.x, cm1, fmaf(x.y, sn, x.x)), fmaf(x.y, cm1, fmaf(-x.x, sn, x.y)));
-}
-static __device__ __noinline__ float2 decay_far(float2 x, float p) {
-  const float em = fabsf(p) <= 0.5f ? expm1_series(p) : expm1f(p);
-  return make_float2(fmaf(x.x, em, x.x), fmaf(x.y, em, x.y));
-}
-// v exp(-i p) and v exp(p)
-__device__ __forceinline__ float2 rotate_by(float2 x, float p) {
-  if (!(fabsf(p) <= 0.125f)) return rotate_far(x, p);
-  float sn, cm1;
-  sin_cosm1_tiny(p, sn, cm1);
-  return make_float2(fmaf(x.x, cm1, fmaf(x.y, sn, x.x)), fmaf(x.y, cm1, fmaf(-x.x, sn, x.y)));
-}
-__device__ __forceinline__ float2 decay_by(float2 x, float p) {
-  if (!(fabsf(p) <= 0.125f)) return decay_far(x, p);
-  const float em = expm1_tiny(p);
-  return make_float2(fmaf(x.x, em, x.x), fmaf(x.y, em, x.y));
-}
-__device__ __forceinline__ double2 rotate_by(double2 x, double p) { return rotate_d(x, p); }
-__device__ __forceinline__ double2 decay_by(double2 x, double p) { return mul_exp_d(x, p); }
-
 // What the pointwise stages of one tile need besides Phys.
 template <typename R>
 struct LineCx {
@@ -125,32 +93,39 @@ struct LineCx {
   int n;
 };
 
-// One local half-step of element m of line l (TWO: two consecutive real-time half-steps
-// as one rotation, see half_all in gpe_fast.cuh for why that is exact).
-template <typename R, bool TWO>
-__device__ __forceinline__ typename Cx<R>::T line_half(const Phys& ph, const LineCx<R>& cx, typename Cx<R>::T x,
-                                                       int l, int m) {
-  const R h = (R)(ph.dt * 0.5);
-  const R rho = x.x * x.x + x.y * x.y;
-  R V = TWO ? fma(cx.vz[m], h + h, cx.c12[l]) : cx.vz[m] + cx.c1[l];
-  R g = (R)0;
-  const long long e = cx.row0 + (long long)l * cx.n + m;
-  if (cx.vd1) V = TWO ? fma(cx.vd1[e] + cx.vd2[e], h, V) : V + cx.vd1[e];
-  if (ph.vre) {
-    const R va = ((const R*)ph.vre)[e];
-    V = TWO ? fma(va, h + h, V) : V + va;
-    if (ph.vim) g = ((const R*)ph.vim)[e] * h;
+// One local half-step of the RAD elements m = q + a*nb of line l (TWO: two consecutive
+// real-time half-steps as one rotation, see half_all in gpe_fast.cuh for why that is
+// exact), a few at a time with their potentials loaded together.
+template <typename R, bool ARR, bool TWO, int RAD>
+__device__ __forceinline__ void line_half_arr(const Phys& ph, const LineCx<R>& cx, typename Cx<R>::T (&v)[RAD], int l,
+                                              int q, int nb) {
+  constexpr int U = sizeof(R) == 8 || ARR ? local_unroll(RAD) : 1;
+  const R h = (R)(ph.dt * 0.5), beta = TWO ? (R)(2.0 * ph.beta) * h : (R)ph.beta;
+  const R c = TWO ? cx.c12[l] : cx.c1[l];
+  const long long row = cx.row0 + (long long)l * cx.n + q;
+#pragma unroll
+  for (int a0 = 0; a0 < RAD; a0 += U) {
+    R V[U], g[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const R vz = cx.vz[q + (a0 + u) * nb];
+      V[u] = TWO ? fma(vz, h + h, c) : vz + c;
+      g[u] = (R)0;
+      if (ARR) {
+        const long long e = row + (a0 + u) * nb;
+        if (cx.vd1) V[u] = TWO ? fma(cx.vd1[e] + cx.vd2[e], h, V[u]) : V[u] + cx.vd1[e];
+        if (ph.vre) V[u] = TWO ? fma(((const R*)ph.vre)[e], h + h, V[u]) : V[u] + ((const R*)ph.vre)[e];
+        if (ph.vim) g[u] = ((const R*)ph.vim)[e] * h;
+      }
+    }
+    local_block<R, ARR, TWO, U>(v + a0, V, g, TWO || ph.kind == 1, beta, h);
   }
-  if (TWO) {
-    R b = (R)(2.0 * ph.beta) * h;
-    if (g != (R)0) b *= two_density<true>(g);
-    x = rotate_by(x, fma(b, rho, V));
-    return g != (R)0 ? decay_by(x, g + g) : x;
-  }
-  const R p = (V + (R)ph.beta * rho) * h;
-  if (ph.kind == 0) return decay_by(x, -p);
-  x = rotate_by(x, p);
-  return g != (R)0 ? decay_by(x, g) : x;
+}
+template <typename R, bool TWO, int RAD>
+__device__ __forceinline__ void line_half(const Phys& ph, const LineCx<R>& cx, typename Cx<R>::T (&v)[RAD], int l,
+                                          int q, int nb) {
+  if (ph.vre || cx.vd1) line_half_arr<R, true, TWO, RAD>(ph, cx, v, l, q, nb);
+  else line_half_arr<R, false, TWO, RAD>(ph, cx, v, l, q, nb);
 }
 
 // ---------------------------------------------------------------- the sweep
@@ -162,7 +137,8 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   constexpr bool TWO_FFT = MODE == FM_Z21 || MODE == FM_XKIN;
   constexpr bool ZM = MODE == FM_Z1 || MODE == FM_Z2 || MODE == FM_Z21 || MODE == FM_DIAGR;
   // one transform: twiddles before the phases; direct prime sums only exist in complex64
-  constexpr bool DIT = !TWO_FFT, DIRECT = DIT && sizeof(R) == 4;
+  constexpr bool DIT = !TWO_FFT;
+  constexpr bool DIRECT = sizeof(R) == 4 && DIT && MODE != FM_Z1 && MODE != FM_Z2;
   constexpr bool SUMS = MODE == FM_DIAGR || MODE == FM_DIAGK || MODE == FM_LZ;
   griddep_launch_dependents();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -289,8 +265,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
             }
           }
         }
-#pragma unroll
-        for (int a = 0; a < RAD; ++a) v[a] = line_half<R, false>(ph, lc, v[a], l, q + a * nb);
+        line_half<R, false, RAD>(ph, lc, v, l, q, nb);
       }
       if (MODE == FM_DIAGR) {
         double n0 = 0.0, n1 = 0.0, n2 = 0.0;
@@ -370,7 +345,8 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       if (TWO_FFT) {
         if (MODE == FM_Z21) {
 #pragma unroll
-          for (int a = 0; a < RAD; ++a) v[a] = line_half<R, true>(ph, lc, conj_<R>(v[a]), l, q + a * nb);
+          for (int a = 0; a < RAD; ++a) v[a].y = -v[a].y;
+          line_half<R, true, RAD>(ph, lc, v, l, q, nb);
         } else {
           const double2 fl = kyz[l];
 #pragma unroll
@@ -401,8 +377,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
           for (int a = 0; a < RAD; ++a) { v[a].x *= (R)ph.inv_m; v[a].y *= (R)ph.inv_m; }
         }
         if (MODE == FM_Z2) {
-#pragma unroll
-          for (int a = 0; a < RAD; ++a) v[a] = line_half<R, false>(ph, lc, v[a], l, q + a * nb);
+          line_half<R, false, RAD>(ph, lc, v, l, q, nb);
           if (op.norm) {
             double sum = 0.0;
 #pragma unroll
@@ -501,6 +476,8 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   }
 }
 
+// Resident blocks: 64 registers in complex64 (80 measured slower: 200^3 236 -> 261 us per
+// step), 128 in complex128.
 template <typename R> struct LineBounds { static constexpr int blocks = sizeof(R) == 4 ? 4 : 2; };
 
 template <typename R, bool ZT, int MODE>
