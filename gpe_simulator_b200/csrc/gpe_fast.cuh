@@ -119,11 +119,10 @@ template <int N, typename R> __host__ __device__ constexpr size_t fast_tables_by
          / 16 * 16;
 }
 
-// the same at run time (host): the shell histogram of a diagnostic x sweep lives
-// in the tables region, so it holds at most this many bytes of bins
-inline size_t fast_tables_bytes_rt(int n, int real_bytes) {
-  const int L = fast_lines(n, real_bytes);
-  return (((size_t)(n + L) * (16 + 8) + (size_t)(n + 3 * L) * real_bytes) + 15) / 16 * 16;
+// bytes of the exchange buffer at run time (host; without its padding): the shell histogram
+// of a diagnostic x sweep takes it, so it holds at most this many bytes of bins
+inline size_t fast_hist_bytes_rt(int n, int real_bytes) {
+  return (size_t)fast_lines(n, real_bytes) * n * 2 * real_bytes;
 }
 
 // shared memory of a fast sweep (bytes)
@@ -500,6 +499,25 @@ __device__ __forceinline__ void z_tables(const Phys& ph, const Sweep& sw, int a0
   }
 }
 
+// Tables of the diagnostic z sweep: the line's static part and its beam's exponential, as
+// potential() rounds them.
+template <int N, typename R>
+__device__ __forceinline__ void diag_tables(const Phys& ph, const Sweep& sw, int a0, FastTables<R>& tb) {
+  constexpr int L = FastCfg<N, R>::L, T = FastCfg<N, R>::T;
+  const R* vax = (const R*)ph.vax;
+  for (int q = threadIdx.x; q < N; q += T) tb.vz[q] = vax[2 * N + q];
+  for (int l = threadIdx.x; l < L; l += T) {
+    const int g = a0 + l, i = g / N, j = g % N;
+    tb.c1[l] = vax[i] + vax[N + j];
+    if (ph.kind == 1 && ph.beam) {
+      const R dx = (R)(ph.x[i] - sw.bc1x), dy = (R)(ph.x[j] - sw.bc1y);
+      tb.c2[l] = rexp(-(dx * dx + dy * dy) * (R)ph.beam_inv_w2);
+    } else {
+      tb.c2[l] = (R)0;
+    }
+  }
+}
+
 template <int N, typename R, int T = FastCfg<N, R>::T>
 __device__ __forceinline__ void x_tables(const Phys& ph, int j, int k0, FastTables<R>& tb) {
   constexpr int L = FastCfg<N, R>::L;
@@ -837,14 +855,14 @@ __device__ __forceinline__ void diag_real_all(const typename Cx<R>::T (&v)[EPT],
 #pragma unroll
     for (int a = 0; a < VALS; ++a) {
       const int m = lane + LANES * a;
-      int i, j, k;
-      tl.coords(l, m, i, j, k);
       const typename Cx<R>::T x = v[s * VALS + a];
       const double rho = (double)x.x * x.x + (double)x.y * x.y;
-      // with a line program the potential comes from the z-sweep tables (static
-      // axes and line terms at t1), plus the static array
-      const double V = ph.ltab ? (double)(tb.vz[m] + tb.c1[l] + (ph.vre ? ((const R*)ph.vre)[tl.gidx(l, m)] : (R)0))
-                                : (double)potential<R>(ph, N, i, j, k, tl.gidx(l, m), cx.t1, cx.b1x, cx.b1y);
+      // the potential from the tables: with a line program those of the z sweeps (static axes
+      // and line terms at t1), else the terms of potential() in its order
+      R Vr = tb.vz[m] + tb.c1[l];
+      if (ph.vre) Vr += ((const R*)ph.vre)[tl.gidx(l, m)];
+      if (!ph.ltab && ph.beam) Vr += (R)ph.beam_amp * tb.c2[l];
+      const double V = (double)Vr;
       n0 += rho;
       n1 = fma(V, rho, n1);
       n2 = fma(rho, rho, n2);
@@ -878,11 +896,9 @@ __device__ __forceinline__ void diag_k_all(const typename Cx<R>::T (&v)[EPT], co
       const double kk = kk_ref(ph.k[i], ph.k[j], ph.k[k]);
       const double w = (double)x.x * x.x + (double)x.y * x.y;
       e = fma(kk, w, e);
-      if (cx.hist) {
-        int sh = (int)floor(sqrt(kk) / cx.shell_w + 0.5);
-        sh = min(sh, cx.nbins - 1);
-        atomicAdd(cx.hist + sh, w);
-      }
+      if (cx.hist)
+        atomicAdd(cx.hist + (threadIdx.x & (cx.copies - 1)) * cx.nbins +
+                      shell_of(kk, cx.shell_t, cx.inv_shell, cx.nbins), w);
     }
     cx.acc[3].add(e);
   }
@@ -1064,9 +1080,7 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
     if (ZM || (MODE == FM_DIAGR && ph.ltab))
       z_tables<N, R>(ph, sw, tl.a0, tb, MODE == FM_Z21, MODE == FM_Z21);
     if (MODE == FM_XKIN) x_tables<N, R>(ph, tl.a0, tl.b0, tb);
-    // diagnostic x sweep: the shell histogram takes the tables region
-    if (MODE == FM_DIAGK && sw.hist)
-      for (int b = threadIdx.x; b < sw.nbins; b += T) ((double*)tail)[b] = 0.0;
+    if (MODE == FM_DIAGR && !ph.ltab) diag_tables<N, R>(ph, sw, tl.a0, tb);
   };
   // psi and the renormalisation scale come from the previous sweep: read them
   // after the grid-dependency wait; the tile's loads are issued first and are in
@@ -1087,9 +1101,12 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
     cx.b1y = sw.bc1y;
   }
   if (MODE == FM_DIAGK) {
-    cx.hist = sw.hist ? (double*)tail : nullptr;
+    // the shell histograms take the exchange buffer once the transform is done with it
+    cx.hist = sw.hist ? (double*)ex : nullptr;
     cx.nbins = sw.nbins;
-    cx.shell_w = sw.shell_w;
+    cx.shell_t = sw.shell_t;
+    cx.inv_shell = sw.inv_shell;
+    cx.copies = hist_copies(sw.nbins, fast_exchange_elems<N, R>() * sizeof(C));
   }
 
   C v[EPT];
@@ -1121,7 +1138,14 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
     if (MODE == FM_Z2 || (MODE == FM_PLAIN && op.inv1)) conj_all(v);
     if (MODE == FM_Z2) fast_pointwise<N, AX, R, MODE, 2, LM, VM, SM>(v, tl, ph, tb, op, cx);
     if (MODE == FM_PLAIN && op.invm) scale_all(v, (R)ph.inv_m);
-    if (MODE == FM_DIAGK) diag_k_all<N, AX, R, LM, VM, SM>(v, tl, ph, cx);
+    if (MODE == FM_DIAGK) {
+      if (cx.hist) {
+        __syncthreads();
+        for (int b = threadIdx.x; b < cx.copies * cx.nbins; b += T) cx.hist[b] = 0.0;
+        __syncthreads();
+      }
+      diag_k_all<N, AX, R, LM, VM, SM>(v, tl, ph, cx);
+    }
     else fast_store<N, AX, R, LM, VM, SM>(v, tl, (C*)sw.dst);
   }
   if (MODE == FM_Z2 && op.norm) {
@@ -1137,7 +1161,11 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
       for (int q = 0; q < 4; ++q) sw.partial[(long long)tile * 4 + q] = a[q].value();
     if (MODE == FM_DIAGK && sw.hist) {
       __syncthreads();
-      for (int b = threadIdx.x; b < sw.nbins; b += T) sw.hist[(long long)tile * sw.nbins + b] = cx.hist[b];
+      for (int b = threadIdx.x; b < sw.nbins; b += T) {
+        double h = cx.hist[b];
+        for (int c = 1; c < cx.copies; ++c) h += cx.hist[c * cx.nbins + b];
+        sw.hist[(long long)tile * sw.nbins + b] = h;
+      }
     }
   }
 }

@@ -83,6 +83,8 @@ struct Sweep {
   int nbins;             // diag k-space: number of shells
   double shell_w;        // shell width
   double* hist;          // per-block shell histograms [gridDim][nbins]
+  const double* shell_t; // [nbins] least k^2 of each shell (shell_of)
+  float inv_shell;       // 1 / shell width, rounded
   const void* vd1;       // dynamic potential with z terms: its values at t1 and t2, [n^3] in
   const void* vd2;       //   precision R (null: none), filled by k_point_table
   const int* live;       // batched imaginary-time instance: 0 = frozen (converged), its
@@ -144,9 +146,11 @@ struct Acc {
   __device__ __forceinline__ double value() const { return s + c; }
 };
 
-__device__ __forceinline__ Acc warp_merge(Acc a) {
+// (first: half the lanes that hold values, as a power of two; the others add zeros)
+__device__ __forceinline__ Acc warp_merge(Acc a, int first = 16) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
+    if (o > first) continue;
     Acc b;
     b.s = __shfl_xor_sync(0xffffffffu, a.s, o);
     b.c = __shfl_xor_sync(0xffffffffu, a.c, o);
@@ -167,11 +171,14 @@ __device__ void block_merge(Acc (&a)[NV], Acc* sh /* [32*NV] */) {
     for (int v = 0; v < NV; ++v) sh[w * NV + v] = a[v];
   __syncthreads();
   if (w == 0) {
+    // (a merge is eight dependent FP64 operations: small blocks skip the rounds over lanes
+    // that hold no warp's sum)
+    const int first = nw > 16 ? 16 : nw > 8 ? 8 : nw > 4 ? 4 : nw > 2 ? 2 : nw > 1 ? 1 : 0;
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       Acc b;
       if (lane < nw) b = sh[lane * NV + v];
-      a[v] = warp_merge(b);
+      a[v] = warp_merge(b, first);
     }
   }
   __syncthreads();
@@ -368,6 +375,23 @@ __device__ __forceinline__ double kk_ref(double kx, double ky, double kz) {
   return __dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kz, kz));
 }
 
+// Shell of k^2, min(floor(sqrt(kk)/w + 0.5), nbins - 1) in FP64 as NumPy evaluates it, without
+// its square root and division: that expression never decreases with kk, so the host finds
+// the least double of every shell (t[b]); an FP32 estimate lands within a shell of the answer
+// and is corrected against those.
+__device__ __forceinline__ int shell_of(double kk, const double* __restrict__ t, float inv_w, int nbins) {
+  int b = min((int)fmaf(sqrtf((float)kk), inv_w, 0.5f), nbins - 1);
+  while (b + 1 < nbins && kk >= __ldg(t + b + 1)) ++b;
+  while (b > 0 && kk < __ldg(t + b)) --b;
+  return b;
+}
+// Copies of a shared shell histogram: neighbouring lanes, whose values mostly share a shell,
+// add to different copies (an FP64 shared-memory atomic is a compare-and-swap loop that
+// repeats for every lane it collides with).
+__host__ __device__ constexpr int hist_copies(int nbins, size_t bytes) {
+  return (size_t)nbins * 64 <= bytes ? 8 : (size_t)nbins * 32 <= bytes ? 4 : (size_t)nbins * 16 <= bytes ? 2 : 1;
+}
+
 // Per-point pointwise stage.
 template <typename R>
 struct PwCtx {
@@ -379,6 +403,9 @@ struct PwCtx {
   double* hist;               // shared-memory shell histogram (PW_DIAG_K)
   int nbins;
   double shell_w;
+  const double* shell_t;      // register-resident sweeps: shell_of's arguments, histogram copies
+  float inv_shell;
+  int copies;
 };
 
 template <typename R>

@@ -193,7 +193,13 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       const R* vax = (const R*)ph.vax;
       const R stat = vax[i] + vax[n + j];
       R b1 = (R)0, b2 = (R)0;
-      if (ph.kind == 1 && ph.beam) {
+      if (MODE == FM_DIAGR) {
+        // (the beam's exponential apart: potential() adds it after the arrays)
+        if (ph.kind == 1 && ph.beam) {
+          const R dx = (R)(ph.x[i] - sw.bc1x), dy = (R)(ph.x[j] - sw.bc1y);
+          c12[l] = rexp(-(dx * dx + dy * dy) * (R)ph.beam_inv_w2);
+        }
+      } else if (ph.kind == 1 && ph.beam) {
         const R dx = (R)(ph.x[i] - sw.bc1x), dy = (R)(ph.x[j] - sw.bc1y), iw = (R)ph.beam_inv_w2;
         b1 = (R)ph.beam_amp * rexp(-dx * dx * iw) * rexp(-dy * dy * iw);
         if (MODE == FM_Z21) {
@@ -218,8 +224,9 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       kyz2[l] = ph.k[a0] * ph.k[a0] + ph.k[z0 + l] * ph.k[z0 + l];
     }
   }
-  if (MODE == FM_DIAGK && sw.hist)
-    for (int b = tid; b < sw.nbins; b += T) hist[b] = 0.0;
+  const int copies = MODE == FM_DIAGK && sw.hist ? hist_copies(sw.nbins, LINE_HIST) : 0;
+  if (MODE == FM_DIAGK)
+    for (int b = tid; b < copies * sw.nbins; b += T) hist[b] = 0.0;
   if (MODE == FM_Z1 || MODE == FM_DIAGR) __syncthreads();   // (other modes read the tables after a phase's barrier)
 
   const bool conj_in = MODE == FM_Z2 || MODE == FM_Z21 || (MODE == FM_PLAIN && op.inv1);
@@ -275,6 +282,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
           const double rho = (double)v[a].x * v[a].x + (double)v[a].y * v[a].y;
           R V = lc.vz[m] + c1[l];
           if (ph.vre) V += ((const R*)ph.vre)[lc.row0 + (long long)l * n + m];
+          if (ph.kind == 1 && ph.beam) V += (R)ph.beam_amp * c12[l];
           if (lc.vd1) V += lc.vd1[lc.row0 + (long long)l * n + m];
           n0 += rho;
           n1 = fma((double)V, rho, n1);
@@ -393,10 +401,8 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
             const double kk = kk_ref(ph.k[q + a * nb], ph.k[a0], ph.k[z0 + l]);
             const double w = (double)v[a].x * v[a].x + (double)v[a].y * v[a].y;
             e = fma(kk, w, e);
-            if (sw.hist) {
-              const int bin = (int)floor(sqrt(kk) / sw.shell_w + 0.5);
-              atomicAdd(hist + min(bin, sw.nbins - 1), w);
-            }
+            if (sw.hist)
+              atomicAdd(hist + (l & (copies - 1)) * sw.nbins + shell_of(kk, sw.shell_t, sw.inv_shell, sw.nbins), w);
           }
           cx.acc[3].add(e);
         } else if (MODE == FM_LZ) {
@@ -471,7 +477,11 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       for (int q = 0; q < 4; ++q) sw.partial[(long long)tile * 4 + q] = a[q].value();
     if (MODE == FM_DIAGK && sw.hist) {
       __syncthreads();
-      for (int b = tid; b < sw.nbins; b += T) sw.hist[(long long)tile * sw.nbins + b] = hist[b];
+      for (int b = tid; b < sw.nbins; b += T) {
+        double h = hist[b];
+        for (int c = 1; c < copies; ++c) h += hist[c * sw.nbins + b];
+        sw.hist[(long long)tile * sw.nbins + b] = h;
+      }
     }
   }
 }

@@ -166,7 +166,9 @@ inline LineShape line_shape_p(const LineGeo& g, int csize) {
   return s;
 }
 
-// dynamic shared memory: tile, per-line tables, reduction scratch (4 KB), histogram bins
+constexpr size_t LINE_HIST = 16 * 1024;   // shared memory for copies of the shell histogram
+
+// dynamic shared memory: tile, per-line tables, reduction scratch, `bins` doubles of histograms
 inline size_t line_smem(const LineGeo& g, const LineShape& s, int csize, bool z, int bins) {
   return (size_t)(z ? s.L * s.pitch : g.span * s.L) * csize + ((size_t)s.L * 24 + 15) / 16 * 16 + 32 * 4 * 16 +
          (size_t)bins * sizeof(double);

@@ -392,13 +392,15 @@ __global__ void k_finish_diag(const double* pa, int na, const double* pb, int nb
 template <typename C>
 __global__ void __launch_bounds__(256) k_kspace(const C* __restrict__ f, int n, const double* __restrict__ k,
                                                 double* __restrict__ partial, double* __restrict__ hist,
-                                                int nbins, double shell_w) {
+                                                int nbins, const double* __restrict__ shell_t, float inv_shell,
+                                                int copies) {
   extern __shared__ double sh_hist[];
   __shared__ Acc red[32];
   if (hist) {
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) sh_hist[b] = 0.0;
+    for (int b = threadIdx.x; b < copies * nbins; b += blockDim.x) sh_hist[b] = 0.0;
     __syncthreads();
   }
+  double* mine = sh_hist + (threadIdx.x & (copies - 1)) * nbins;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   double e = 0.0;
@@ -411,11 +413,7 @@ __global__ void __launch_bounds__(256) k_kspace(const C* __restrict__ f, int n, 
       const C v = row[z];
       const double w = (double)v.x * v.x + (double)v.y * v.y;
       e = fma(kk, w, e);
-      if (hist) {
-        int sh = (int)floor(sqrt(kk) / shell_w + 0.5);
-        sh = min(sh, nbins - 1);
-        atomicAdd(sh_hist + sh, w);
-      }
+      if (hist) atomicAdd(mine + shell_of(kk, shell_t, inv_shell, nbins), w);
     }
   }
   Acc a[1];
@@ -424,7 +422,37 @@ __global__ void __launch_bounds__(256) k_kspace(const C* __restrict__ f, int n, 
   if (threadIdx.x == 0) partial[(long long)blockIdx.x * 4 + 3] = a[0].value();
   if (hist) {
     __syncthreads();
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) hist[(long long)blockIdx.x * nbins + b] = sh_hist[b];
+    for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
+      double h = sh_hist[b];
+      for (int c = 1; c < copies; ++c) h += sh_hist[c * nbins + b];
+      hist[(long long)blockIdx.x * nbins + b] = h;
+    }
+  }
+}
+
+// Modes per shell (exact counts): the shells are those of the k-space reductions.  A warp
+// takes a row, counts collect in shared memory when the bins fit.
+__global__ void __launch_bounds__(256) k_shell_counts(int n, const double* __restrict__ k, int nbins,
+                                                      const double* __restrict__ shell_t, float inv_shell, int shared,
+                                                      unsigned long long* __restrict__ out) {
+  extern __shared__ unsigned cnt[];
+  if (shared) {
+    for (int b = threadIdx.x; b < nbins; b += blockDim.x) cnt[b] = 0u;
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n * n; r += warps) {
+    const double kx = k[r / n], ky = k[r % n];
+    for (int z = lane; z < n; z += 32) {
+      const int b = shell_of(kk_ref(kx, ky, k[z]), shell_t, inv_shell, nbins);
+      if (shared) atomicAdd(cnt + b, 1u);
+      else atomicAdd(out + b, 1ull);
+    }
+  }
+  if (shared) {
+    __syncthreads();
+    for (int b = threadIdx.x; b < nbins; b += blockDim.x)
+      if (cnt[b]) atomicAdd(out + b, (unsigned long long)cnt[b]);
   }
 }
 
@@ -758,7 +786,14 @@ struct gpe_plan {
   bool fixed = false;              // sweeps compiled for this side exist
   // their geometry, tiles and tables: [0] steps, [1] transforms and reductions (complex64:
   // the radices of the Stockham passes, so that these results keep their rounding)
-  struct LineSet { LineGeo geo{}; LineShape z{}, p{}; bool ok = false; void* d_tw = nullptr; void* d_bf = nullptr; };
+  struct LineSet {
+    LineGeo geo{};
+    LineShape z{}, p{};
+    bool ok = false;
+    void* d_tw = nullptr;
+    void* d_bf = nullptr;
+    size_t off_tw[LINE_PMAX] = {}, off_twi[LINE_PMAX] = {}, off_bf[LINE_PMAX] = {};
+  };
   LineSet ls[2];
   bool plane = false;              // y and z sweeps fused per x-plane (opt-in; complex64, n = 128, 256)
   bool tma = false;                // plain y/x sweeps stage their pencils by TMA (opt-in; complex64, n = 128, 256)
@@ -774,6 +809,8 @@ struct gpe_plan {
   double shell_w = 0;
   std::vector<long long> counts;
   // device buffers
+  void* d_tables = nullptr;        // one allocation behind all tables and small buffers below
+  double* d_shell = nullptr;       // least k^2 of each shell
   double* d_x = nullptr;
   double* d_k = nullptr;
   double2* d_kin = nullptr;
@@ -1090,7 +1127,9 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   const bool line = !p->fixed || o.tr == 2;
   const gpe_plan::LineSet& ls = p->ls[o.tr ? 1 : 0];
   const LineShape& shape = fax == FZ ? ls.z : ls.p;
-  const size_t smem = line ? line_smem(ls.geo, shape, (int)p->csize, fax == FZ, sw.hist ? sw.nbins : 0) : 0;
+  const size_t smem = line ? line_smem(ls.geo, shape, (int)p->csize, fax == FZ,
+                                      sw.hist ? hist_copies(sw.nbins, LINE_HIST) * sw.nbins : 0)
+                          : 0;
   const cudaError_t e =
       line ? (p->dtype == GPE_C64 ? launch_line<float>(fax, p->ph, sw, o, ls.geo, shape, smem, st)
                                   : launch_line<double>(fax, p->ph, sw, o, ls.geo, shape, smem, st))
@@ -1234,6 +1273,28 @@ int ensure_hist(gpe_plan* p) {
   return GPE_OK;
 }
 
+// The least double kk >= 0 of every shell b, floor(sqrt(kk)/w + 0.5) >= b: the expression never
+// decreases with kk (each of its operations rounds monotonically), so the boundary is found
+// by bisection over the doubles, which order as their bits.
+std::vector<double> shell_starts(double w, int nbins) {
+  std::vector<double> t(nbins, 0.0);
+  for (int b = 1; b < nbins; ++b) {
+    double lo_d = t[b - 1], hi_d = (b + 1.0) * w * ((b + 1.0) * w) * 2.0;
+    long long lo, hi;   // the shell of lo is below b (or lo = 0), that of hi is not
+    memcpy(&lo, &lo_d, 8);
+    memcpy(&hi, &hi_d, 8);
+    while (lo < hi) {
+      const long long mid = lo + (hi - lo) / 2;
+      double x;
+      memcpy(&x, &mid, 8);
+      if (std::floor(std::sqrt(x) / w + 0.5) >= b) hi = mid;
+      else lo = mid + 1;
+    }
+    memcpy(&t[b], &hi, 8);
+  }
+  return t;
+}
+
 // The point tables' memory: taken when the plan is made (a step then allocates nothing, as
 // under stream capture), and only where it is a small part of what is free; without it
 // the potential is evaluated per point in the Stockham sweeps.
@@ -1336,22 +1397,43 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
     p->nbins = (int)std::floor(std::sqrt(3.0) * (n / 2) + 0.5) + 1;
     p->shell_w = dk;
   }
-  p->counts.assign(p->nbins, 0);
-  for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j)
-      for (int l = 0; l < n; ++l) {
-        const double kk = p->k[i] * p->k[i] + p->k[j] * p->k[j] + p->k[l] * p->k[l];
-        int s = (int)std::floor(std::sqrt(kk) / p->shell_w + 0.5);
-        p->counts[std::min(s, p->nbins - 1)]++;
-      }
+  p->counts.assign(p->nbins, 0);   // (filled by create)
   p->max_tiles = std::max(tiles_of(p, AX_Z), tiles_of(p, AX_X));
   for (const auto& s : p->ls)
     if (s.ok) p->max_tiles = std::max(p->max_tiles, std::max(s.z.tiles, s.p.tiles));
   return GPE_OK;
 }
 
+// A plan's tables, collected on the host and brought over with one allocation and one
+// copy (an allocation and a copy each cost more than the tables' bytes).
+struct Tables {
+  std::vector<char> host;
+  size_t room_bytes = 0;
+  struct Item { void** dst; size_t off; bool room; };
+  std::vector<Item> items;
+  static size_t aligned(size_t b) { return (b + 255) / 256 * 256; }
+  // a table with its contents
+  template <typename T> void put(T** dst, const void* data, size_t bytes) {
+    items.push_back({(void**)dst, host.size(), false});
+    const char* c = (const char*)data;
+    host.insert(host.end(), c, c + bytes);
+    host.resize(aligned(host.size()), 0);
+  }
+  // uninitialised room, behind the tables
+  template <typename T> void room(T** dst, size_t bytes) {
+    items.push_back({(void**)dst, room_bytes, true});
+    room_bytes += aligned(bytes);
+  }
+  int commit(void** base) {
+    CU(cudaMalloc(base, host.size() + room_bytes));
+    CU(cudaMemcpy(*base, host.data(), host.size(), cudaMemcpyHostToDevice));
+    for (const Item& i : items) *i.dst = (char*)*base + i.off + (i.room ? host.size() : 0);
+    return GPE_OK;
+  }
+};
+
 template <typename R>
-int upload_tables(gpe_plan* p, const gpe_desc* d) {
+int make_tables(gpe_plan* p, const gpe_desc* d, Tables& tabs) {
   const int n = p->n;
   // twiddles W_n^j = exp(-2 pi i j/n), computed in long double and rounded once
   std::vector<typename Cx<R>::T> tw(n), twl(n);
@@ -1364,9 +1446,9 @@ int upload_tables(gpe_plan* p, const gpe_desc* d) {
     twl[j].x = sizeof(R) == 4 ? (R)(double)(c - (long double)tw[j].x) : (R)0;
     twl[j].y = sizeof(R) == 4 ? (R)(double)(s - (long double)tw[j].y) : (R)0;
   }
-  CU(cudaMalloc(&p->d_tw, 2 * n * sizeof(tw[0])));
-  CU(cudaMemcpy(p->d_tw, tw.data(), n * sizeof(tw[0]), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((char*)p->d_tw + n * sizeof(tw[0]), twl.data(), n * sizeof(tw[0]), cudaMemcpyHostToDevice));
+  std::vector<typename Cx<R>::T> both(tw);
+  both.insert(both.end(), twl.begin(), twl.end());
+  tabs.put(&p->d_tw, both.data(), both.size() * sizeof(both[0]));
   // run-time-length sweeps: twiddles in the order of each phase's lanes, butterfly tables
   for (auto& ls : p->ls) {
     if (!ls.ok) continue;
@@ -1393,16 +1475,14 @@ int upload_tables(gpe_plan* p, const gpe_desc* d) {
           for (int c = 0; c < g.nl[q]; ++c) push(g.np[q] * k * c);
       }
     }
-    CU(cudaMalloc(&ls.d_tw, lt.size() * sizeof(lt[0])));
-    CU(cudaMemcpy(ls.d_tw, lt.data(), lt.size() * sizeof(lt[0]), cudaMemcpyHostToDevice));
-    CU(cudaMalloc(&ls.d_bf, lb.size() * sizeof(int)));
-    CU(cudaMemcpy(ls.d_bf, lb.data(), lb.size() * sizeof(int), cudaMemcpyHostToDevice));
+    tabs.put(&ls.d_tw, lt.data(), lt.size() * sizeof(lt[0]));
+    tabs.put(&ls.d_bf, lb.data(), lb.size() * sizeof(int));
+    // (offsets until the tables have their address: bind_line_tables)
     for (int q = 0; q < g.P; ++q) {
-      g.tw[q] = (const char*)ls.d_tw + tw0[q] * sizeof(lt[0]);
-      g.twi[q] = (const char*)ls.d_tw + twi0[q] * sizeof(lt[0]);
-      g.bf[q] = (const char*)ls.d_bf + bf0[q] * sizeof(int);
+      ls.off_tw[q] = tw0[q] * sizeof(lt[0]);
+      ls.off_twi[q] = twi0[q] * sizeof(lt[0]);
+      ls.off_bf[q] = bf0[q] * sizeof(int);
     }
-    g.w = p->d_tw;
   }
   // packed sweeps: entries (hi.x, hi.x, hi.y, hi.y), then the residuals, [value][lane]: the
   // first phase's W_512^(p k3), then the second's W_64^(p1 k1)
@@ -1419,8 +1499,7 @@ int upload_tables(gpe_plan* p, const gpe_desc* d) {
       };
       table(64, 8, 1);
       table(8, 8, 8);
-      CU(cudaMalloc(&p->d_twp, tp.size() * sizeof(tp[0])));
-      CU(cudaMemcpy(p->d_twp, tp.data(), tp.size() * sizeof(tp[0]), cudaMemcpyHostToDevice));
+      tabs.put(&p->d_twp, tp.data(), tp.size() * sizeof(tp[0]));
     }
   }
   // static axis potentials
@@ -1435,9 +1514,21 @@ int upload_tables(gpe_plan* p, const gpe_desc* d) {
       vax[a * n + i] = (R)host_eval(prog, a == 0 ? c : 0.0, a == 1 ? c : 0.0, a == 2 ? c : 0.0, 0.0);
     }
   }
-  CU(cudaMalloc(&p->d_vax, 3 * n * sizeof(R)));
-  CU(cudaMemcpy(p->d_vax, vax.data(), 3 * n * sizeof(R), cudaMemcpyHostToDevice));
+  tabs.put(&p->d_vax, vax.data(), 3 * n * sizeof(R));
   return GPE_OK;
+}
+
+void bind_line_tables(gpe_plan* p) {
+  for (auto& ls : p->ls) {
+    if (!ls.ok) continue;
+    LineGeo& g = ls.geo;
+    for (int q = 0; q < g.P; ++q) {
+      g.tw[q] = (const char*)ls.d_tw + ls.off_tw[q];
+      g.twi[q] = (const char*)ls.d_tw + ls.off_twi[q];
+      g.bf[q] = (const char*)ls.d_bf + ls.off_bf[q];
+    }
+    g.w = p->d_tw;
+  }
 }
 
 int build_static(gpe_plan* p, const void* v, int v_kind, cudaStream_t st) {
@@ -1466,9 +1557,8 @@ int build_static(gpe_plan* p, const void* v, int v_kind, cudaStream_t st) {
 void free_plan(gpe_plan* p) {
   for (auto& r : p->recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   for (auto e : p->pool) cudaEventDestroy(e);
-  void* bufs[] = {p->d_x, p->d_k, p->d_kin, p->d_kth, p->d_vax, p->d_vre, p->d_vim, p->d_prog_g, p->d_dyn, p->d_line, p->d_ltab,
-                  p->d_tw, p->d_partial, p->d_ticket, p->d_scale, p->d_status, p->d_hist, p->d_out,
-                  p->d_work, p->d_plane, p->d_proj, p->ls[0].d_tw, p->ls[0].d_bf, p->ls[1].d_tw, p->ls[1].d_bf, p->d_twp, p->d_pprog, p->d_ptab};
+  // (the tables share one allocation)
+  void* bufs[] = {p->d_tables, p->d_vre, p->d_vim, p->d_hist, p->d_work, p->d_proj, p->d_ptab};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete p;
@@ -1479,69 +1569,74 @@ int create(const gpe_desc* d, gpe_plan** out) {
   int rc = fill_plan(p, d);
   if (rc != GPE_OK) { free_plan(p); return rc; }
   const int n = p->n;
-  CU(cudaMalloc(&p->d_x, n * sizeof(double)));
-  CU(cudaMemcpy(p->d_x, p->x.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-  CU(cudaMalloc(&p->d_k, n * sizeof(double)));
-  CU(cudaMemcpy(p->d_k, p->k.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+  Tables tabs;
+  tabs.put(&p->d_x, p->x.data(), n * sizeof(double));
+  tabs.put(&p->d_k, p->k.data(), n * sizeof(double));
+  const std::vector<double> shell = shell_starts(p->shell_w, p->nbins);
+  tabs.put(&p->d_shell, shell.data(), shell.size() * sizeof(double));
   // kinetic factors per axis: exp(-i ckin k^2 dt) or exp(-ckin k^2 dt)
   std::vector<double2> kin(n);
+  std::vector<double> kth(n);
   for (int i = 0; i < n; ++i) {
     const double ph = p->ckin * p->k[i] * p->k[i] * p->dt;
     kin[i] = p->kind == GPE_IMAGINARY ? make_double2(std::exp(-ph), 0.0)
                                       : make_double2(std::cos(ph), -std::sin(ph));
+    kth[i] = ph;
   }
-  CU(cudaMalloc(&p->d_kin, n * sizeof(double2)));
-  CU(cudaMemcpy(p->d_kin, kin.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
-  std::vector<double> kth(n);
-  for (int i = 0; i < n; ++i) kth[i] = p->ckin * p->k[i] * p->k[i] * p->dt;
-  CU(cudaMalloc(&p->d_kth, n * sizeof(double)));
-  CU(cudaMemcpy(p->d_kth, kth.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-  rc = p->dtype == GPE_C64 ? upload_tables<float>(p, d) : upload_tables<double>(p, d);
+  tabs.put(&p->d_kin, kin.data(), n * sizeof(double2));
+  tabs.put(&p->d_kth, kth.data(), n * sizeof(double));
+  rc = p->dtype == GPE_C64 ? make_tables<float>(p, d, tabs) : make_tables<double>(p, d, tabs);
   if (rc != GPE_OK) { free_plan(p); return rc; }
-  if (!p->prog_static_g.empty()) {
-    CU(cudaMalloc(&p->d_prog_g, p->prog_static_g.size() * sizeof(double)));
-    CU(cudaMemcpy(p->d_prog_g, p->prog_static_g.data(), p->prog_static_g.size() * sizeof(double),
-                  cudaMemcpyHostToDevice));
-  }
-  if (!p->prog_dyn.empty()) {
-    CU(cudaMalloc(&p->d_dyn, p->prog_dyn.size() * sizeof(double)));
-    CU(cudaMemcpy(p->d_dyn, p->prog_dyn.data(), p->prog_dyn.size() * sizeof(double), cudaMemcpyHostToDevice));
-  }
+  auto program = [&](double** dst, const std::vector<double>& v) {
+    if (!v.empty()) tabs.put(dst, v.data(), v.size() * sizeof(double));
+  };
+  program(&p->d_prog_g, p->prog_static_g);
+  program(&p->d_dyn, p->prog_dyn);
   if (p->has_point) {
     std::vector<double> all;
     PointProg& q = p->pprog;
-    auto put = [&](const std::vector<double>& v, int& off, int& len) {
+    auto add = [&](const std::vector<double>& v, int& off, int& len) {
       off = (int)all.size();
       len = (int)v.size();
       all.insert(all.end(), v.begin(), v.end());
     };
     q.nrow = (int)p->point.rows.size();
     q.nz = (int)p->point.zs.size();
-    for (int k = 0; k < q.nrow; ++k) put(p->point.rows[k], q.row_off[k], q.row_len[k]);
-    for (int k = 0; k < q.nz; ++k) put(p->point.zs[k], q.z_off[k], q.z_len[k]);
-    put(p->point.residual, q.off, q.len);
-    CU(cudaMalloc(&p->d_pprog, all.size() * sizeof(double)));
-    CU(cudaMemcpy(p->d_pprog, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice));
-    q.base = p->d_pprog;
+    for (int k = 0; k < q.nrow; ++k) add(p->point.rows[k], q.row_off[k], q.row_len[k]);
+    for (int k = 0; k < q.nz; ++k) add(p->point.zs[k], q.z_off[k], q.z_len[k]);
+    add(p->point.residual, q.off, q.len);
+    program(&p->d_pprog, all);
   }
-  if (!p->prog_line.empty()) {
-    CU(cudaMalloc(&p->d_line, p->prog_line.size() * sizeof(double)));
-    CU(cudaMemcpy(p->d_line, p->prog_line.data(), p->prog_line.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CU(cudaMalloc(&p->d_ltab, 2 * (size_t)n * n * (p->dtype == GPE_C64 ? 4 : 8)));
-  }
-  CU(cudaMalloc(&p->d_partial, 2 * 4 * (size_t)p->max_tiles * sizeof(double)));
-  CU(cudaMalloc(&p->d_ticket, sizeof(unsigned)));
-  CU(cudaMemset(p->d_ticket, 0, sizeof(unsigned)));
-  if (p->plane) {
-    CU(cudaMalloc(&p->d_plane, (2 + 3 * (size_t)n) * sizeof(unsigned)));
-    CU(cudaMemset(p->d_plane, 0, (2 + 3 * (size_t)n) * sizeof(unsigned)));
-  }
-  CU(cudaMalloc(&p->d_scale, 4 * sizeof(double)));
+  program(&p->d_line, p->prog_line);
   const double one[4] = {1.0, 1.0, 1.0, 0.0};
-  CU(cudaMemcpy(p->d_scale, one, sizeof(one), cudaMemcpyHostToDevice));
-  CU(cudaMalloc(&p->d_status, sizeof(int)));
-  CU(cudaMemset(p->d_status, 0, sizeof(int)));
-  CU(cudaMalloc(&p->d_out, (4 + p->nbins) * sizeof(double)));
+  tabs.put(&p->d_scale, one, sizeof(one));
+  const unsigned zero = 0;
+  tabs.put(&p->d_ticket, &zero, sizeof(zero));
+  tabs.put(&p->d_status, &zero, sizeof(zero));
+  if (p->plane) {
+    const std::vector<unsigned> none(2 + 3 * (size_t)n, 0u);
+    tabs.put(&p->d_plane, none.data(), none.size() * sizeof(unsigned));
+  }
+  const std::vector<unsigned long long> counts(p->nbins, 0ull);
+  unsigned long long* d_counts = nullptr;
+  tabs.put(&d_counts, counts.data(), counts.size() * sizeof(counts[0]));
+  tabs.room(&p->d_partial, 2 * 4 * (size_t)p->max_tiles * sizeof(double));
+  tabs.room(&p->d_out, (4 + p->nbins) * sizeof(double));
+  if (!p->prog_line.empty()) tabs.room(&p->d_ltab, 2 * (size_t)n * n * (p->dtype == GPE_C64 ? 4 : 8));
+  rc = tabs.commit(&p->d_tables);
+  if (rc != GPE_OK) { free_plan(p); return rc; }
+  bind_line_tables(p);
+  p->pprog.base = p->d_pprog;
+  {
+    // modes per shell, on the device (the host loop over n^3 modes took 60 ms at 256^3)
+    const size_t smem = (size_t)p->nbins * sizeof(unsigned);
+    const int shared = smem <= 48 * 1024;
+    k_shell_counts<<<std::max(1, std::min(592, (n * n + 7) / 8)), 256, shared ? smem : 0>>>(
+        n, p->d_k, p->nbins, p->d_shell, (float)(1.0 / p->shell_w), shared, d_counts);
+    CU(cudaGetLastError());
+    static_assert(sizeof(p->counts[0]) == sizeof(unsigned long long), "counts");
+    CU(cudaMemcpy(p->counts.data(), d_counts, p->nbins * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+  }
   Phys& ph = p->ph;
   ph.kind = p->kind;
   ph.beta = p->beta;
@@ -1682,15 +1777,18 @@ int kspace_reduce(gpe_plan* p, const void* f, bool hist, int& nb, cudaStream_t s
     CU(cudaGetDevice(&dev));
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   }
-  const size_t smem = hist ? (size_t)p->nbins * sizeof(double) : 0;
+  const int copies = hist_copies(p->nbins, 24 * 1024);
+  const size_t smem = hist ? (size_t)copies * p->nbins * sizeof(double) : 0;
   if (smem > 48 * 1024) return fail(GPE_ERR_UNSUPPORTED, "too many n(k) bins for the shared histogram");
   nb = std::max(1, std::min(p->max_tiles, std::min(4 * sms, (p->n * p->n + 7) / 8)));
   double* part = p->d_partial + 4 * (size_t)p->max_tiles;
   double* h = hist ? p->d_hist : nullptr;
   if (p->dtype == GPE_C64)
-    k_kspace<float2><<<nb, 256, smem, st>>>((const float2*)f, p->n, p->d_k, part, h, p->nbins, p->shell_w);
+    k_kspace<float2><<<nb, 256, smem, st>>>((const float2*)f, p->n, p->d_k, part, h, p->nbins, p->d_shell,
+                                        (float)(1.0 / p->shell_w), copies);
   else
-    k_kspace<double2><<<nb, 256, smem, st>>>((const double2*)f, p->n, p->d_k, part, h, p->nbins, p->shell_w);
+    k_kspace<double2><<<nb, 256, smem, st>>>((const double2*)f, p->n, p->d_k, part, h, p->nbins, p->d_shell,
+                                        (float)(1.0 / p->shell_w), copies);
   CU(cudaGetLastError());
   ++p->launches;
   return GPE_OK;
@@ -1728,7 +1826,7 @@ void diag_tiles(const gpe_plan* p, bool fast, int& na, int& nb) {
 // and the shell histogram (if wanted) fits their shared tables region.
 bool diag_fast(const gpe_plan* p, bool hist) {
   if (!p->fast || !hist) return p->fast;
-  if (p->fixed) return (size_t)p->nbins * sizeof(double) <= fast_tables_bytes_rt(p->n, (int)p->csize / 2);
+  if (p->fixed) return (size_t)p->nbins * sizeof(double) <= fast_hist_bytes_rt(p->n, (int)p->csize / 2);
   return line_smem(p->ls[1].geo, p->ls[1].p, (int)p->csize, false, p->nbins) <= 96 * 1024;
 }
 
@@ -1744,7 +1842,8 @@ int diag_launch(gpe_plan* p, const void* psi, double t, bool hist, cudaStream_t 
     s.partial = p->d_partial + 4 * (size_t)p->max_tiles;
     s.hist = hist ? p->d_hist : nullptr;
     s.nbins = p->nbins;
-    s.shell_w = p->shell_w;
+    s.shell_t = p->d_shell;
+    s.inv_shell = (float)(1.0 / p->shell_w);
     return fsweep(p, AX_X, s, tr_ops(FM_DIAGK), st);
   }
   Sweep s = mk_sweep(psi, p->d_work);
@@ -2058,6 +2157,15 @@ int gpe_diagnostics(gpe_plan* p, const void* psi, double t, double* scalars, dou
     for (int b = 0; b < p->nbins; ++b) nk[b] = h[4 + b] * p->ph.dx3 * p->ph.inv_m;
   if (counts)
     for (int b = 0; b < p->nbins; ++b) counts[b] = p->counts[b];
+  return GPE_OK;
+}
+
+int gpe_read_pairs(const double* a, const double* b, double* out, void* stream) {
+  if (!a || !out) return fail(GPE_ERR_ARG, "null argument");
+  cudaStream_t st = (cudaStream_t)stream;
+  CU(cudaMemcpyAsync(out, a, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (b) CU(cudaMemcpyAsync(out + 2, b, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  CU(cudaStreamSynchronize(st));
   return GPE_OK;
 }
 

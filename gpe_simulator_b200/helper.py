@@ -6,12 +6,14 @@ Drop-in counterparts of ``gpe/grids.py``, ``gpe/helper.py`` and
 """
 
 from collections import OrderedDict
+import ctypes
 import math
 
 import numpy as np
 import torch
 
-from .plan import Plan
+from . import _lib
+from .plan import Plan, _stream
 
 # utility plans by (grid, dtype, device, shell binning), least recently used first;
 # the oldest is dropped once more than _UTIL_MAX are held (a plan frees its tables when
@@ -27,20 +29,48 @@ def get_grids(N_grids, simulation_range, device="cuda"):
     return torch.from_numpy(x).to(device), torch.from_numpy(k).to(device)
 
 
-def utility_plan(psi, x_array, k_array=None, nbins=0):
+def _host(axis):
+    return axis.detach().cpu().numpy() if isinstance(axis, torch.Tensor) else np.asarray(axis)
+
+
+def first_two(*axes):
+    """The first two values of each axis (one or two of them), as floats.  CUDA float64 axes
+    are read natively, one synchronisation for all; the values are read at every call, an
+    axis may be changed in place."""
+    if all(isinstance(a, torch.Tensor) and a.is_cuda and a.dtype == torch.float64 and a.is_contiguous()
+           and a.numel() >= 2 for a in axes) and len({a.device for a in axes}) == 1:
+        out = (ctypes.c_double * 4)()
+        ptr = [ctypes.c_void_p(a.data_ptr()) for a in axes] + [None]
+        with torch.cuda.device(axes[0].device):
+            _lib.check(_lib.load().gpe_read_pairs(ptr[0], ptr[1], out, _stream()))
+        return [(out[2 * i], out[2 * i + 1]) for i in range(len(axes))]
+    return [(float(h[0]), float(h[1])) for h in map(_host, axes)]
+
+
+def utility_plan(psi, x_array, k_array=None, nbins=0, pairs=None):
     """Plan without physics, for FFTs and reductions on ``psi``'s grid (``nbins``:
     0 = the reference's shell binning, else that many uniform bins).  Plans are
-    cached, so repeated diagnostics on one grid create no new device tables."""
+    cached by the grid's values, so repeated diagnostics on one grid create no new
+    device tables.  ``pairs``: ``first_two(x_array[, k_array])`` if already read."""
     n = psi.shape[0]
-    xs = x_array.detach().cpu().numpy() if isinstance(x_array, torch.Tensor) else np.asarray(x_array)
+    if pairs is None:
+        pairs = first_two(x_array) if k_array is None else first_two(x_array, k_array)
+    x0, x1 = pairs[0]
     if k_array is None:
-        L = (xs[1] - xs[0]) * n
-        ks = 2 * np.pi * np.fft.fftfreq(n, L / n)
+        # element 1 of 2 pi fftfreq(n, L/n)
+        L = (x1 - x0) * n
+        k1 = 2 * np.pi * ((1 if n > 2 else -1) * (1.0 / (n * (L / n))))
     else:
-        ks = k_array.detach().cpu().numpy() if isinstance(k_array, torch.Tensor) else np.asarray(k_array)
-    key = (n, psi.dtype, psi.device.index, float(xs[0]), float(xs[1]), float(ks[1]), int(nbins or 0))
+        k1 = pairs[1][1]
+    key = (n, psi.dtype, psi.device.index, x0, x1, float(k1), int(nbins or 0))
     plan = _UTIL.get(key)
     if plan is None:
+        xs = _host(x_array)
+        if k_array is None:
+            L = (xs[1] - xs[0]) * n
+            ks = 2 * np.pi * np.fft.fftfreq(n, L / n)
+        else:
+            ks = _host(k_array)
         with torch.cuda.device(psi.device):
             plan = Plan(n, xs, ks, dtype=psi.dtype, kind="imaginary", beta=0.0, dt=0.0, nk_bins=int(nbins or 0))
         _UTIL[key] = plan

@@ -9,7 +9,7 @@ import math
 
 import numpy as np
 
-from .helper import utility_plan
+from .helper import first_two, utility_plan
 
 
 def shell_geometry(n, dk, nbins=None):
@@ -38,8 +38,8 @@ def nk_extraction(psi_k, x_array, k_array, slab_size=16, nbins=None):
     no slabs.  ``nbins`` selects the uniform-bin extension.
     """
     n = psi_k.shape[0]
-    ks = k_array.detach().cpu().numpy()
-    dk = abs(float(ks[1] - ks[0]))
-    plan = utility_plan(psi_k, x_array, k_array, nbins=nbins or 0)
+    pairs = first_two(x_array, k_array)
+    dk = abs(pairs[1][1] - pairs[1][0])
+    plan = utility_plan(psi_k, x_array, k_array, nbins=nbins or 0, pairs=pairs)
     Nk, counts = plan.shells(psi_k)
     return assemble(Nk, counts, n, dk, nbins)

@@ -186,6 +186,11 @@ int  gpe_angular_momentum(gpe_plan* plan, const void* psi, double* lz, void* str
 #define GPE_PROJ_PHASE_XY        64u   /* arg psi at z = n/2 */
 int  gpe_projections(gpe_plan* plan, const void* psi, unsigned which, double* out, void* stream);
 
+/* The first two doubles of one or two device arrays (b nullable): out[0..1] from a,
+ * out[2..3] from b, with one synchronisation of `stream` (the grid spacing of axes a
+ * caller passes with every call, e.g. get_N's x_array) */
+int  gpe_read_pairs(const double* a, const double* b, double* out, void* stream);
+
 /* accounting: kernel launches issued by this plan since creation */
 int  gpe_launch_count(const gpe_plan* plan, long long* count);
 /* per-launch timing: enable = 1 brackets every sweep launch with CUDA events on its
