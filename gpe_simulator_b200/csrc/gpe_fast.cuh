@@ -1177,6 +1177,9 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
 // except Z21 and XKIN at n = 256, which run 4 blocks of 64 registers (a few
 // hundred bytes of spills in Z21): 4486 -> 4541 steps/s at 256^3, the gain
 // being in the overlap of the programmatically launched sweeps.
+// At n = 128 the fused modes run 7 blocks of 72 registers: a 128^3 sweep is 1024 tiles, one
+// wave of 7 x 148 = 1036 blocks but 1.15 waves of 6 (imaginary time 51.0 -> 45.8 us per
+// step, stirred 35.1 -> 31.9; 8 blocks of 64 registers 46.0, 32.4).
 // At n = 512 (three radix-8 phases, 16 values per thread, 512-thread blocks of
 // about 98 KB of shared memory) two blocks per SM, 64 registers: 378 -> 415
 // steps/s at 512^3 against the earlier 32 x 16 split (32 values per thread, one
@@ -1185,7 +1188,7 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
 template <int N, typename R, int MODE> struct FastBounds {
   static constexpr int value = (sizeof(R) == 4 && (N == 128 || N == 256))
                                    ? (MODE == FM_PLAIN ? 1024 : MODE == FM_DIAGR ? 512
-                                      : (N == 256 && (MODE == FM_Z21 || MODE == FM_XKIN)) ? 1024 : 768) /
+                                      : N == 128 && MODE != FM_DIAGK ? 896 : (N == 256 && (MODE == FM_Z21 || MODE == FM_XKIN)) ? 1024 : 768) /
                                          FastCfg<N, R>::T
                                : (sizeof(R) == 4 && N == 512)
                                    ? (MODE == FM_DIAGR ? 512 : 1024) / FastCfg<N, R>::T : 0;

@@ -41,23 +41,30 @@ constexpr int FM_LZ = 7;          // forward transform, angular-momentum sums, n
 // b / d for b, d < 2^16 by the rounded-up reciprocal mg = ceil(2^32 / d)
 __device__ __forceinline__ int div_mg(int b, unsigned mg) { return mg ? (int)__umulhi((unsigned)b, mg) : b; }
 
-template <typename F> __device__ __forceinline__ void by_radix(int r, F&& f) {
+// RMAX: largest radix of the launch's geometry (8 or 16).  The radices up to 8 need half the
+// registers of 16, so their own instantiations run twice the warps per SM.
+template <int RMAX, typename F> __device__ __forceinline__ void by_radix(int r, F&& f) {
   switch (r) {
-    case 2: f(std::integral_constant<int, 2>{}); break;
-    case 3: f(std::integral_constant<int, 3>{}); break;
-    case 4: f(std::integral_constant<int, 4>{}); break;
-    case 5: f(std::integral_constant<int, 5>{}); break;
-    case 6: f(std::integral_constant<int, 6>{}); break;
-    case 7: f(std::integral_constant<int, 7>{}); break;
-    case 8: f(std::integral_constant<int, 8>{}); break;
-    case 9: f(std::integral_constant<int, 9>{}); break;
-    case 10: f(std::integral_constant<int, 10>{}); break;
-    case 11: f(std::integral_constant<int, 11>{}); break;
-    case 12: f(std::integral_constant<int, 12>{}); break;
-    case 13: f(std::integral_constant<int, 13>{}); break;
-    case 14: f(std::integral_constant<int, 14>{}); break;
-    case 15: f(std::integral_constant<int, 15>{}); break;
-    default: f(std::integral_constant<int, 16>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); return;
+    case 3: f(std::integral_constant<int, 3>{}); return;
+    case 4: f(std::integral_constant<int, 4>{}); return;
+    case 5: f(std::integral_constant<int, 5>{}); return;
+    case 6: f(std::integral_constant<int, 6>{}); return;
+    case 7: f(std::integral_constant<int, 7>{}); return;
+    case 8: f(std::integral_constant<int, 8>{}); return;
+    default: break;
+  }
+  if constexpr (RMAX > 8) {
+    switch (r) {
+      case 9: f(std::integral_constant<int, 9>{}); return;
+      case 10: f(std::integral_constant<int, 10>{}); return;
+      case 11: f(std::integral_constant<int, 11>{}); return;
+      case 12: f(std::integral_constant<int, 12>{}); return;
+      case 13: f(std::integral_constant<int, 13>{}); return;
+      case 14: f(std::integral_constant<int, 14>{}); return;
+      case 15: f(std::integral_constant<int, 15>{}); return;
+      default: f(std::integral_constant<int, 16>{}); return;
+    }
   }
 }
 
@@ -129,7 +136,7 @@ __device__ __forceinline__ void line_half(const Phys& ph, const LineCx<R>& cx, t
 }
 
 // ---------------------------------------------------------------- the sweep
-template <typename R, bool ZT, int MODE>
+template <typename R, bool ZT, int MODE, int RMAX>
 __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const FastOps& op, const LineGeo& g,
                                           const LineShape& sh, int ax, int tile, int ntiles) {
   using C = typename Cx<R>::T;
@@ -243,7 +250,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   C* __restrict__ dst = (C*)sw.dst;
 
   // phase 0: HBM -> registers -> shared memory
-  by_radix(g.r[0], [&](auto rc) {
+  by_radix<RMAX>(g.r[0], [&](auto rc) {
     constexpr int RAD = decltype(rc)::value;
     const int nb = g.nb[0], total = count(0), S0 = g.S[0];
     const TW* tw = (const TW*)g.tw[0];
@@ -304,7 +311,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   __syncthreads();
   // middle phases, in place
   for (int p = 1; p < P - 1; ++p) {
-    by_radix(g.r[p], [&](auto rc) {
+    by_radix<RMAX>(g.r[p], [&](auto rc) {
       constexpr int RAD = decltype(rc)::value;
       // (twiddle row length and this butterfly's place in it)
       const int total = count(p), S = g.S[p], row = DIT ? g.np[p] : g.nl[p];
@@ -333,7 +340,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
     __syncthreads();
   }
   // last phase: shared memory -> registers, pointwise, then HBM or the transform back
-  by_radix(g.r[P - 1], [&](auto rc) {
+  by_radix<RMAX>(g.r[P - 1], [&](auto rc) {
     constexpr int RAD = decltype(rc)::value;
     const int nb = g.nb[P - 1], total = count(P - 1);
     const int2* bf = (const int2*)g.bf[P - 1];
@@ -424,7 +431,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   if (TWO_FFT) {
     __syncthreads();
     for (int p = P - 2; p > 0; --p) {
-      by_radix(g.r[p], [&](auto rc) {
+      by_radix<RMAX>(g.r[p], [&](auto rc) {
         constexpr int RAD = decltype(rc)::value;
         const int total = count(p), S = g.S[p], nl = g.nl[p];
         const TW* tw = (const TW*)g.tw[p];
@@ -444,7 +451,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       });
       __syncthreads();
     }
-    by_radix(g.r[0], [&](auto rc) {
+    by_radix<RMAX>(g.r[0], [&](auto rc) {
       constexpr int RAD = decltype(rc)::value;
       const int nb = g.nb[0], total = count(0), S0 = g.S[0];
       const TW* tw = (const TW*)g.tw[0];
@@ -486,19 +493,24 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   }
 }
 
-// Resident blocks: 64 registers in complex64 (80 measured slower: 200^3 236 -> 261 us per
-// step), 128 in complex128.
-template <typename R> struct LineBounds { static constexpr int blocks = sizeof(R) == 4 ? 4 : 2; };
+// Resident blocks.  Radices to 16: 64 registers in complex64 (80 measured slower: 200^3
+// 236 -> 261 us per step), 128 in complex128.  Radices to 8: 64 registers, the complex128 x
+// sweep with its FP64 factors 80 (per step, complex128: 200^3 450 -> 349 us at 4 blocks, 385
+// at 3, 422 at 2; 512^3 x sweep 1.84 ms at 4 blocks, 1.49 at 3, where its 68 KB tiles allow
+// no more; complex64 at 48 registers: 125^3 82 -> 90 us, 384^3 1.55 -> 1.48 ms).
+template <typename R, int MODE, int RMAX> struct LineBounds {
+  static constexpr int blocks = sizeof(R) == 4 ? 4 : RMAX > 8 ? 2 : MODE == FM_XKIN ? 3 : 4;
+};
 
-template <typename R, bool ZT, int MODE>
-__global__ void __launch_bounds__(LINE_T, LineBounds<R>::blocks) k_line(Phys ph, Sweep sw, FastOps op, LineGeo g,
+template <typename R, bool ZT, int MODE, int RMAX>
+__global__ void __launch_bounds__(LINE_T, LineBounds<R, MODE, RMAX>::blocks) k_line(Phys ph, Sweep sw, FastOps op, LineGeo g,
                                                                       LineShape sh, int ax) {
-  line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, tile_of(op), gridDim.x);
+  line_body<R, ZT, MODE, RMAX>(ph, sw, op, g, sh, ax, tile_of(op), gridDim.x);
 }
 
 // Batched launch: blockIdx.y selects the instance (structs staged in shared memory).
-template <typename R, bool ZT, int MODE>
-__global__ void __launch_bounds__(LINE_T, LineBounds<R>::blocks) k_line_batch(const Phys* __restrict__ phs,
+template <typename R, bool ZT, int MODE, int RMAX>
+__global__ void __launch_bounds__(LINE_T, LineBounds<R, MODE, RMAX>::blocks) k_line_batch(const Phys* __restrict__ phs,
                                                                             const Sweep* __restrict__ sws,
                                                                             FastOps op, LineGeo g, LineShape sh,
                                                                             int ax) {
@@ -508,7 +520,7 @@ __global__ void __launch_bounds__(LINE_T, LineBounds<R>::blocks) k_line_batch(co
   copy_words(&sw, sws + blockIdx.y);
   __syncthreads();
   if (batch_frozen(sw.live)) return;
-  line_body<R, ZT, MODE>(ph, sw, op, g, sh, ax, tile_of(op), gridDim.x);
+  line_body<R, ZT, MODE, RMAX>(ph, sw, op, g, sh, ax, tile_of(op), gridDim.x);
 }
 
 // host: launch one sweep (one translation unit per precision and group of modes)

@@ -19,10 +19,10 @@ template <typename K> static cudaError_t line_attr(K kern, int& attr_dev) {
   return e;
 }
 
-template <typename R, bool ZT, int MODE>
-cudaError_t line_one(int ax, const Phys& ph, const Sweep& sw, const FastOps& op, const LineGeo& g,
+template <typename R, bool ZT, int MODE, int RMAX>
+cudaError_t line_one_r(int ax, const Phys& ph, const Sweep& sw, const FastOps& op, const LineGeo& g,
                      const LineShape& sh, size_t smem, cudaStream_t st) {
-  constexpr auto kern = &k_line<R, ZT, MODE>;
+  constexpr auto kern = &k_line<R, ZT, MODE, RMAX>;
   static int attr_dev = -1;
   const cudaError_t e = line_attr(kern, attr_dev);
   if (e != cudaSuccess) return e;
@@ -39,15 +39,29 @@ cudaError_t line_one(int ax, const Phys& ph, const Sweep& sw, const FastOps& op,
   return cudaLaunchKernelEx(&cfg, kern, ph, sw, op, g, sh, ax);
 }
 
-template <typename R, bool ZT, int MODE>
-cudaError_t line_batch_one(int ax, const Phys* phs, const Sweep* sws, int count, const FastOps& op,
+template <typename R, bool ZT, int MODE, int RMAX>
+cudaError_t line_batch_one_r(int ax, const Phys* phs, const Sweep* sws, int count, const FastOps& op,
                            const LineGeo& g, const LineShape& sh, size_t smem, cudaStream_t st) {
-  constexpr auto kern = &k_line_batch<R, ZT, MODE>;
+  constexpr auto kern = &k_line_batch<R, ZT, MODE, RMAX>;
   static int attr_dev = -1;
   const cudaError_t e = line_attr(kern, attr_dev);
   if (e != cudaSuccess) return e;
   kern<<<dim3((unsigned)sh.tiles, (unsigned)count), sh.T, smem, st>>>(phs, sws, op, g, sh, ax);
   return cudaGetLastError();
+}
+
+// by the largest radix of the geometry
+template <typename R, bool ZT, int MODE>
+cudaError_t line_one(int ax, const Phys& ph, const Sweep& sw, const FastOps& op, const LineGeo& g,
+                     const LineShape& sh, size_t smem, cudaStream_t st) {
+  return g.rmax <= 8 ? line_one_r<R, ZT, MODE, 8>(ax, ph, sw, op, g, sh, smem, st)
+                     : line_one_r<R, ZT, MODE, 16>(ax, ph, sw, op, g, sh, smem, st);
+}
+template <typename R, bool ZT, int MODE>
+cudaError_t line_batch_one(int ax, const Phys* phs, const Sweep* sws, int count, const FastOps& op,
+                           const LineGeo& g, const LineShape& sh, size_t smem, cudaStream_t st) {
+  return g.rmax <= 8 ? line_batch_one_r<R, ZT, MODE, 8>(ax, phs, sws, count, op, g, sh, smem, st)
+                     : line_batch_one_r<R, ZT, MODE, 16>(ax, phs, sws, count, op, g, sh, smem, st);
 }
 
 #define GPE_LINE_ONE(R, ZT, MODE)                                                                               \

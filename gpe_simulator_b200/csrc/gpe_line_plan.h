@@ -20,6 +20,7 @@ struct LineGeo {
   unsigned mg_nb[LINE_PMAX];      // ceil(2^32 / nb) (0: nb = 1)
   int span;                       // shared elements of one line
   int np[LINE_PMAX];              // product of the earlier radices (the prefixes of a butterfly)
+  int rmax;                       // largest radix
   int direct;                     // prime radices 7, 11, 13 by the direct sum (as the Stockham passes)
   const void* bf[LINE_PMAX];      // p > 0: int2 {first position, prefix << 16 | column} of butterfly q
   const void* tw[LINE_PMAX];      // p < P - 1: W^(k column) as [k - 1][column], after the phase
@@ -81,6 +82,7 @@ inline bool line_geometry(int n, const std::vector<int>& r, LineGeo& g) {
   for (int p = 0; p < g.P; ++p) {
     later /= r[p];
     g.r[p] = r[p];
+    g.rmax = std::max(g.rmax, r[p]);
     g.nb[p] = n / r[p];
     g.nl[p] = later;
     g.np[p] = n / (r[p] * later);
