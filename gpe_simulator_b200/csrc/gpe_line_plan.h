@@ -130,7 +130,10 @@ inline int line_threads(const LineGeo& g, int L) {
   return T;
 }
 
-constexpr int LINE_TILES_MIN = 2 * 148;   // at least two blocks per SM where the grid has them
+// At least a block per SM where the grid has them.  (Two per SM were smaller blocks with more
+// partial sums to finish: 35^3 complex64 imaginary time 37.8 -> 33.1 us per step, 60^3 48.9
+// -> 40.4; half a block per SM 38.8 and 37.9, larger sides the same.)
+constexpr int LINE_TILES_MIN = 148;
 
 // z tiles: about 32 KB of consecutive lines, fewer while that leaves SMs without a block.
 inline LineShape line_shape_z(const LineGeo& g, int csize) {

@@ -118,7 +118,8 @@ typedef struct gpe_desc {
      * (0 = FP32 phase evaluation); ignored for complex128 */
     int local_fp64;
     /* sweep path: 0 = fastest available (register-resident sweeps for n = 32, 48,
-     * 64, 96, 128, 160, 256, else generic); 1 = generic mixed-radix sweeps only;
+     * 64, 96, 128, 160, 256 (512 in complex64) compiled, with the side at run time
+     * for every other n of two radices or more, else generic); 1 = generic mixed-radix sweeps only;
      * 2 = same as 0; 3 = complex64 n = 128, 256: the y and z sweeps of each
      * x-plane fused into one persistent launch (psi crosses HBM once per launch
      * instead of once per sweep; identical results, measured slower on B200
