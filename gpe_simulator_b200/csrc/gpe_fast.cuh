@@ -1173,10 +1173,8 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
 // Resident blocks per SM that the register allocation must allow, 0 = the
 // compiler's choice.  Measured for complex64 at n = 128, 256: the plain FFT
 // sweeps are memory-bound and want 1024 threads per SM (64 registers at
-// T = 256); the fused modes keep 768 (80 registers) for their extra live state,
-// except Z21 and XKIN at n = 256, which run 4 blocks of 64 registers (a few
-// hundred bytes of spills in Z21): 4486 -> 4541 steps/s at 256^3, the gain
-// being in the overlap of the programmatically launched sweeps.
+// T = 256).  (The modes with pointwise work at n = 256 take two lines per thread,
+// gpe_packed.cuh.)
 // At n = 128 the fused modes run 7 blocks of 72 registers: a 128^3 sweep is 1024 tiles, one
 // wave of 7 x 148 = 1036 blocks but 1.15 waves of 6 (imaginary time 51.0 -> 45.8 us per
 // step, stirred 35.1 -> 31.9; 8 blocks of 64 registers 46.0, 32.4).
@@ -1188,8 +1186,7 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
 template <int N, typename R, int MODE> struct FastBounds {
   static constexpr int value = (sizeof(R) == 4 && (N == 128 || N == 256))
                                    ? (MODE == FM_PLAIN ? 1024 : MODE == FM_DIAGR ? 512
-                                      : N == 128 && MODE != FM_DIAGK ? 896 : (N == 256 && (MODE == FM_Z21 || MODE == FM_XKIN)) ? 1024 : 768) /
-                                         FastCfg<N, R>::T
+                                      : MODE == FM_DIAGK ? 768 : 896) / FastCfg<N, R>::T
                                : (sizeof(R) == 4 && N == 512)
                                    ? (MODE == FM_DIAGR ? 512 : 1024) / FastCfg<N, R>::T : 0;
 };

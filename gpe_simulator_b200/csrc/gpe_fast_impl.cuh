@@ -7,8 +7,8 @@
 
 namespace gpe {
 
-// the kernel of (N, AX, R, MODE), its threads and shared memory: the 512-point
-// complex64 sweeps take two lines per thread; explicit occupancy bounds where measured
+// the kernel of (N, AX, R, MODE), its threads and shared memory: the 256- and
+// 512-point complex64 sweeps of steps take two lines per thread; explicit occupancy bounds where measured
 template <int N, int AX, typename R, int MODE, bool TR> struct FastKernel {
   static constexpr bool PACK = sizeof(R) == 4 && !TR && pack_sweep(N, MODE);
   static constexpr int T = PACK ? PackCfg<N>::T : FastCfg<N, R>::T;

@@ -67,12 +67,11 @@ template <bool INV> __device__ __forceinline__ C2 rot2(C2 v, float ch, float cl,
             fma2(v.y, f2(ch), fma2(v.x, f2(-sh), fma2(v.y, f2(cl), v.x * f2(-sl)))));
 }
 
-// twiddle-table entry of both lines: hi.x, hi.y and lo.x, lo.y, each twice
-struct TwP { float4 hi, lo; };
-
-// v * w (INV: v * conj(w)) for w = hi + lo
-template <bool INV> __device__ __forceinline__ C2 tw2(C2 v, const float4& h, const float4& l) {
-  const F2 wx = f2(h.x, h.y), wy = f2(h.z, h.w), lx = f2(l.x, l.y), ly = f2(l.z, l.w);
+// v * w (INV: v * conj(w)) for a twiddle {hi.x, hi.y, lo.x, lo.y}, the same for both lines.
+// (Entries stored as pairs saved the copies into pairs but doubled the shared-memory reads,
+// which bound the z sweeps.)
+template <bool INV> __device__ __forceinline__ C2 tw2(C2 v, const float4& w) {
+  const F2 wx = f2(w.x), wy = f2(w.y), lx = f2(w.z), ly = f2(w.w);
   if (INV) {
     const F2 nx = -v.x;
     return c2(fma2(v.x, wx, fma2(v.y, wy, fma2(v.x, lx, v.y * ly))),

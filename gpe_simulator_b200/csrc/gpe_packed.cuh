@@ -25,9 +25,9 @@ template <int N> struct PackCfg {
   // exchange buffer (16-byte elements)
   static constexpr int EX = THREE ? LP * N : LP * (N + (N1 > N2 ? N1 : N2));
   static constexpr size_t EXB = (size_t)EX * 16;
-  // twiddles: hi and lo of the split (N1 lanes, N2 values), then of (N2, N1) when that differs
-  // (n = 512: of the 64 second-phase ones)
-  static constexpr int TW = 2 * N + (THREE ? 128 : N1 == N2 ? 0 : 2 * N);
+  // twiddles of the split (N1 lanes, N2 values), then of (N2, N1) when that differs (n = 512:
+  // the 64 second-phase ones)
+  static constexpr int TW = N + (THREE ? 64 : N1 == N2 ? 0 : N);
   // tables of a z sweep: reduction scratch, vz, c1, c2, c12; of an x sweep: kx, kyz, kx2, kyz2
   static constexpr size_t ZB = 32 * 16 + (size_t)(N + 3 * L) * 4, XB = (size_t)(N + L) * 24;
 };
@@ -67,11 +67,9 @@ __device__ __forceinline__ C2 ex_load(const ulonglong2* p) {
   return v;
 }
 
-// fft_2phase of gpe_fast.cuh on line pairs; th, tl: hi and lo entries of this split's
-// twiddles, [k2*A + lane].
+// fft_2phase of gpe_fast.cuh on line pairs; tw: this split's twiddles, [k2*A + lane].
 template <int N, int A, int B, int AX, int QA, int QB, int V, bool INV, bool TAIL>
-__device__ __forceinline__ void pack_2phase(C2 (&v)[V], ulonglong2* ex, const float4* th,
-                                            const float4* tl) {
+__device__ __forceinline__ void pack_2phase(C2 (&v)[V], ulonglong2* ex, const float4* tw) {
   constexpr int LP = PackCfg<N>::LP, T = PackCfg<N>::T;
   static_assert(QA * B <= V && QB * A <= V, "register array too small");
   constexpr bool WARP_LOCAL = AX == FZ && A == B && QA == 1 && QB == 1 && 32 % A == 0 && LP * A == T;
@@ -83,7 +81,7 @@ __device__ __forceinline__ void pack_2phase(C2 (&v)[V], ulonglong2* ex, const fl
     C2* x = v + s * B;
     Dft2<B, INV>::run(x);
 #pragma unroll
-    for (int k2 = 1; k2 < B; ++k2) x[k2] = tw2<INV>(x[k2], th[k2 * A + lane], tl[k2 * A + lane]);
+    for (int k2 = 1; k2 < B; ++k2) x[k2] = tw2<INV>(x[k2], tw[k2 * A + lane]);
 #pragma unroll
     for (int k2 = 0; k2 < B; ++k2)
       ex_store(ex + (AX == FZ ? (lp * B + k2) * (A + 1) + lane : (k2 * A + lane) * LP + lp), x[k2]);
@@ -107,9 +105,7 @@ __device__ __forceinline__ void pack_2phase(C2 (&v)[V], ulonglong2* ex, const fl
 
 // fft_3phase of gpe_fast.cuh on line pairs (n = 512).
 template <int N, int AX, int Q, int V, bool INV, bool TAIL>
-__device__ __forceinline__ void pack_3phase(C2 (&v)[V], ulonglong2* ex, const float4* tah,
-                                            const float4* tal, const float4* tbh,
-                                            const float4* tbl) {
+__device__ __forceinline__ void pack_3phase(C2 (&v)[V], ulonglong2* ex, const float4* twa, const float4* twb) {
   constexpr int LP = PackCfg<N>::LP, T = PackCfg<N>::T;
   constexpr int RD = 8, A = 64;
   static_assert(N == RD * RD * RD && Q * RD <= V && Q * T == LP * A, "three-phase layout");
@@ -126,7 +122,7 @@ __device__ __forceinline__ void pack_3phase(C2 (&v)[V], ulonglong2* ex, const fl
     C2* x = v + s * RD;
     Dft2<RD, INV>::run(x);
 #pragma unroll
-    for (int k3 = 1; k3 < RD; ++k3) x[k3] = tw2<INV>(x[k3], tah[k3 * A + p], tal[k3 * A + p]);
+    for (int k3 = 1; k3 < RD; ++k3) x[k3] = tw2<INV>(x[k3], twa[k3 * A + p]);
 #pragma unroll
     for (int k3 = 0; k3 < RD; ++k3) ex_store(ex + e1(lp, k3, p), x[k3]);
   }
@@ -148,9 +144,9 @@ __device__ __forceinline__ void pack_3phase(C2 (&v)[V], ulonglong2* ex, const fl
     const int p1 = q0 & 7;   // (the same in every slot of a thread: slots are 32 lanes apart)
 #pragma unroll
     for (int k1 = 1; k1 < RD; ++k1) {
-      const float4 h = tbh[k1 * RD + p1], l = tbl[k1 * RD + p1];
+      const float4 w = twb[k1 * RD + p1];
 #pragma unroll
-      for (int s = 0; s < Q; ++s) v[s * RD + k1] = tw2<INV>(v[s * RD + k1], h, l);
+      for (int s = 0; s < Q; ++s) v[s * RD + k1] = tw2<INV>(v[s * RD + k1], w);
     }
   }
 #pragma unroll
@@ -393,10 +389,8 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
   tb.c1 = tb.vz + N;
   tb.c2 = tb.c1 + L;
   tb.c12 = tb.c2 + L;
-  const float4* t1h = tw;
-  const float4* t1l = t1h + N;
-  const float4* t2h = N1 == N2 ? t1h : t1l + N;
-  const float4* t2l = t2h + (THREE ? 64 : N);
+  const float4* t1 = tw;
+  const float4* t2 = N1 == N2 ? t1 : t1 + N;
   // (plan constants: copied past the registers, in flight with the tile's loads)
   for (int q = threadIdx.x; q < PackCfg<N>::TW; q += PackCfg<N>::T) cp_async16(tw + q, (const float4*)sw.twp + q);
   const FastTile<N, AX, float> tl(tile);
@@ -423,8 +417,8 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
   }
   auto first = [&](auto inv) {
     constexpr bool INV = decltype(inv)::value;
-    if constexpr (THREE) pack_3phase<N, AX, S1, V_, INV, TWO_FFT>(v, ex, t1h, t1l, t2h, t2l);
-    else pack_2phase<N, N1, N2, AX, S1, S2, V_, INV, TWO_FFT>(v, ex, t1h, t1l);
+    if constexpr (THREE) pack_3phase<N, AX, S1, V_, INV, TWO_FFT>(v, ex, t1, t2);
+    else pack_2phase<N, N1, N2, AX, S1, S2, V_, INV, TWO_FFT>(v, ex, t1);
   };
   using std::integral_constant;
   if constexpr (MODE == FM_Z2 || MODE == FM_Z21) {
@@ -449,8 +443,8 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
       pack_kin<N, LM, VM, SM, V_, false, false>(v, ph, tb);
     }
     constexpr bool INV = MODE == FM_XKIN;
-    if constexpr (THREE) pack_3phase<N, AX, S1, V_, INV, false>(v, ex, t1h, t1l, t2h, t2l);
-    else pack_2phase<N, N2, N1, AX, S2, S1, V_, INV, false>(v, ex, t2h, t2l);
+    if constexpr (THREE) pack_3phase<N, AX, S1, V_, INV, false>(v, ex, t1, t2);
+    else pack_2phase<N, N2, N1, AX, S2, S1, V_, INV, false>(v, ex, t2);
     pack_store<N, AX, N1, N2, S1>(v, tl, (float2*)sw.dst, vec);
   } else {
     if constexpr (MODE == FM_Z2) pack_half_dispatch<N, LM, VM, SM>(v, tl, ph, tb);
@@ -484,7 +478,8 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
 
 // Resident blocks per SM asked of the register allocation: 512 threads at 128 registers
 // (two lines of 16 values take 64).  With 96 or 80 registers (640, 768 threads) the loads of
-// a tile no longer fit in flight together: 512^3 2111 -> 2806 us per step at 768.
+// a tile no longer fit in flight together: 512^3 2111 -> 2806 us per step at 768.  (2111 was with twiddle
+// entries twice the size; 1944 now.)
 template <int N, int MODE> struct PackBounds {
   static constexpr int value = 512 / PackCfg<N>::T;
 };
@@ -508,13 +503,14 @@ k_pack_batch(const Phys* __restrict__ phs, const Sweep* __restrict__ sws, FastOp
   pack_body<N, AX, MODE>(ph, sw, op, tile_of(op), gridDim.x);
 }
 
-// Sweeps that take two lines per thread: the steps at n = 512 (transforms and reductions
-// keep one line per thread, and with it their results to the last bit).  Per step at 512^3 (real time, stirred):
-// 2294 -> 2111 us (two steps of one call 5049 -> 4634), z 589 -> 562, y 427 -> 400, x 770 -> 713.  Not below: at n = 256 the
-// instructions fall just as much (fused z sweep 53.4 -> 34.7 M per launch) but with 16
-// warps per SM instead of 32 the time does not (z 74, y 46, x 74 us either way), and at
-// n = 128 a step took 39.7 us against 34.7.
+// Sweeps that take two lines per thread: the steps' at n = 512; at n = 256 the fused z sweep and
+// the x sweep (transforms, reductions and the y sweeps at 256, which HBM bounds, keep one line
+// per thread; so do Z1 and Z2 there, which run the arithmetic of the plane-fused launches to
+// the last bit).  Per step, 512^3 stirred 2294 -> 1944 us (z 589 -> 501, y 427 -> 377, x 770 -> 696);
+// 256^3 stirred 207.8 -> 199.9 (z 69.2 -> 62.7, x 70.0 -> 66.1).  At n = 128 there are too few
+// warps for it: 31.9 -> 36.8.
 constexpr bool pack_sweep(int n, int mode) {
+  if (n == 256) return mode == FM_Z21 || mode == FM_XKIN;
   return n == 512 && (mode == FM_PLAIN || mode == FM_Z1 || mode == FM_Z2 || mode == FM_Z21 || mode == FM_XKIN);
 }
 

@@ -832,7 +832,7 @@ struct gpe_plan {
   double* d_line = nullptr;
   void* d_ltab = nullptr;          // [2][n*n] per-line dynamic potential (line form), precision of psi
   void* d_tw = nullptr;
-  void* d_twp = nullptr;         // packed complex64 sweeps (n = 512): twiddles in lane order
+  void* d_twp = nullptr;         // packed complex64 sweeps (n = 256, 512): twiddles in lane order
   double* d_partial = nullptr;   // 2 areas of 4*max_tiles doubles
   unsigned* d_ticket = nullptr;
   unsigned* d_plane = nullptr;   // plane-fused launches: ticket, finished blocks, per (plane, stage) counts
@@ -1484,21 +1484,24 @@ int make_tables(gpe_plan* p, const gpe_desc* d, Tables& tabs) {
       ls.off_bf[q] = bf0[q] * sizeof(int);
     }
   }
-  // packed sweeps: entries (hi.x, hi.x, hi.y, hi.y), then the residuals, [value][lane]: the
-  // first phase's W_512^(p k3), then the second's W_64^(p1 k1)
+  // packed sweeps: entries {hi, lo}, [value][lane]: n = 512 the first phase's W_512^(p k3), then
+  // the second's W_64^(p1 k1); n = 256 W_256^(n1 k2)
   if constexpr (sizeof(R) == 4) {
-    if (n == 512) {
+    if (n == 512 || n == 256) {
       std::vector<float4> tp;
       auto table = [&](int lanes, int vals, int stride) {
-        for (int part = 0; part < 2; ++part)
-          for (int k = 0; k < vals; ++k)
-            for (int l = 0; l < lanes; ++l) {
-              const float2 w = (part ? twl : tw)[stride * k * l];
-              tp.push_back(make_float4(w.x, w.x, w.y, w.y));
-            }
+        for (int k = 0; k < vals; ++k)
+          for (int l = 0; l < lanes; ++l) {
+            const int e = stride * k * l;
+            tp.push_back(make_float4(tw[e].x, tw[e].y, twl[e].x, twl[e].y));
+          }
       };
-      table(64, 8, 1);
-      table(8, 8, 8);
+      if (n == 512) {
+        table(64, 8, 1);
+        table(8, 8, 8);
+      } else {
+        table(16, 16, 1);
+      }
       tabs.put(&p->d_twp, tp.data(), tp.size() * sizeof(tp[0]));
     }
   }
