@@ -2226,7 +2226,7 @@ int gpe_status(gpe_plan* p, int* flags, void* stream) {
 
 // ================================================================ batches
 // Many independent imaginary-time solves of mixed grid sizes advanced together.
-// Instances are grouped by grid size; every sweep of a step is one launch per
+// Instances are grouped by grid size, kind and sweep family; every sweep of a step is one launch per
 // group whose grid is (tiles, instances): blockIdx.y picks the instance, whose
 // physics and pointers come from device arrays.  One Strang step of all groups
 // is captured once as a CUDA graph with one parallel branch per group and
@@ -2286,10 +2286,12 @@ enum { ROLE_Z1N = 0, ROLE_Z1, ROLE_Y1, ROLE_X, ROLE_Y2, ROLE_Z2, ROLE_SC, ROLE_D
 // steps of a real-time group's time table per upload (longer calls are chunked)
 constexpr int BATCH_CLOCK_STEPS = 1024;
 
-// Group of (grid size, kind), created on first use.
+// Group of (grid size, kind, sweep family), created on first use.  (An accuracy mode or
+// generic_only puts an instance on the Stockham sweeps: they carry those modes, and their
+// tiles and shared memory are not the register-resident sweeps'.)
 int batch_group(gpe_batch* b, const gpe_plan* p, bool make_streams) {
   for (size_t q = 0; q < b->groups.size(); ++q)
-    if (b->groups[q].n == p->n && b->groups[q].kind == p->kind) return (int)q;
+    if (b->groups[q].n == p->n && b->groups[q].kind == p->kind && b->groups[q].fast == p->fast) return (int)q;
   gpe_batch::Group g;
   g.n = p->n;
   g.kind = p->kind;
