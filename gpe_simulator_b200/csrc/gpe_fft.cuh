@@ -294,10 +294,35 @@ template <int B, int E> struct SFor {
   }
 };
 
-// R = R1*R2 from two smaller DFTs with compile-time twiddles W_R^(n2 k1).
+// R = R1*R2 from two smaller DFTs.  complex64: compile-time twiddles W_R^(n2 k1) between them
+// (split constants; the rounding that complex64 transforms have always had).  complex128
+// with R1, R2 coprime: I. J. Good's index maps ("The interaction algorithm and practical
+// Fourier analysis", 1958), n = R2 n1 + R1 n2, k1 = k mod R1, k2 = k mod R2 (all mod R), with
+// no twiddles and so without their rounding.
 template <int R1, int R2, typename D1 = Dft<R1>, typename D2 = Dft<R2>> struct DftSplitG {
+  static constexpr bool coprime(int a, int b) { return b == 0 ? a == 1 : coprime(b, a % b); }
   template <typename C> __device__ __forceinline__ static void run(C* v, const C* tw, const C* twl, int unused) {
     C y[R2][R1];
+    if constexpr (sizeof(C) == 16 && coprime(R1, R2)) {
+      constexpr int R = R1 * R2;
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) {
+#pragma unroll
+        for (int n1 = 0; n1 < R1; ++n1) y[n2][n1] = v[(R2 * n1 + R1 * n2) % R];
+        D1::run(y[n2], tw, twl, unused);
+      }
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) {
+        C z[R2];
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) z[n2] = y[n2][k1];
+        D2::run(z, tw, twl, unused);
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+          if (k % R1 == k1) v[k] = z[k % R2];
+      }
+      return;
+    }
     SFor<0, R2>::run([&](auto n2c) {
       constexpr int n2 = decltype(n2c)::value;
 #pragma unroll
