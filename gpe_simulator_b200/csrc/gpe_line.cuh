@@ -282,7 +282,6 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
         line_half<R, false, RAD>(ph, lc, v, l, q, nb);
       }
       if (MODE == FM_DIAGR) {
-        double n0 = 0.0, n1 = 0.0, n2 = 0.0;
 #pragma unroll
         for (int a = 0; a < RAD; ++a) {
           const int m = q + a * nb;
@@ -291,13 +290,10 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
           if (ph.vre) V += ((const R*)ph.vre)[lc.row0 + (long long)l * n + m];
           if (ph.kind == 1 && ph.beam) V += (R)ph.beam_amp * c12[l];
           if (lc.vd1) V += lc.vd1[lc.row0 + (long long)l * n + m];
-          n0 += rho;
-          n1 = fma((double)V, rho, n1);
-          n2 = fma(rho, rho, n2);
+          cx.acc[0].add(rho);
+          cx.acc[1].add((double)V * rho);
+          cx.acc[2].add(rho * rho);
         }
-        cx.acc[0].add(n0);
-        cx.acc[1].add(n1);
-        cx.acc[2].add(n2);
       }
       line_dft<RAD, DIRECT>(g, v);
       if (!DIT) {
@@ -394,31 +390,24 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
         if (MODE == FM_Z2) {
           line_half<R, false, RAD>(ph, lc, v, l, q, nb);
           if (op.norm) {
-            double sum = 0.0;
 #pragma unroll
-            for (int a = 0; a < RAD; ++a)
-              sum = fma((double)v[a].x, (double)v[a].x, fma((double)v[a].y, (double)v[a].y, sum));
-            cx.acc[0].add(sum);
+            for (int a = 0; a < RAD; ++a) cx.acc[0].add((double)v[a].x * v[a].x + (double)v[a].y * v[a].y);
           }
         }
         if (MODE == FM_DIAGK) {
-          double e = 0.0;
 #pragma unroll
           for (int a = 0; a < RAD; ++a) {
             const double kk = kk_ref(ph.k[q + a * nb], ph.k[a0], ph.k[z0 + l]);
             const double w = (double)v[a].x * v[a].x + (double)v[a].y * v[a].y;
-            e = fma(kk, w, e);
+            cx.acc[3].add(kk * w);
             if (sw.hist)
               atomicAdd(hist + (l & (copies - 1)) * sw.nbins + shell_of(kk, sw.shell_t, sw.inv_shell, sw.nbins), w);
           }
-          cx.acc[3].add(e);
         } else if (MODE == FM_LZ) {
           // y sweep: sum x k_y |v|^2; x sweep: sum y k_x |v|^2 (a0 is the other axis' index)
-          double e = 0.0;
 #pragma unroll
           for (int a = 0; a < RAD; ++a)
-            e = fma(ph.k[q + a * nb], (double)v[a].x * v[a].x + (double)v[a].y * v[a].y, e);
-          cx.acc[3].add(ph.x[a0] * e);
+            cx.acc[3].add(ph.x[a0] * ph.k[q + a * nb] * ((double)v[a].x * v[a].x + (double)v[a].y * v[a].y));
         } else {
           C* p = dst + base + (long long)l * lstride + (long long)q * nstride;
           const long long st = (long long)nb * nstride;

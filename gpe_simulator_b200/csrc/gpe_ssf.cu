@@ -503,9 +503,9 @@ __global__ void __launch_bounds__(256) k_scale(Sweep sw, long long count) {
 }
 
 // Norm of a state into the plan's scale: a streaming read (8 loads in flight per thread,
-// summed in plain FP64 in a fixed order, then compensated across threads and blocks).
-// Bound by HBM; the no-transform Stockham sweep it replaces staged every element through
-// shared memory with a division for its coordinates: 53 us at 128^3 complex128.
+// every element added with compensation).  Bound by HBM; the no-transform Stockham sweep it
+// replaces staged every element through shared memory with a division for its coordinates:
+// 53 us at 128^3 complex128.
 constexpr int NORM_UNROLL = 8;
 template <typename R>
 __global__ void __launch_bounds__(256) k_norm(Phys ph, Sweep sw, long long count) {
@@ -518,11 +518,8 @@ __global__ void __launch_bounds__(256) k_norm(Phys ph, Sweep sw, long long count
     C v[NORM_UNROLL];
 #pragma unroll
     for (int q = 0; q < NORM_UNROLL; ++q) v[q] = e0 + q * 256 < count ? psi[e0 + q * 256] : mk((R)0, (R)0);
-    double sum = 0.0;
 #pragma unroll
-    for (int q = 0; q < NORM_UNROLL; ++q)
-      sum = fma((double)v[q].x, (double)v[q].x, fma((double)v[q].y, (double)v[q].y, sum));
-    a[0].add(sum);
+    for (int q = 0; q < NORM_UNROLL; ++q) a[0].add((double)v[q].x * v[q].x + (double)v[q].y * v[q].y);
   }
   block_merge<1>(a, red);
   norm_finish(ph, sw, a[0], red);
