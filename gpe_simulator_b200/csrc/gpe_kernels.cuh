@@ -115,13 +115,16 @@ struct LineSlots {
 // a / d for d's correctly rounded reciprocal r: one Newton correction of a*r by its exact
 // remainder gives the correctly rounded quotient (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990) in three operations instead of
-// a division per component.  A reciprocal that is zero or not finite (a norm that is
-// not) takes the division itself, which then gives what it always gave.
+// a division per component.  The remainder is taken as q d - a, so that a zero keeps its
+// sign.  For components below 2^-968 the remainder underflows and the quotient can be a unit
+// in the last place off (a test for them cost 2% of an imaginary step at 64^3).  A
+// reciprocal that is zero or not finite (a norm that is not) takes the division itself,
+// which then gives what it always gave.
 static __device__ __noinline__ double div_far(double a, double d) { return a / d; }
 __device__ __forceinline__ double div_by(double a, double d, double r) {
   if (!(fabs(r) > 0.0 && fabs(r) <= 1.7976931348623157e308)) return div_far(a, d);
   const double q = a * r;
-  return fma(fma(-q, d, a), r, q);
+  return fma(-fma(q, d, -a), r, q);
 }
 
 __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
