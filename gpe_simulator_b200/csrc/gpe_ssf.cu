@@ -826,6 +826,7 @@ struct gpe_plan {
   void* d_ptab = nullptr;
   double pt_t[2] = {0.0, 0.0};
   bool pt_ok[2] = {false, false};
+  cudaEvent_t tab_ev = nullptr;    // plans with line or point tables: end of the call that used them last
   double* d_line = nullptr;
   void* d_ltab = nullptr;          // [2][n*n] per-line dynamic potential (line form), precision of psi
   void* d_tw = nullptr;
@@ -1213,6 +1214,29 @@ struct PdlChain {
   ~PdlChain() { p->pdl_chain = false; p->pdl_prev = false; p->pt_ok[0] = p->pt_ok[1] = false; }
 };
 
+// The line and point tables are the plan's: a call that writes them waits for the one before
+// on whatever stream that ran, so that calls on several streams keep their order on them
+// (steps without tables share nothing in real time and need none).  A captured call cannot
+// take part in that: its replays come at any time, beside other calls.  It runs on the
+// Stockham sweeps, which evaluate the potential per point and share nothing (line tables of
+// compiled sides stay: replays of those are the caller's to order).
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) { cudaGetLastError(); return false; }
+  return s != cudaStreamCaptureStatusNone;
+}
+struct TableUse {
+  gpe_plan* p;
+  cudaStream_t st;
+  cudaError_t err = cudaSuccess;
+  TableUse(gpe_plan* q, cudaStream_t s, bool captured) : p(captured ? nullptr : q), st(s) {
+    if (p && p->tab_ev) err = cudaStreamWaitEvent(st, p->tab_ev, 0);
+  }
+  ~TableUse() {
+    if (p && p->tab_ev && err == cudaSuccess) cudaEventRecord(p->tab_ev, st);
+  }
+};
+
 Sweep mk_sweep(const void* src, void* dst) {
   Sweep s;
   memset(&s, 0, sizeof(s));
@@ -1557,6 +1581,7 @@ int build_static(gpe_plan* p, const void* v, int v_kind, cudaStream_t st) {
 void free_plan(gpe_plan* p) {
   for (auto& r : p->recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   for (auto e : p->pool) cudaEventDestroy(e);
+  if (p->tab_ev) cudaEventDestroy(p->tab_ev);
   // (the tables share one allocation)
   void* bufs[] = {p->d_tables, p->d_vre, p->d_vim, p->d_hist, p->d_work, p->d_proj, p->d_ptab};
   for (void* b : bufs)
@@ -1627,6 +1652,7 @@ int create(const gpe_desc* d, gpe_plan** out) {
   if (rc != GPE_OK) { free_plan(p); return rc; }
   bind_line_tables(p);
   p->pprog.base = p->d_pprog;
+  if (p->has_point || p->d_ltab) CU(cudaEventCreateWithFlags(&p->tab_ev, cudaEventDisableTiming));
   {
     // modes per shell, on the device (the host loop over n^3 modes took 60 ms at 256^3)
     const size_t smem = (size_t)p->nbins * sizeof(unsigned);
@@ -2020,6 +2046,9 @@ int gpe_step(gpe_plan* p, void* psi, int nsteps, long long step0, void* stream) 
   if (nsteps < 0) return fail(GPE_ERR_ARG, "nsteps must be >= 0");
   cudaStream_t st = (cudaStream_t)stream;
   const bool imag = p->kind == GPE_IMAGINARY;
+  const bool captured = p->tab_ev && capturing(st), fast = p->fast && !(captured && !p->fixed);
+  TableUse tables(p, st, captured);
+  CU(tables.err);
   PdlChain chain(p);
   if (p->plane && nsteps > 0) {
     // per step: XKIN, then one plane-fused launch [inverse y, z, forward y]; the
@@ -2049,7 +2078,7 @@ int gpe_step(gpe_plan* p, void* psi, int nsteps, long long step0, void* stream) 
     if (imag) TRY(scale_sweep(p, psi, st));
     return GPE_OK;
   }
-  if (p->fast && nsteps > 0) {
+  if (fast && nsteps > 0) {
     // real time fuses each step's last z sweep with the next step's first
     TRY(fast_front(p, psi, t_mid_host(p, step0), false, st,
                    p->has_point && nsteps > 1 ? t_mid_host(p, step0 + 1) : 0.0));
@@ -2073,8 +2102,11 @@ int gpe_step_at(gpe_plan* p, void* psi, double t, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   // reference: t_mid = float(t) + dt/2 (gpe/make_propagator.py:94)
   const double tm = t + p->dt / 2;
+  const bool captured = p->tab_ev && capturing(st), fast = p->fast && !(captured && !p->fixed);
+  TableUse tables(p, st, captured);
+  CU(tables.err);
   PdlChain chain(p);
-  if (p->fast) {
+  if (fast) {
     TRY(fast_front(p, psi, tm, false, st));
     TRY(fast_middle(p, psi, st));
     TRY(fast_back(p, psi, tm, tm, false, st));
@@ -2146,6 +2178,8 @@ int gpe_diagnostics(gpe_plan* p, const void* psi, double t, double* scalars, dou
   cudaStream_t st = (cudaStream_t)stream;
   TRY(ensure_work(p));
   TRY(ensure_hist(p));
+  TableUse tables(p, st, false);
+  CU(tables.err);
   const bool hist = nk != nullptr;
   TRY(diag_launch(p, psi, t, hist, st));
   int na = 0, nb = 0;
