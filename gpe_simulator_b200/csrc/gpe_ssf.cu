@@ -620,15 +620,15 @@ struct PointProg {
 constexpr int POINT_ROWS = 16;     // rows (x, y) of a block
 constexpr int POINT_LANES = 4;     // points a thread evaluates together
 
-// V(x, y, z, t) of every point at up to two times: blockIdx.y picks the time.  A block
-// evaluates its rows' values and the z values once (FP64, in shared memory), then runs the
+// V(x, y, z, t) of the points of `rows` rows from row0 on at up to two times: blockIdx.y picks
+// the time.  A block evaluates its rows' values and the z values once (FP64, in shared memory), then runs the
 // residual program over its rows, four points per thread so that decoding an operation is
 // paid once for four.  Bound by FP64 issue and the residual's operations.  Before, the
 // whole program ran per point and half-step inside the Stockham z sweeps: five steps of a
 // formula moving a plug along z at 105^3 complex128 took 3518 us, now 528 us.
 template <typename R>
 __global__ void __launch_bounds__(128) k_point_table(PointProg pp, const double* __restrict__ x, int n,
-                                                     LineSlots sl, R* tab1, R* tab2) {
+                                                     LineSlots sl, int row0, int rows, R* tab1, R* tab2) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ double sh[];
   double* zt = sh;                                  // [nz][n]
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(128) k_point_table(PointProg pp, const double*
   double* prog = rt + (size_t)pp.nrow * POINT_ROWS; // residual program
   const double* slots = blockIdx.y ? sl.s2 : sl.s1;
   R* tab = blockIdx.y ? tab2 : tab1;
-  const int r0 = blockIdx.x * POINT_ROWS, nr = min(POINT_ROWS, n * n - r0);
+  const int b0 = blockIdx.x * POINT_ROWS, nr = min(POINT_ROWS, rows - b0), r0 = row0 + b0;
   for (int q = threadIdx.x; q < pp.nz * n; q += blockDim.x) {
     const int k = q / n, z = q - k * n;
     zt[q] = eval_program(pp.base + pp.z_off[k], pp.z_len[k], 0.0, 0.0, x[z], 0.0, slots);
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(128) k_point_table(PointProg pp, const double*
     }
 #pragma unroll
     for (int a = 0; a < POINT_LANES; ++a)
-      if (zq + a * per_row < n) tab[(long long)g * n + zq + a * per_row] = (R)st[0][a];
+      if (zq + a * per_row < n) tab[(long long)(b0 + r) * n + zq + a * per_row] = (R)st[0][a];
   }
 }
 
@@ -818,12 +818,14 @@ struct gpe_plan {
   double* d_prog_g = nullptr;
   double* d_dyn = nullptr;
   // dynamic potential with z terms: its point form, the programs on the device, and its
-  // values [2][n^3] at two times (pt_t; the first pt_n hold within the current call)
+  // values at two times, [2][pt_rows][n]: whole (pt_rows = n^2, at the times pt_t where pt_ok
+  // within the current call), or of the piece of rows that is swept next
   PointForm point;
   bool has_point = false;
   PointProg pprog{};
   double* d_pprog = nullptr;
   void* d_ptab = nullptr;
+  int pt_rows = 0;
   double pt_t[2] = {0.0, 0.0};
   bool pt_ok[2] = {false, false};
   cudaEvent_t tab_ev = nullptr;    // plans with line or point tables: end of the call that used them last
@@ -964,10 +966,45 @@ int line_table(gpe_plan* p, double t1, double t2, bool two, cudaStream_t st) {
   return GPE_OK;
 }
 
-// The point tables of the next z sweep: slots of d_ptab with the potential at t1 (and t2),
-// evaluating what the two slots do not hold yet in one launch.  Like the line table, inside
-// a step sequence a programmatic dependent of the sweep before it, and the z sweep after it
-// is one of it.
+// One launch of k_point_table: rows [row0, row0 + rows) at `first` into table slot a and, if
+// b >= 0, at `second` into slot b.  Like the line table, inside a step sequence a programmatic
+// dependent of the sweep before it, and the z sweep after it is one of it.
+int point_launch(gpe_plan* p, double first, int a, double second, int b, int row0, int rows, cudaStream_t st) {
+  LineSlots sl;
+  memset(&sl, 0, sizeof(sl));
+  auto fill = [&](double* s, double t) {
+    for (size_t k = 0; k < p->point.slots.size(); ++k) s[k] = host_eval(p->point.slots[k], 0.0, 0.0, 0.0, t);
+    s[GPE_LINE_SLOTS - 1] = t;
+  };
+  fill(sl.s1, first);
+  fill(sl.s2, second);
+  const size_t bytes = (size_t)p->pt_rows * p->n * (p->dtype == GPE_C64 ? 4 : 8);
+  char* ta = (char*)p->d_ptab + a * bytes;
+  char* tb = b >= 0 ? (char*)p->d_ptab + b * bytes : ta;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((rows + POINT_ROWS - 1) / POINT_ROWS), b >= 0 ? 2 : 1);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes =
+      ((size_t)p->pprog.nz * p->n + (size_t)p->pprog.nrow * POINT_ROWS + p->pprog.len) * sizeof(double);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
+  const cudaError_t e =
+      p->dtype == GPE_C64 ? cudaLaunchKernelEx(&cfg, k_point_table<float>, p->pprog, (const double*)p->d_x, p->n, sl,
+                                               row0, rows, (float*)ta, (float*)tb)
+                          : cudaLaunchKernelEx(&cfg, k_point_table<double>, p->pprog, (const double*)p->d_x, p->n, sl,
+                                               row0, rows, (double*)ta, (double*)tb);
+  if (e != cudaSuccess) return fail(GPE_ERR_CUDA, std::string("point table: ") + cudaGetErrorString(e));
+  ++p->launches;
+  p->pdl_prev = p->pdl_chain;
+  return GPE_OK;
+}
+
+// Whole point tables of the next z sweep: slots of d_ptab with the potential at t1 (and t2),
+// evaluating what the two slots do not hold yet in one launch.
 int point_tables(gpe_plan* p, double t1, double t2, bool two, Sweep& sw, cudaStream_t st) {
   auto find = [&](double t) { return p->pt_ok[0] && p->pt_t[0] == t ? 0 : p->pt_ok[1] && p->pt_t[1] == t ? 1 : -1; };
   int a = find(t1), b = two ? find(t2) : -1;
@@ -975,45 +1012,16 @@ int point_tables(gpe_plan* p, double t1, double t2, bool two, Sweep& sw, cudaStr
   if (need_a) a = b == 0 ? 1 : 0;
   if (two && t1 == t2) b = a;
   else if (need_b) b = 1 - a;
-  const size_t bytes = (size_t)p->n * p->n * p->n * (p->dtype == GPE_C64 ? 4 : 8);
-  char* tab = (char*)p->d_ptab;
   if (need_a || need_b) {
-    LineSlots sl;
-    memset(&sl, 0, sizeof(sl));
-    auto fill = [&](double* s, double t) {
-      for (size_t k = 0; k < p->point.slots.size(); ++k) s[k] = host_eval(p->point.slots[k], 0.0, 0.0, 0.0, t);
-      s[GPE_LINE_SLOTS - 1] = t;
-    };
-    const int first = need_a ? a : b, second = need_a && need_b ? b : first;
-    fill(sl.s1, need_a ? t1 : t2);
-    fill(sl.s2, t2);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((p->n * p->n + POINT_ROWS - 1) / POINT_ROWS), need_a && need_b ? 2 : 1);
-    cfg.blockDim = dim3(128);
-    cfg.dynamicSmemBytes =
-        ((size_t)p->pprog.nz * p->n + (size_t)p->pprog.nrow * POINT_ROWS + p->pprog.len) * sizeof(double);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
-    const cudaError_t e =
-        p->dtype == GPE_C64
-            ? cudaLaunchKernelEx(&cfg, k_point_table<float>, p->pprog, (const double*)p->d_x, p->n, sl,
-                                 (float*)(tab + first * bytes), (float*)(tab + second * bytes))
-            : cudaLaunchKernelEx(&cfg, k_point_table<double>, p->pprog, (const double*)p->d_x, p->n, sl,
-                                 (double*)(tab + first * bytes), (double*)(tab + second * bytes));
-    if (e != cudaSuccess) return fail(GPE_ERR_CUDA, std::string("point table: ") + cudaGetErrorString(e));
-    ++p->launches;
-    p->pdl_prev = p->pdl_chain;
+    TRY(point_launch(p, need_a ? t1 : t2, need_a ? a : b, t2, need_a && need_b ? b : -1, 0, p->n * p->n, st));
     if (need_a) { p->pt_t[a] = t1; p->pt_ok[a] = true; }
     if (need_b) { p->pt_t[b] = t2; p->pt_ok[b] = true; }
   }
   // (outside a step sequence nothing is kept for a later call)
   if (!p->pdl_chain) p->pt_ok[0] = p->pt_ok[1] = false;
-  sw.vd1 = tab + a * bytes;
-  sw.vd2 = two ? tab + b * bytes : sw.vd1;
+  const size_t bytes = (size_t)p->n * p->n * p->n * (p->dtype == GPE_C64 ? 4 : 8);
+  sw.vd1 = (char*)p->d_ptab + a * bytes;
+  sw.vd2 = two ? (char*)p->d_ptab + b * bytes : sw.vd1;
   return GPE_OK;
 }
 
@@ -1088,19 +1096,9 @@ const CUtensorMap* tma_maps(gpe_plan* p, const void* base, int fax) {
   return &c.map[which];
 }
 
-// Register-resident sweep (n with a fast split); same accounting as sweep().
-int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
-  beam_centres(p, sw);
-  if (p->d_ltab && needs_lines(op.mode)) TRY(line_table(p, sw.t1, sw.t2, op.mode == FM_Z21, st));
-  if (p->has_point && needs_lines(op.mode))
-    TRY(point_tables(p, sw.t1, sw.t2, op.mode == FM_Z21 || (op.mode == FM_Z1 && sw.t2 != 0.0), sw, st));
-  sw.pp = p->pp;
-  sw.tw = p->d_tw;
-  sw.tw_lo = (const char*)p->d_tw + (size_t)p->n * p->csize;
-  sw.twp = p->d_twp;
-  sw.ticket = p->d_ticket;
-  sw.scale = p->d_scale;
-  sw.status = p->d_status;
+// Launch of a sweep whose tables are ready; tiles [tile0, tile0 + ntiles) of a run-time-length
+// sweep (ntiles 0: all).
+int fsweep_launch(gpe_plan* p, int ax, const Sweep& sw, const FastOps& op, int tile0, int ntiles, cudaStream_t st) {
   gpe_plan::Rec r{ax, nullptr, nullptr};
   if (p->prof) {
     r.a = pooled_event(p);
@@ -1110,21 +1108,14 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   const int fax = ax == AX_Z ? FZ : ax == AX_Y ? FY : FX;
   FastOps o = op;
   o.vec = ((uintptr_t)sw.src | (uintptr_t)sw.dst) % 16 == 0;
-  // A sweep takes its tiles in the order opposite to the sweep before it, so that it starts
-  // on what that one left in L2; only the y sweep after an x sweep keeps the x sweep's
-  // order.  256^3 complex64 (134 MB against 126 MB of L2): 225.9 -> 215.1 us per step; every
-  // order measured within 2% of this one but the plain one.  States that fit in L2 with
-  // room for their successor's writes gain nothing and keep the plain order.
-  if (p->pdl_chain && (size_t)p->n * p->n * p->n * p->csize > ((size_t)48 << 20)) {
-    o.rev = p->sweep_dir;
-    if (ax != AX_X) p->sweep_dir ^= 1;
-  }
+  o.tile0 = tile0;
   o.pdl = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
   p->pdl_prev = p->pdl_chain;
   const CUtensorMap* map = p->tma && o.tr != 2 && o.mode == FM_PLAIN && fax != FZ ? tma_maps(p, sw.src, fax) : nullptr;
   const bool line = !p->fixed || o.tr == 2;
   const gpe_plan::LineSet& ls = p->ls[o.tr ? 1 : 0];
-  const LineShape& shape = fax == FZ ? ls.z : ls.p;
+  LineShape shape = fax == FZ ? ls.z : ls.p;
+  if (ntiles) shape.tiles = ntiles;
   const size_t smem = line ? line_smem(ls.geo, shape, (int)p->csize, fax == FZ,
                                       sw.hist ? hist_copies(sw.nbins, LINE_HIST) * sw.nbins : 0)
                           : 0;
@@ -1139,6 +1130,52 @@ int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
   if (p->prof) {
     CU(cudaEventRecord(r.b, st));
     p->recs.push_back(r);
+  }
+  return GPE_OK;
+}
+
+// Register-resident sweep, compiled or run-time-length, with the tables it reads; same
+// accounting as sweep().
+int fsweep(gpe_plan* p, int ax, Sweep sw, const FastOps& op, cudaStream_t st) {
+  beam_centres(p, sw);
+  if (p->d_ltab && needs_lines(op.mode)) TRY(line_table(p, sw.t1, sw.t2, op.mode == FM_Z21, st));
+  sw.pp = p->pp;
+  sw.tw = p->d_tw;
+  sw.tw_lo = (const char*)p->d_tw + (size_t)p->n * p->csize;
+  sw.twp = p->d_twp;
+  sw.ticket = p->d_ticket;
+  sw.scale = p->d_scale;
+  sw.status = p->d_status;
+  FastOps o = op;
+  // A sweep takes its tiles in the order opposite to the sweep before it, so that it starts
+  // on what that one left in L2; only the y sweep after an x sweep keeps the x sweep's
+  // order.  256^3 complex64 (134 MB against 126 MB of L2): 225.9 -> 215.1 us per step; every
+  // order measured within 2% of this one but the plain one.  States that fit in L2 with
+  // room for their successor's writes gain nothing and keep the plain order.
+  if (p->pdl_chain && (size_t)p->n * p->n * p->n * p->csize > ((size_t)48 << 20)) {
+    o.rev = p->sweep_dir;
+    if (ax != AX_X) p->sweep_dir ^= 1;
+  }
+  if (!p->has_point || !needs_lines(op.mode)) return fsweep_launch(p, ax, sw, o, 0, 0, st);
+  const int n = p->n;
+  if (p->pt_rows == n * n) {
+    TRY(point_tables(p, sw.t1, sw.t2, op.mode == FM_Z21 || (op.mode == FM_Z1 && sw.t2 != 0.0), sw, st));
+    return fsweep_launch(p, ax, sw, o, 0, 0, st);
+  }
+  // tables of as many tiles as they hold, then the sweep of these, and on
+  const LineShape& z = p->ls[op.tr ? 1 : 0].z;
+  const bool two = op.mode == FM_Z21;
+  const int most = p->pt_rows / z.L;
+  const size_t row = (size_t)n * (p->dtype == GPE_C64 ? 4 : 8);
+  o.rev = 0;
+  for (int t0 = 0; t0 < z.tiles; t0 += most) {
+    const int nt = std::min(most, z.tiles - t0), row0 = t0 * z.L, rows = std::min(nt * z.L, n * n - row0);
+    TRY(point_launch(p, sw.t1, 0, sw.t2, two ? 1 : -1, row0, rows, st));
+    // (addresses of the cube's element 0 in tables that begin at row0; the sweep reads its
+    // own tiles' elements only)
+    sw.vd1 = (const void*)((uintptr_t)p->d_ptab - row0 * row);
+    sw.vd2 = two ? (const void*)((uintptr_t)p->d_ptab + ((size_t)p->pt_rows - row0) * row) : sw.vd1;
+    TRY(fsweep_launch(p, ax, sw, o, t0, nt, st));
   }
   return GPE_OK;
 }
@@ -1188,7 +1225,7 @@ int psweep(gpe_plan* p, void* psi, int mz, const FastOps* ops, int nstage, int z
 
 FastOps mk_ops(int mode, int inv1 = 0, int invm = 0, int scale = 0, int norm = 0) {
   FastOps o;
-  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.vec = 0; o.rev = 0; o.pf = 0;
+  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.tile0 = 0; o.pdl = 0; o.vec = 0; o.rev = 0; o.pf = 0;
   return o;
 }
 
@@ -1316,18 +1353,26 @@ std::vector<double> shell_starts(double w, int nbins) {
   return t;
 }
 
-// The point tables' memory: taken when the plan is made (a step then allocates nothing, as
-// under stream capture), and only where it is a small part of what is free; without it
-// the potential is evaluated per point in the Stockham sweeps.
-bool point_memory(gpe_plan* p) {
-  const size_t bytes = 2 * (size_t)p->n * p->n * p->n * (p->dtype == GPE_C64 ? 4 : 8);
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 ||
-      cudaMalloc(&p->d_ptab, bytes) != cudaSuccess) {
+// The point tables' memory, taken when the plan is made (a step then allocates nothing): whole
+// tables, which a multi-step call evaluates once per step, where they are at most a quarter
+// of what is free; else tables of as many rows as fit POINT_PIECE, halved while there is no
+// room for them, which the z sweeps take piece by piece at both times.  The values and the
+// sweeps are the same, so results do not depend on which it is.
+constexpr size_t POINT_PIECE = (size_t)128 << 20;   // bytes of the rows at one time
+bool point_memory(gpe_plan* p, bool pieces) {
+  const size_t row = (size_t)p->n * (p->dtype == GPE_C64 ? 4 : 8), all = (size_t)p->n * p->n;
+  size_t free_b = 0, total_b = 0, rows = all;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return false; }
+  const size_t least = std::min(all, (size_t)32);   // a z tile has at most 32 rows
+  if (pieces) rows = std::max(least, (all + 3) / 4);
+  else if (2 * all * row > free_b / 4) rows = std::max(least, std::min(all, POINT_PIECE / row));
+  while (cudaMalloc(&p->d_ptab, 2 * rows * row) != cudaSuccess) {
     cudaGetLastError();
     p->d_ptab = nullptr;
-    return false;
+    if (rows == least) return false;
+    rows = std::max(least, rows / 2);
   }
+  p->pt_rows = (int)rows;
   return true;
 }
 
@@ -1398,8 +1443,11 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
   }
   p->has_point = p->has_point && p->line && d->generic_only != 1 && !(d->local_fp64 && d->dtype == GPE_C64) &&
                  !d->exact_local;
-  if (p->has_point && point_memory(p)) { line_ok = true; p->fixed = false; }
-  else p->has_point = false;
+  if (p->has_point) {
+    if (!point_memory(p, d->generic_only == 5)) return fail(GPE_ERR_OOM, "no device memory for the potential's tables");
+    line_ok = true;
+    p->fixed = false;
+  }
   p->fast = (p->fixed || p->line) && d->generic_only != 1 && line_ok && !(d->local_fp64 && d->dtype == GPE_C64) &&
             !d->exact_local;
   if (!p->fast) { p->prog_line.clear(); p->slot_progs.clear(); }

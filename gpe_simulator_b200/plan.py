@@ -71,8 +71,9 @@ class Plan:
     beam; ``nk_bins``: 0 = the reference's shell binning, else uniform bins.
     Options that keep results identical: ``path`` (``"default"``, ``"tma"``,
     ``"plane"`` or ``"auto"``: the sweep path, see ``tune.py``; ``tma`` and
-    ``fuse_planes`` are the older switches for two of them) and
-    ``generic_only`` (mixed-radix sweeps only).  Options that change results on
+    ``fuse_planes`` are the older switches for two of them), ``point_pieces``
+    (tables of a dynamic potential with z terms for a quarter of the grid at a
+    time: less memory, more time) and ``generic_only`` (mixed-radix sweeps only).  Options that change results on
     purpose: ``local_fp64`` (complex64 local factor in FP64) and ``exact_local``
     (exact local sub-flows).
     """
@@ -80,7 +81,7 @@ class Plan:
     def __init__(self, n, x_array, k_array, *, dtype, kind, beta, dt, kinetic_coeff=1.0,
                  static_expr="0", dynamic_expr="0", k_cut=None, beam=None, nk_bins=0,
                  local_fp64=None, generic_only=False, fuse_planes=False, exact_local=False, tma=False,
-                 path=None):
+                 path=None, point_pieces=False):
         if not torch.cuda.is_available():
             raise RuntimeError("gpe_simulator_b200 needs a CUDA device (sm_100a)")
         self.lib = _lib.load()
@@ -132,7 +133,8 @@ class Plan:
             local_fp64 = False
         d.local_fp64 = 1 if local_fp64 else 0
         # sweep path: 0 fastest, 1 generic only, 3 y/z sweeps fused per x-plane (complex64 n = 128, 256),
-        # 4 fastest with the y/x pencils staged by TMA (complex64 n = 128, 256; identical results).
+        # 4 fastest with the y/x pencils staged by TMA (complex64 n = 128, 256; identical results),
+        # 5 fastest with point tables in pieces (identical results).
         # ``path`` names it instead: "default", "tma", "plane", or "auto" (timed once per device,
         # size, dtype and kind, then cached; see tune.py)
         if path is not None:
@@ -143,7 +145,7 @@ class Plan:
                 raise ValueError("path must be 'default', 'tma', 'plane' or 'auto'")
             tma, fuse_planes = path == "tma", path == "plane"
         self.path = "plane" if fuse_planes else ("tma" if tma else "default")
-        d.generic_only = 1 if generic_only else (3 if fuse_planes else (4 if tma else 0))
+        d.generic_only = 1 if generic_only else (3 if fuse_planes else 4 if tma else 5 if point_pieces else 0)
         # exact local sub-flows: an accuracy mode that departs from the reference on purpose
         d.exact_local = 1 if exact_local else 0
         self.local_fp64 = bool(local_fp64)

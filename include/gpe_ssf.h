@@ -127,7 +127,10 @@ typedef struct gpe_desc {
      * complex64 n = 128, 256 stage the pencils of their plain y/x sweeps by TMA
      * in persistent double-buffered launches (identical results; the y sweep
      * times the same alone, and the step is 4-5% slower because a persistent
-     * grid ends the overlap of neighbouring launches). */
+     * grid ends the overlap of neighbouring launches); 5 = as 0, and the tables of a
+     * dynamic potential with z terms hold a quarter of the grid at a time (identical
+     * results, a quarter of the tables' memory, each time evaluated twice; plans whose
+     * whole tables would pass a quarter of the free memory take pieces by themselves). */
     int generic_only;
     /* 1 = exact local sub-flows (an accuracy mode that departs from the reference
      * on purpose; evaluated in FP64 on the generic sweeps): imaginary time
