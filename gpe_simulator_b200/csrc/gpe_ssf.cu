@@ -1323,10 +1323,20 @@ int ensure_work(gpe_plan* p) {
   return GPE_OK;
 }
 
+// Histograms a plan has room for: one per tile of an x sweep (the only sweeps that write
+// them), whichever sweeps those are.
+int hist_tiles(const gpe_plan* p) {
+  int t = tiles_of(p, AX_X);
+  if (p->fast) {
+    if (p->ls[1].ok) t = std::max(t, p->ls[1].p.tiles);
+    if (p->fixed) t = std::max(t, p->n * (p->n / fast_lines(p->n, (int)p->csize / 2)));
+  }
+  return t;
+}
+
 int ensure_hist(gpe_plan* p) {
   if (p->d_hist) return GPE_OK;
-  // per-tile histograms of the generic or the register-resident x sweep
-  const size_t bytes = (size_t)p->max_tiles * p->nbins * sizeof(double);
+  const size_t bytes = (size_t)hist_tiles(p) * p->nbins * sizeof(double);
   CU(cudaMalloc(&p->d_hist, bytes));
   return GPE_OK;
 }
@@ -1469,7 +1479,7 @@ int fill_plan(gpe_plan* p, const gpe_desc* d) {
   p->counts.assign(p->nbins, 0);   // (filled by create)
   p->max_tiles = std::max(tiles_of(p, AX_Z), tiles_of(p, AX_X));
   for (const auto& s : p->ls)
-    if (s.ok) p->max_tiles = std::max(p->max_tiles, std::max(s.z.tiles, s.p.tiles));
+    if (s.ok && p->fast) p->max_tiles = std::max(p->max_tiles, std::max(s.z.tiles, s.p.tiles));
   return GPE_OK;
 }
 
@@ -1843,8 +1853,8 @@ int fft3d(gpe_plan* p, const void* in, void* out, bool inverse, cudaStream_t st)
 // k-space reductions of a spectrum `f` (no FFT): per-block sums of k^2 |f|^2
 // (+ shell histograms) into partial area B; `nb` = the blocks to finish.
 int kspace_reduce(gpe_plan* p, const void* f, bool hist, int& nb, cudaStream_t st) {
-  TRY(ensure_hist(p));
-  // at most max_tiles blocks (the partial and histogram areas), 4 per SM
+  if (hist) TRY(ensure_hist(p));
+  // at most as many blocks as the partial and histogram areas hold, 4 per SM
   static int sms = 0;
   if (!sms) {
     int dev = 0;
@@ -1854,7 +1864,7 @@ int kspace_reduce(gpe_plan* p, const void* f, bool hist, int& nb, cudaStream_t s
   const int copies = hist_copies(p->nbins, 24 * 1024);
   const size_t smem = hist ? (size_t)copies * p->nbins * sizeof(double) : 0;
   if (smem > 48 * 1024) return fail(GPE_ERR_UNSUPPORTED, "too many n(k) bins for the shared histogram");
-  nb = std::max(1, std::min(p->max_tiles, std::min(4 * sms, (p->n * p->n + 7) / 8)));
+  nb = std::max(1, std::min(hist_tiles(p), std::min(4 * sms, (p->n * p->n + 7) / 8)));
   double* part = p->d_partial + 4 * (size_t)p->max_tiles;
   double* h = hist ? p->d_hist : nullptr;
   if (p->dtype == GPE_C64)
@@ -2225,10 +2235,11 @@ int gpe_diagnostics(gpe_plan* p, const void* psi, double t, double* scalars, dou
   if (!p || !psi || !scalars) return fail(GPE_ERR_ARG, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   TRY(ensure_work(p));
-  TRY(ensure_hist(p));
+  const bool hist = nk != nullptr;
+  // (the Stockham x sweep always bins)
+  if (hist || !diag_fast(p, hist)) TRY(ensure_hist(p));
   TableUse tables(p, st, false);
   CU(tables.err);
-  const bool hist = nk != nullptr;
   TRY(diag_launch(p, psi, t, hist, st));
   int na = 0, nb = 0;
   diag_tiles(p, diag_fast(p, hist), na, nb);
@@ -2613,7 +2624,7 @@ int group_upload(gpe_batch* b, gpe_batch::Group& g) {
   for (int q = 0; q < m; ++q) {
     gpe_plan* p = b->plans[g.members[q]];
     TRY(ensure_work(p));
-    TRY(ensure_hist(p));
+    if (!diag_fast(p, false)) TRY(ensure_hist(p));
     hph[q] = p->ph;
     for (int role = 0; role < ROLE_COUNT; ++role) {
       Sweep s = role_sweep(role, b->psis[g.members[q]], p);
