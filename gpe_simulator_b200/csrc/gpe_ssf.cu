@@ -2539,7 +2539,10 @@ int group_launch(gpe_batch* b, gpe_batch::Group& g, int role, cudaStream_t st) {
       CU(launch_line_batch<R>(fax, g.d_ph, sws, count, op, ls.geo, shape, smem, st));
     }
   } else {
+    // (a Stockham sweep's shared memory ends with its instance's shells: room for the most)
     gpe_plan* p = b->plans[g.members[0]];
+    for (int i : g.members)
+      if (b->plans[i]->nbins > p->nbins) p = b->plans[i];
     Sweep geo = mk_sweep(nullptr, nullptr);
     int tiles = 0, threads = 0;
     size_t smem = 0;

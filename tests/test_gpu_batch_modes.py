@@ -1,4 +1,4 @@
-"""Batches whose instances differ in their accuracy mode: each keeps its own."""
+"""Batches whose instances of one size differ in accuracy mode or shell binning."""
 
 import pytest
 import torch
@@ -37,5 +37,34 @@ def test_modes_of_one_size(cuda, monkeypatch, n, modes, dtype):
                     static_expr=inst.static_expr, **({mode: True} if mode else {}))
         plan.step(p, 4)
         assert torch.equal(p, q)
+        want = plan.diagnostics(q)
+        assert [want[k] for k in ("N", "E_kin", "E_pot", "E_int", "E", "mu")] == list(d)
+
+
+@pytest.mark.parametrize("bins", [(0, 3000), (3000, 0)])
+def test_shell_binnings_of_one_size(cuda, monkeypatch, bins):
+    """The Stockham x sweep of a prime side bins into shared memory behind its tile: the launch
+    makes room for the instance with the most shells."""
+    from gpe_simulator_b200 import batch as mod
+    from gpe_simulator_b200.plan import Plan
+    fill = mod._fill_desc
+
+    def fill_bins(d, inst, *rest):
+        fill(d, inst, *rest)
+        d.nk_bins = inst.bins
+
+    monkeypatch.setattr(mod, "_fill_desc", fill_bins)
+    insts = [mod.Instance(n=13, simulation_range=10.0, beta=300.0, dt=2e-3, static_expr="x**2+y**2+2*z**2")
+             for _ in bins]
+    for inst, nb in zip(insts, bins):
+        inst.bins = nb
+    psis = mod.initial_states(insts, torch.complex64)
+    b = mod.Batch(insts, torch.complex64)
+    b.bind(psis)
+    b.step(2)
+    diag = b.diagnostics()
+    for inst, q, d in zip(insts, psis, diag):
+        plan = Plan(13, inst.x, inst.k, dtype=torch.complex64, kind="imaginary", beta=inst.beta, dt=inst.dt,
+                    static_expr=inst.static_expr, nk_bins=inst.bins)
         want = plan.diagnostics(q)
         assert [want[k] for k in ("N", "E_kin", "E_pot", "E_int", "E", "mu")] == list(d)
