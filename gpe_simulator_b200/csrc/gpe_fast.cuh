@@ -197,6 +197,10 @@ __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename C
   constexpr int L = FastCfg<N, R>::L;
   constexpr int T = FastCfg<N, R>::T;
   static_assert(QA * B <= V && QB * A <= V, "register array too small");
+  // (the arithmetic of the packed sweeps, gpe_packed.cuh)
+  constexpr bool NAMED = N == 256 && sizeof(R) == 4;
+  using DftA = typename std::conditional<NAMED, DftSplit<4, 4, true>, Dft<A>>::type;
+  using DftB = typename std::conditional<NAMED, DftSplit<4, 4, true>, Dft<B>>::type;
   // Z tiles with A == B lanes per line in both phases and one slot per thread:
   // every line is owned by the same warp in both phases (32/A lines per warp)
   // and its exchange rows are its own, so a warp barrier suffices.
@@ -208,9 +212,12 @@ __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename C
     int l, lane;
     slot<AX, L, T>(gs, A, l, lane);
     C* x = v + s * B;
-    Dft<B>::run(x, (const C*)nullptr, (const C*)nullptr, N / B);
+    DftB::run(x, (const C*)nullptr, (const C*)nullptr, N / B);
 #pragma unroll
-    for (int k2 = 1; k2 < B; ++k2) x[k2] = tw_apply(x[k2], tw[k2 * A + lane]);
+    for (int k2 = 1; k2 < B; ++k2) {
+      if constexpr (NAMED) x[k2] = tw_named(x[k2], tw[k2 * A + lane]);
+      else x[k2] = tw_apply(x[k2], tw[k2 * A + lane]);
+    }
     // exchange layout: Z tiles [l][k2][A + 1] (odd pitch), P tiles [k2][lane][L]
 #pragma unroll
     for (int k2 = 0; k2 < B; ++k2) {
@@ -232,7 +239,7 @@ __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename C
       const int idx = AX == FZ ? (l * B + k2) * (A + 1) + n1 : (k2 * A + n1) * L + l;
       x[n1] = ex[idx];
     }
-    Dft<A>::run(x, (const C*)nullptr, (const C*)nullptr, N / A);
+    DftA::run(x, (const C*)nullptr, (const C*)nullptr, N / A);
   }
   if (ASYNC_NEXT) fence_proxy_async_smem();
   if (TAIL) {
@@ -693,6 +700,27 @@ __device__ __forceinline__ void local_block(typename Cx<R>::T* v, const R (&V)[U
 // elements per local_block: the largest of 5, 4, 3, 2 that divides n (1: none does)
 constexpr int local_unroll(int n) { return n % 4 == 0 ? 4 : n % 5 == 0 ? 5 : n % 3 == 0 ? 3 : n % 2 == 0 ? 2 : 1; }
 
+// Phase of an element's half-step (TWO: of both), and exp(-i phase) - 1 times 1 + am; NAMED as in
+// gpe_fft.cuh.
+template <bool NAMED, bool ARR, bool TWO, typename C, typename R>
+__device__ __forceinline__ R local_phase(C x, R V, R g, R beta, R h) {
+  R rho;
+  if constexpr (NAMED) rho = fma(x.x, x.x, x.y * x.y);
+  else rho = x.x * x.x + x.y * x.y;
+  if constexpr (TWO) return fma(beta * two_density<ARR>(g), rho, V);
+  else if constexpr (NAMED) return fma(beta, rho, V) * h;
+  else return (V + beta * rho) * h;
+}
+template <bool NAMED> __device__ __forceinline__ void times_amplitude(float am, float& cm1, float& sn) {
+  if constexpr (NAMED) {
+    cm1 = fmaf(am, cm1, am + cm1);
+    sn = fmaf(sn, am, sn);
+  } else {
+    cm1 = am + cm1 + am * cm1;
+    sn = sn + sn * am;
+  }
+}
+
 // One local half-step over all registers (layout LANES x VALS, element m = lane +
 // LANES*a, Z tiles: m = z index), potential vz[m] + ctab[l] (+ arrays).  complex64:
 // each element whose phase is within the short series' range (|phase| <= 1/8,
@@ -742,6 +770,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
     }
     return;
   }
+  constexpr bool NAMED = N == 256;
   static_assert(SLOTS * VALS <= 64, "pending mask");
   // complex64: elements whose phase exceeds the short series' range
   using Mask = typename std::conditional<(SLOTS * VALS <= 32), unsigned, unsigned long long>::type;
@@ -764,8 +793,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
         g = ph.vim ? ((const R*)ph.vim)[row + m] * h : (R)0;
       }
       const typename Cx<R>::T x = v[e];
-      const R phs = TWO ? fma(beta * two_density<ARR>(g), x.x * x.x + x.y * x.y, V)
-                        : (V + beta * (x.x * x.x + x.y * x.y)) * h;
+      const R phs = local_phase<NAMED, ARR, TWO>(x, V, g, beta, h);
       if (fabs(phs) <= (R)0.125) {
         if (!REAL) {
           const float em = expm1_tiny((float)-phs);
@@ -773,7 +801,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
         } else {
           float sn, cm1;
           sin_cosm1_tiny((float)phs, sn, cm1);
-          if (ARR) { const float am = expm1f((float)(TWO ? g + g : g)); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
+          if (ARR) { const float am = expm1f((float)(TWO ? g + g : g)); times_amplitude<NAMED>(am, cm1, sn); }
           v[e] = mk(fma(x.x, (R)cm1, fma(x.y, (R)sn, x.x)), fma(x.y, (R)cm1, fma(-x.x, (R)sn, x.y)));
         }
       } else {
@@ -803,8 +831,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
         g = ph.vim ? ((const R*)ph.vim)[row + m] * h : (R)0;
       }
       const typename Cx<R>::T x = v[e];
-      const float p = (float)(TWO ? fma(beta * two_density<ARR>(g), x.x * x.x + x.y * x.y, V)
-                                  : (V + beta * (x.x * x.x + x.y * x.y)) * h);
+      const float p = (float)local_phase<NAMED, ARR, TWO>(x, V, g, beta, h);
       if (!REAL) {
         const float em = fabsf(p) <= 0.5f ? expm1_series(-p) : expm1f(-p);
         v[e] = mk(fma(x.x, (R)em, x.x), fma(x.y, (R)em, x.y));
@@ -817,7 +844,7 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
           sincosf(0.5f * p, &sh, &ch);
           cm1 = -2.0f * sh * sh; sn = 2.0f * sh * ch;
         }
-        if (ARR) { const float am = expm1f((float)(TWO ? g + g : g)); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
+        if (ARR) { const float am = expm1f((float)(TWO ? g + g : g)); times_amplitude<NAMED>(am, cm1, sn); }
         v[e] = mk(fma(x.x, (R)cm1, fma(x.y, (R)sn, x.x)), fma(x.y, (R)cm1, fma(-x.x, (R)sn, x.y)));
       }
     }

@@ -100,8 +100,21 @@ __device__ __forceinline__ float2 tw_apply(float2 v, float4 w) {
 }
 __device__ __forceinline__ double2 tw_apply(double2 v, double2 w) { return cmul(v, w); }
 
+// The complex64 products above with every fused operation named.  Which of two products of a
+// sum the compiler fuses differs between kernels, for the low parts once in some 1e10
+// operations visibly; kernels that promise each other the same bits although one packs
+// two lines and one does not (n = 256) use these.
+__device__ __forceinline__ float2 rot_named(float2 v, float ch, float cl, float sh, float sl) {
+  return make_float2(fmaf(v.x, ch, fmaf(v.y, sh, fmaf(v.x, cl, __fmul_rn(v.y, sl)))),
+                     fmaf(v.y, ch, fmaf(-v.x, sh, fmaf(v.y, cl, __fmul_rn(-v.x, sl)))));
+}
+__device__ __forceinline__ float2 tw_named(float2 v, float4 w) {
+  return make_float2(fmaf(v.x, w.x, fmaf(-v.y, w.y, fmaf(v.x, w.z, __fmul_rn(-v.y, w.w)))),
+                     fmaf(v.x, w.y, fmaf(v.y, w.x, fmaf(v.x, w.w, __fmul_rn(v.y, w.z)))));
+}
+
 // v * W_16^q, W_16 = exp(-2 pi i / 16), q known at compile time after unrolling
-template <typename C> __device__ __forceinline__ C mul_w16(C v, int q) {
+template <bool NAMED = false, typename C> __device__ __forceinline__ C mul_w16(C v, int q) {
   using R = decltype(v.x);
   using k = K<R>;
   q &= 15;
@@ -116,6 +129,10 @@ template <typename C> __device__ __forceinline__ C mul_w16(C v, int q) {
     return mk(kmul(a * v.x - b * v.y, k::R2, k::R2L), kmul(a * v.y + b * v.x, k::R2, k::R2L));
   }
   // odd multiples of pi/8: v * (cos - i sin) of pi q / 8
+  auto rot = [](C u, R ch, R cl, R sh, R sl) {
+    if constexpr (NAMED) return rot_named(u, ch, cl, sh, sl);
+    else return gpe::rot(u, ch, cl, sh, sl);
+  };
   switch (q) {
     case 1:  return rot(v, k::C8, k::C8L, k::S8, k::S8L);
     case 3:  return rot(v, k::S8, k::S8L, k::C8, k::C8L);
@@ -180,7 +197,7 @@ template <> struct Dft<5> {
 };
 
 // R = R1*R2 from two smaller DFTs: n = R2*n1 + n2, k = k1 + R1*k2.
-template <int R1, int R2> struct DftSplit {
+template <int R1, int R2, bool NAMED = false> struct DftSplit {
   template <typename C> __device__ __forceinline__ static void run(C* v, const C* tw, const C* twl, int unused) {
     using Rl = decltype(v[0].x);
     constexpr int RR = R1 * R2;
@@ -194,7 +211,7 @@ template <int R1, int R2> struct DftSplit {
       for (int k1 = 1; k1 < R1; ++k1) {
         if (n2 == 0) continue;
         // W_RR^(n2 k1) = W_16^(q), RR in {8, 16}
-        y[n2][k1] = mul_w16(y[n2][k1], (16 / RR) * ((n2 * k1) % RR));
+        y[n2][k1] = mul_w16<NAMED>(y[n2][k1], (16 / RR) * ((n2 * k1) % RR));
       }
     }
 #pragma unroll
@@ -211,8 +228,7 @@ template <int R1, int R2> struct DftSplit {
 
 // ---- compile-time roots for composite radices other than 8 and 16
 // cos and sin of 2 pi e / rr evaluated at compile time: exact quadrant and
-// half-quadrant reduction in integers, then Taylor series to x^23 on |t| <= pi/4.
-// Compile-time cosines and sines.  The Taylor sums are carried in pairs of doubles (sums and
+// half-quadrant reduction in integers, then Taylor series on |t| <= pi/4.  They are carried in pairs of doubles (sums and
 // products by their exact errors: T. J. Dekker, "A floating-point technique for extending the
 // available precision", 1971) and rounded once: summed in plain doubles they were up to 1.4
 // ulp off, the same error in every butterfly of a radix, and complex128 steps at 105^3 had

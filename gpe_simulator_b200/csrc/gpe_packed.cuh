@@ -175,8 +175,7 @@ __device__ __forceinline__ void pack_3phase(C2 (&v)[V], ulonglong2* ex, const fl
 // elements outside the packed short series, and array potentials.
 template <bool REAL, bool ARR, bool TWO>
 __device__ __forceinline__ float2 half_one(float2 x, float V, float g, float beta, float h) {
-  const float p = TWO ? fmaf(beta * two_density<ARR>(g), x.x * x.x + x.y * x.y, V)
-                      : (V + beta * (x.x * x.x + x.y * x.y)) * h;
+  const float p = local_phase<true, ARR, TWO>(x, V, g, beta, h);
   if (!REAL) {
     const float em = fabsf(p) <= 0.125f ? expm1_tiny(-p) : fabsf(p) <= 0.5f ? expm1_series(-p) : expm1f(-p);
     return make_float2(fmaf(x.x, em, x.x), fmaf(x.y, em, x.y));
@@ -192,7 +191,7 @@ __device__ __forceinline__ float2 half_one(float2 x, float V, float g, float bet
     cm1 = -2.0f * sh * sh;
     sn = 2.0f * sh * ch;
   }
-  if (ARR) { const float am = expm1f(TWO ? g + g : g); cm1 = am + cm1 + am * cm1; sn = sn + sn * am; }
+  if (ARR) times_amplitude<true>(expm1f(TWO ? g + g : g), cm1, sn);
   return make_float2(fmaf(x.x, cm1, fmaf(x.y, sn, x.x)), fmaf(x.y, cm1, fmaf(-x.x, sn, x.y)));
 }
 
