@@ -114,7 +114,7 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// per-tile table bytes (kx, kyz, kxy2, kz2, vz, c1, c2, c12), rounded to 16
+// per-tile table bytes (kx, kyz, kx2, kyz2, vz, c1, c2, c12), rounded to 16
 template <int N, typename R> __host__ __device__ constexpr size_t fast_tables_bytes() {
   return (((size_t)(N + FastCfg<N, R>::L) * (16 + 8) + (size_t)(N + 3 * FastCfg<N, R>::L) * sizeof(R)) + 15)
          / 16 * 16;
@@ -467,8 +467,8 @@ struct FastTables {
   R* c12;         // [L] c1 + c2
   double2* kx;    // [N] kinetic factors along the transform axis (X tiles)
   double2* kyz;   // [L] kinetic factor of (j, k_l)
-  double* kxy2;    // [N] kx^2 + ky^2 of the tile's row (cutoff; the sums of kk_ref)
-  double* kz2;   // [L] kz^2 of the line
+  double* kx2;    // [N] k^2 along x (cutoff)
+  double* kyz2;   // [L] k_j^2 + k_kl^2
 };
 
 // two: the tables of the fused z sweep (c2, c12 at the second half-step's time).
@@ -531,7 +531,7 @@ __device__ __forceinline__ void x_tables(const Phys& ph, int j, int k0, FastTabl
   constexpr int L = FastCfg<N, R>::L;
   for (int q = threadIdx.x; q < N; q += T) {
     tb.kx[q] = ph.kin[q];
-    tb.kxy2[q] = __dadd_rn(__dmul_rn(ph.k[q], ph.k[q]), __dmul_rn(ph.k[j], ph.k[j]));
+    tb.kx2[q] = ph.k[q] * ph.k[q];
   }
   if (threadIdx.x < L) {
     const int k = k0 + threadIdx.x;
@@ -540,7 +540,7 @@ __device__ __forceinline__ void x_tables(const Phys& ph, int j, int k0, FastTabl
     // line instead of one per element in the z sweep that follows)
     const double2 f = ph.kind == 0 ? make_double2(a.x * b.x, 0.0) : cmul(a, b);
     tb.kyz[threadIdx.x] = make_double2(f.x * ph.inv_m, f.y * ph.inv_m);
-    tb.kz2[threadIdx.x] = __dmul_rn(ph.k[k], ph.k[k]);
+    tb.kyz2[threadIdx.x] = ph.k[j] * ph.k[j] + ph.k[k] * ph.k[k];
   }
 }
 
@@ -560,7 +560,7 @@ __device__ __forceinline__ typename Cx<R>::T fast_kin(const Phys& ph, const Fast
     out = mk((R)(vx * fx - vy * fy), (R)(vx * fy + vy * fx));
   }
   if (CUT) {
-    const bool drop = __dadd_rn(tb.kxy2[i], tb.kz2[l]) > ph.kcut2;
+    const bool drop = tb.kx2[i] + tb.kyz2[l] > ph.kcut2;
     out = drop ? mk((R)0, (R)0) : out;
   }
   return out;
@@ -1075,9 +1075,9 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
   FastTables<R> tb;
   tb.kx = (double2*)tail;
   tb.kyz = tb.kx + N;
-  tb.kxy2 = (double*)(tb.kyz + L);
-  tb.kz2 = tb.kxy2 + N;
-  tb.vz = (R*)(tb.kz2 + L);
+  tb.kx2 = (double*)(tb.kyz + L);
+  tb.kyz2 = tb.kx2 + N;
+  tb.vz = (R*)(tb.kyz2 + L);
   tb.c1 = tb.vz + N;
   tb.c2 = tb.c1 + L;
   tb.c12 = tb.c2 + L;

@@ -342,21 +342,14 @@ __device__ __forceinline__ typename Cx<R>::T halfstep(const Phys& ph, typename C
   return mk(v.x * c + v.y * s, v.y * c - v.x * s);
 }
 
-// kx^2 + ky^2 + kz^2 rounded as NumPy evaluates it (each product and sum rounded, left to
-// right, no fused multiply-add), so that modes on a shell's boundary fall in the same shell
-// as in the reference's nk_extraction, and modes on the cutoff sphere are kept or dropped as
-// by the reference's k^2 > k_cut^2, on every sweep path and along every axis.
-__device__ __forceinline__ double kk_ref(double kx, double ky, double kz) {
-  return __dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kz, kz));
-}
-
 // Kinetic factor at wavenumber indices (i,j,k) applied in FP64
 // (reference gpe/kernels.py:3-66).
 template <typename R>
 __device__ __forceinline__ typename Cx<R>::T kinetic(const Phys& ph, typename Cx<R>::T v, int n, int i,
                                                      int j, int k) {
   if (ph.kcut) {
-    if (kk_ref(ph.k[i], ph.k[j], ph.k[k]) > ph.kcut2) return mk((R)0, (R)0);
+    const double kk = ph.k[i] * ph.k[i] + ph.k[j] * ph.k[j] + ph.k[k] * ph.k[k];
+    if (kk > ph.kcut2) return mk((R)0, (R)0);
   }
   if (sizeof(R) == 4 && ph.kind == 0) {
     // complex64 imaginary time: exponent summed in FP64, factor applied as v + v*(f - 1)
@@ -376,6 +369,13 @@ __device__ __forceinline__ typename Cx<R>::T kinetic(const Phys& ph, typename Cx
   f = cmul(cmul(a, b), c);
   const double vx = v.x, vy = v.y;
   return mk((R)(vx * f.x - vy * f.y), (R)(vx * f.y + vy * f.x));
+}
+
+// |k|^2 = kx^2 + ky^2 + kz^2 rounded as NumPy evaluates it (each product and sum
+// rounded, left to right, no fused multiply-add), so shell indices at exact
+// boundaries agree with the reference's nk_extraction.
+__device__ __forceinline__ double kk_ref(double kx, double ky, double kz) {
+  return __dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kz, kz));
 }
 
 // Shell of k^2, min(floor(sqrt(kk)/w + 0.5), nbins - 1) in FP64 as NumPy evaluates it, without

@@ -93,7 +93,7 @@ struct LineCx {
   const R* c1;            // [L] line part of the potential at t1 (shared)
   const R* c12;           // [L] (line parts at t1 and t2) dt/2 (shared; fused half-steps)
   const double2* kyz;     // [L] kinetic factor of the line, with 1/M (shared)
-  const double* kz2;      // [L] k_z^2 of the line (shared)
+  const double* kyz2;     // [L] k_y^2 + k_z^2 of the line (shared)
   const R* vd1;           // dynamic potential with z terms at t1 (t2), per point (global, null: none)
   const R* vd2;
   long long row0;         // z tiles: global index of line 0
@@ -156,7 +156,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   R* c1 = (R*)tail;
   R* c12 = c1 + L;
   double2* kyz = (double2*)tail;
-  double* kz2 = (double*)(kyz + L);
+  double* kyz2 = (double*)(kyz + L);
   Acc* red = (Acc*)(tail + ((size_t)L * 24 + 15) / 16 * 16);
   double* hist = (double*)(red + 32 * 4);
   lc.vz = (const R*)ph.vax + 2 * n;
@@ -165,7 +165,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
   lc.vd1 = (const R*)sw.vd1;
   lc.vd2 = (const R*)sw.vd2;
   lc.kyz = kyz;
-  lc.kz2 = kz2;
+  lc.kyz2 = kyz2;
   lc.n = n;
 
   // the tile's lines
@@ -228,7 +228,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       const double2 a = ph.kin[a0], b = ph.kin[z0 + l];
       const double2 f = ph.kind == 0 ? make_double2(a.x * b.x, 0.0) : cmul(a, b);
       kyz[l] = make_double2(f.x * ph.inv_m, f.y * ph.inv_m);
-      kz2[l] = __dmul_rn(ph.k[z0 + l], ph.k[z0 + l]);
+      kyz2[l] = ph.k[a0] * ph.k[a0] + ph.k[z0 + l] * ph.k[z0 + l];
     }
   }
   const int copies = MODE == FM_DIAGK && sw.hist ? hist_copies(sw.nbins, LINE_HIST) : 0;
@@ -371,10 +371,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
             } else {
               const double wx = fx.x * fl.x - fx.y * fl.y, wy = fx.x * fl.y + fx.y * fl.x;
               v[a] = mk((R)(vx * wx - vy * wy), -(R)(vx * wy + vy * wx));
-              if (ph.kcut) {   // (kk_ref's sum)
-                const double kxy2 = __dadd_rn(__dmul_rn(ph.k[i], ph.k[i]), __dmul_rn(ph.k[a0], ph.k[a0]));
-                if (__dadd_rn(kxy2, kz2[l]) > ph.kcut2) v[a] = mk((R)0, (R)0);
-              }
+              if (ph.kcut && ph.k[i] * ph.k[i] + kyz2[l] > ph.kcut2) v[a] = mk((R)0, (R)0);
             }
           }
         }

@@ -28,7 +28,7 @@ template <int N> struct PackCfg {
   // twiddles of the split (N1 lanes, N2 values), then of (N2, N1) when that differs (n = 512:
   // the 64 second-phase ones)
   static constexpr int TW = N + (THREE ? 64 : N1 == N2 ? 0 : N);
-  // tables of a z sweep: reduction scratch, vz, c1, c2, c12; of an x sweep: kx, kyz, kxy2, kz2
+  // tables of a z sweep: reduction scratch, vz, c1, c2, c12; of an x sweep: kx, kyz, kx2, kyz2
   static constexpr size_t ZB = 32 * 16 + (size_t)(N + 3 * L) * 4, XB = (size_t)(N + L) * 24;
 };
 template <int N, int MODE> constexpr size_t pack_smem() {
@@ -382,8 +382,8 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
   FastTables<float> tb;
   tb.kx = (double2*)tail;
   tb.kyz = tb.kx + N;
-  tb.kxy2 = (double*)(tb.kyz + L);
-  tb.kz2 = tb.kxy2 + N;
+  tb.kx2 = (double*)(tb.kyz + L);
+  tb.kyz2 = tb.kx2 + N;
   tb.vz = (float*)(red + 32);
   tb.c1 = tb.vz + N;
   tb.c2 = tb.c1 + L;
