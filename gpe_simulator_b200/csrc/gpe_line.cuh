@@ -228,7 +228,7 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
       const double2 a = ph.kin[a0], b = ph.kin[z0 + l];
       const double2 f = ph.kind == 0 ? make_double2(a.x * b.x, 0.0) : cmul(a, b);
       kyz[l] = make_double2(f.x * ph.inv_m, f.y * ph.inv_m);
-      kyz2[l] = ph.k[a0] * ph.k[a0] + ph.k[z0 + l] * ph.k[z0 + l];
+      kyz2[l] = fma(ph.k[a0], ph.k[a0], __dmul_rn(ph.k[z0 + l], ph.k[z0 + l]));
     }
   }
   const int copies = MODE == FM_DIAGK && sw.hist ? hist_copies(sw.nbins, LINE_HIST) : 0;
@@ -371,7 +371,9 @@ __device__ __forceinline__ void line_body(const Phys& ph, const Sweep& sw, const
             } else {
               const double wx = fx.x * fl.x - fx.y * fl.y, wy = fx.x * fl.y + fx.y * fl.x;
               v[a] = mk((R)(vx * wx - vy * wy), -(R)(vx * wy + vy * wx));
-              if (ph.kcut && ph.k[i] * ph.k[i] + kyz2[l] > ph.kcut2) v[a] = mk((R)0, (R)0);
+              // (fused operations named: the rounding of this sum decides which modes of exactly
+              // the cutoff's length stay, and must not depend on the compiler)
+              if (ph.kcut && fma(ph.k[i], ph.k[i], kyz2[l]) > ph.kcut2) v[a] = mk((R)0, (R)0);
             }
           }
         }
