@@ -94,7 +94,6 @@ struct FastOps {
   int pdl;          // host: launch as a programmatic dependent of the previous sweep
   int vec;          // host: src and dst aligned to 16 bytes (packed sweeps)
   int rev;          // tiles in descending order (see tile_of)
-  int tile0;        // first tile of the launch (run-time-length sweeps)
   int pf;           // tiles ahead whose lines a block prefetches into L2 (0 = none): the
                     // tile the block that follows it on the SM will process
 };

@@ -496,7 +496,7 @@ template <typename R, int MODE, int RMAX> struct LineBounds {
 template <typename R, bool ZT, int MODE, int RMAX>
 __global__ void __launch_bounds__(LINE_T, LineBounds<R, MODE, RMAX>::blocks) k_line(Phys ph, Sweep sw, FastOps op, LineGeo g,
                                                                       LineShape sh, int ax) {
-  line_body<R, ZT, MODE, RMAX>(ph, sw, op, g, sh, ax, op.tile0 + tile_of(op), gridDim.x);
+  line_body<R, ZT, MODE, RMAX>(ph, sw, op, g, sh, ax, sh.tile0 + tile_of(op), gridDim.x);
 }
 
 // Batched launch: blockIdx.y selects the instance (structs staged in shared memory).

@@ -35,7 +35,8 @@ struct LineShape {
   int pitch;                      // z tiles: shared elements from one line to the next
   int tpr;                        // y/x tiles per row
   int T;                          // threads
-  int tiles;
+  int tiles;                      // of the launch
+  int tile0;                      // its first one
 };
 
 inline unsigned line_magic(int d) { return d == 1 ? 0u : (unsigned)((0x100000000ull + d - 1) / d); }

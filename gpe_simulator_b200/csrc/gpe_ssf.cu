@@ -1108,14 +1108,13 @@ int fsweep_launch(gpe_plan* p, int ax, const Sweep& sw, const FastOps& op, int t
   const int fax = ax == AX_Z ? FZ : ax == AX_Y ? FY : FX;
   FastOps o = op;
   o.vec = ((uintptr_t)sw.src | (uintptr_t)sw.dst) % 16 == 0;
-  o.tile0 = tile0;
   o.pdl = p->pdl_chain && p->pdl_prev && !p->prof ? 1 : 0;
   p->pdl_prev = p->pdl_chain;
   const CUtensorMap* map = p->tma && o.tr != 2 && o.mode == FM_PLAIN && fax != FZ ? tma_maps(p, sw.src, fax) : nullptr;
   const bool line = !p->fixed || o.tr == 2;
   const gpe_plan::LineSet& ls = p->ls[o.tr ? 1 : 0];
   LineShape shape = fax == FZ ? ls.z : ls.p;
-  if (ntiles) shape.tiles = ntiles;
+  if (ntiles) { shape.tile0 = tile0; shape.tiles = ntiles; }
   const size_t smem = line ? line_smem(ls.geo, shape, (int)p->csize, fax == FZ,
                                       sw.hist ? hist_copies(sw.nbins, LINE_HIST) * sw.nbins : 0)
                           : 0;
@@ -1225,7 +1224,7 @@ int psweep(gpe_plan* p, void* psi, int mz, const FastOps* ops, int nstage, int z
 
 FastOps mk_ops(int mode, int inv1 = 0, int invm = 0, int scale = 0, int norm = 0) {
   FastOps o;
-  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.tile0 = 0; o.pdl = 0; o.vec = 0; o.rev = 0; o.pf = 0;
+  o.mode = mode; o.inv1 = inv1; o.invm = invm; o.scale = scale; o.norm = norm; o.tr = 0; o.pdl = 0; o.vec = 0; o.rev = 0; o.pf = 0;
   return o;
 }
 
