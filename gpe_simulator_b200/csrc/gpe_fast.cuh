@@ -249,8 +249,7 @@ __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename C
 // One forward FFT of every line of the tile for N = 8^3 (n = 512), in three
 // radix-8 phases over 64 lanes per line.  In and out the registers are in
 // layout (64 lanes, 8 values): slot s of lane p holds v[s][b] = x[p + 64 b] on
-// entry and X[p + 64 k] on return, so the two transforms of a fused sweep need
-// no change of layout between them.  Index split: n = p + 64 b with p = p1 + 8 p2,
+// entry and X[p + 64 k] on return.  Index split: n = p + 64 b with p = p1 + 8 p2,
 // k = k3 + 8 k1 + 64 k2.
 //   phase 1 (lane p):         DFT8 over b -> k3, times W_512^(p k3)     (twa[k3*64 + p])
 //   phase 2 (role p1 + 8 k3): DFT8 over p2 -> k1, times W_64^(p1 k1)    (twb[k1*8 + p1])
@@ -260,7 +259,7 @@ __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename C
 // accesses of a half warp avoid bank conflicts in both directions; P tiles
 // line-fastest, [k][role][l].  A thread's two slots are 32 lanes apart, so its
 // p1 is the same in both: each W_64 twiddle is loaded once for the two.
-template <int N, int AX, typename R, int Q, int V, bool TAIL = true>
+template <int N, int AX, typename R, int Q, int V>
 __device__ __forceinline__ void fft_3phase(typename Cx<R>::T (&v)[V], typename Cx<R>::T* ex,
                                            const typename TwE<R>::T* twa, const typename TwE<R>::T* twb) {
   using C = typename Cx<R>::T;
@@ -329,7 +328,6 @@ __device__ __forceinline__ void fft_3phase(typename Cx<R>::T (&v)[V], typename C
     for (int p1 = 0; p1 < RD; ++p1) x[p1] = ex[e2(l, k3, k1, p1)];
     Dft<RD>::run(x, (const C*)nullptr, (const C*)nullptr, N / RD);
   }
-  if (TAIL) sync();   // frees the exchange buffer for a next transform
 }
 
 template <typename R>
@@ -462,25 +460,24 @@ template <typename R>
 struct FastTables {
   R* vz;          // [N] static potential along z (Z tiles)
   R* c1;          // [L] vx(i) + vy(j_l) + beam(i, j_l; t1)
-  R* c2;          // [L] same at t2
-  R* c12;         // [L] c1 + c2
+  R* c2;          // [L] diagnostics: the beam's exponential
+  R* c12;         // [L] fused z sweep: (c1 + the same at t2) dt/2
   double2* kx;    // [N] kinetic factors along the transform axis (X tiles)
   double2* kyz;   // [L] kinetic factor of (j, k_l)
   double* kx2;    // [N] k^2 along x (cutoff)
   double* kyz2;   // [L] k_j^2 + k_kl^2
 };
 
-// two: the tables of the fused z sweep (c2, c12 at the second half-step's time).
-// pre (real time, two half-steps as one rotation): vz and
+// two: the tables of the fused z sweep (real time, two half-steps as one rotation): vz and
 // c12 are stored already multiplied by dt (vz by dt, c12 by dt/2), so that the
 // phase (2 vz + c12 + 2 beta |psi|^2) dt/2 is one add and one fma per point.
 template <int N, typename R, int T = FastCfg<N, R>::T>
 __device__ __forceinline__ void z_tables(const Phys& ph, const Sweep& sw, int a0, FastTables<R>& tb,
-                                         bool two, bool pre = false) {
+                                         bool two) {
   constexpr int L = FastCfg<N, R>::L;
   const R* vax = (const R*)ph.vax;
   const R h = (R)(ph.dt * 0.5), dt2 = h + h;
-  for (int q = threadIdx.x; q < N; q += T) tb.vz[q] = pre ? vax[2 * N + q] * dt2 : vax[2 * N + q];
+  for (int q = threadIdx.x; q < N; q += T) tb.vz[q] = two ? vax[2 * N + q] * dt2 : vax[2 * N + q];
   if (threadIdx.x < L) {
     const int g = a0 + threadIdx.x, i = g / N, j = g % N;
     const R base = vax[i] + vax[N + j];
@@ -501,8 +498,7 @@ __device__ __forceinline__ void z_tables(const Phys& ph, const Sweep& sw, int a0
       if (two) b2 += lt[(long long)N * N + g];
     }
     tb.c1[threadIdx.x] = base + b1;
-    tb.c2[threadIdx.x] = base + b2;
-    tb.c12[threadIdx.x] = pre ? ((base + b1) + (base + b2)) * h : (base + b1) + (base + b2);
+    if (two) tb.c12[threadIdx.x] = ((base + b1) + (base + b2)) * h;
   }
 }
 
@@ -1105,7 +1101,7 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
       }
     }
     if (ZM || (MODE == FM_DIAGR && ph.ltab))
-      z_tables<N, R>(ph, sw, tl.a0, tb, MODE == FM_Z21, MODE == FM_Z21);
+      z_tables<N, R>(ph, sw, tl.a0, tb, MODE == FM_Z21);
     if (MODE == FM_XKIN) x_tables<N, R>(ph, tl.a0, tl.b0, tb);
     if (MODE == FM_DIAGR && !ph.ltab) diag_tables<N, R>(ph, sw, tl.a0, tb);
   };
@@ -1121,11 +1117,6 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
     cx.sc_div = __ldcg(sw.scale);
     cx.sc_rcp = __ldcg(sw.scale + 1);
     cx.sc_mul = (R)cx.sc_rcp;
-  }
-  if (MODE == FM_DIAGR) {
-    cx.t1 = sw.t1;
-    cx.b1x = sw.bc1x;
-    cx.b1y = sw.bc1y;
   }
   if (MODE == FM_DIAGK) {
     // the shell histograms take the exchange buffer once the transform is done with it
@@ -1151,14 +1142,14 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
   if (MODE == FM_DIAGR) diag_real_all<N, AX, R, N1, N2, S1>(v, tl, ph, tb, cx);
   // the first transform frees the exchange buffer only when a second one follows
   constexpr bool TWO_FFT = MODE == FM_Z21 || MODE == FM_XKIN;
-  if constexpr (THREE) fft_3phase<N, AX, R, S1, EPT, TWO_FFT>(v, ex, t1, t2);
+  static_assert(!(THREE && TWO_FFT), "the fused 512-point sweeps are packed");
+  if constexpr (THREE) fft_3phase<N, AX, R, S1, EPT>(v, ex, t1, t2);
   else fft_2phase<N, N1, N2, AX, R, S1, S2, EPT, false, TWO_FFT>(v, ex, t1);
-  if (MODE == FM_Z21 || MODE == FM_XKIN) {
+  if constexpr (TWO_FFT) {
     if (MODE == FM_Z21) conj_all(v);  // finish the inverse before the physics
     fast_pointwise<N, AX, R, MODE, 1, LM, VM, SM>(v, tl, ph, tb, op, cx);
     if (MODE == FM_XKIN) conj_all(v);  // start the inverse
-    if constexpr (THREE) fft_3phase<N, AX, R, S1, EPT, false>(v, ex, t1, t2);
-    else fft_2phase<N, N2, N1, AX, R, S2, S1, EPT, false, false>(v, ex, t2);
+    fft_2phase<N, N2, N1, AX, R, S2, S1, EPT, false, false>(v, ex, t2);
     if (MODE == FM_XKIN) conj_all(v);
     fast_store<N, AX, R, N1, N2, S1>(v, tl, (C*)sw.dst);
   } else {
@@ -1205,10 +1196,10 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
 // At n = 128 the fused modes run 7 blocks of 72 registers: a 128^3 sweep is 1024 tiles, one
 // wave of 7 x 148 = 1036 blocks but 1.15 waves of 6 (imaginary time 51.0 -> 45.8 us per
 // step, stirred 35.1 -> 31.9; 8 blocks of 64 registers 46.0, 32.4).
-// At n = 512 (three radix-8 phases, 16 values per thread, 512-thread blocks of
-// about 98 KB of shared memory) two blocks per SM, 64 registers: 378 -> 415
-// steps/s at 512^3 against the earlier 32 x 16 split (32 values per thread, one
-// block of 128 registers per SM).
+// At n = 512 (transforms and diagnostics only, the steps' sweeps are packed; three radix-8
+// phases, 16 values per thread, 512-thread blocks of about 98 KB of shared memory) two
+// blocks per SM, 64 registers: a plain sweep 427 us, 640 us with a 32 x 16 split (32 values
+// per thread, one block of 128 registers per SM).
 // The diagnostic z sweep (FP64 potential per point) keeps 512 threads per SM.
 template <int N, typename R, int MODE> struct FastBounds {
   static constexpr int value = (sizeof(R) == 4 && (N == 128 || N == 256))

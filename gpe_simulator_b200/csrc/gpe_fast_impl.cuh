@@ -11,8 +11,14 @@ namespace gpe {
 // 512-point complex64 sweeps of steps take two lines per thread; explicit occupancy bounds where measured
 template <int N, int AX, typename R, int MODE, bool TR> struct FastKernel {
   static constexpr bool PACK = sizeof(R) == 4 && !TR && pack_sweep(N, MODE);
-  static constexpr int T = PACK ? PackCfg<N>::T : FastCfg<N, R>::T;
-  static constexpr size_t SMEM = PACK ? pack_smem<N, MODE>() : fast_smem_bytes<N, R>();
+  static constexpr int threads() {
+    if constexpr (PACK) return PackCfg<N>::T;
+    else return FastCfg<N, R>::T;
+  }
+  static constexpr size_t smem() {
+    if constexpr (PACK) return pack_smem<N, MODE>();
+    else return fast_smem_bytes<N, R>();
+  }
   static constexpr auto one() {
     constexpr int B = FastBounds<N, R, MODE>::value;
     if constexpr (PACK) return &k_pack<N, AX, MODE>;
@@ -43,9 +49,9 @@ template <int N, int AX, typename R, int MODE, bool TR = false>
 static cudaError_t launch_fast_one(const Phys& ph, const Sweep& sw, const FastOps& op_in, cudaStream_t st) {
   constexpr int L = FastCfg<N, R>::L;
   using FK = FastKernel<N, AX, R, MODE, TR>;
-  constexpr int T = FK::T;
+  constexpr int T = FK::threads();
   const int tiles = AX == FZ ? N * N / L : N * (N / L);
-  constexpr size_t smem = FK::SMEM;
+  constexpr size_t smem = FK::smem();
   constexpr auto kern = FK::one();
   static int attr_dev = -1, resident = 0;
   int dev = 0;
@@ -106,9 +112,9 @@ static cudaError_t launch_fastb_one(const Phys* phs, const Sweep* sws, int count
                                     cudaStream_t st) {
   constexpr int L = FastCfg<N, R>::L;
   using FK = FastKernel<N, AX, R, MODE, TR>;
-  constexpr int T = FK::T;
+  constexpr int T = FK::threads();
   const int tiles = AX == FZ ? N * N / L : N * (N / L);
-  constexpr size_t smem = FK::SMEM;
+  constexpr size_t smem = FK::smem();
   constexpr auto kern = FK::batch();
   static int attr_dev = -1, resident = 0;
   int dev = 0;

@@ -124,41 +124,9 @@ template <bool INV> struct Dft2<4, INV> {
     v[3] = INV ? p : m;
   }
 };
-template <bool INV> struct Dft2<3, INV> {
-  __device__ __forceinline__ static void run(C2* v) {
-    using k = K<float>;
-    const C2 s = v[1] + v[2], d = v[1] - v[2];
-    const C2 a = c2(fma2(s.x, f2(-0.5f), v[0].x), fma2(s.y, f2(-0.5f), v[0].y));
-    const F2 ky = kmul2(d.y, k::H3, k::H3L), kx = kmul2(d.x, k::H3, k::H3L);
-    v[0] = v[0] + s;
-    const C2 p = c2(a.x + ky, a.y - kx), m = c2(a.x - ky, a.y + kx);
-    v[1] = INV ? m : p;
-    v[2] = INV ? p : m;
-  }
-};
-template <bool INV> struct Dft2<5, INV> {
-  __device__ __forceinline__ static void run(C2* v) {
-    using k = K<float>;
-    const C2 a1 = v[1] + v[4], b1 = v[1] - v[4], a2 = v[2] + v[3], b2 = v[2] - v[3], x0 = v[0];
-    const C2 p1 = c2(x0.x + kmul2(a1.x, k::C1, k::C1L) + kmul2(a2.x, k::C2, k::C2L),
-                     x0.y + kmul2(a1.y, k::C1, k::C1L) + kmul2(a2.y, k::C2, k::C2L));
-    const C2 p2 = c2(x0.x + kmul2(a1.x, k::C2, k::C2L) + kmul2(a2.x, k::C1, k::C1L),
-                     x0.y + kmul2(a1.y, k::C2, k::C2L) + kmul2(a2.y, k::C1, k::C1L));
-    const C2 s1 = c2(kmul2(b1.x, k::S1, k::S1L) + kmul2(b2.x, k::S2, k::S2L),
-                     kmul2(b1.y, k::S1, k::S1L) + kmul2(b2.y, k::S2, k::S2L));
-    const C2 s2 = c2(kmul2(b1.x, k::S2, k::S2L) - kmul2(b2.x, k::S1, k::S1L),
-                     kmul2(b1.y, k::S2, k::S2L) - kmul2(b2.y, k::S1, k::S1L));
-    v[0] = x0 + (a1 + a2);
-    const C2 q1 = c2(p1.x + s1.y, p1.y - s1.x), q4 = c2(p1.x - s1.y, p1.y + s1.x);
-    const C2 q2 = c2(p2.x + s2.y, p2.y - s2.x), q3 = c2(p2.x - s2.y, p2.y + s2.x);
-    v[1] = INV ? q4 : q1;
-    v[4] = INV ? q1 : q4;
-    v[2] = INV ? q3 : q2;
-    v[3] = INV ? q2 : q3;
-  }
-};
-// R = R1*R2 with W_16 twiddles (8, 16) or compile-time roots (6, 10, 12)
+// R = R1*R2 in {8, 16} with W_16 twiddles
 template <int R1, int R2, bool INV> struct DftSplit2 {
+  static_assert(16 % (R1 * R2) == 0, "W_16 twiddles");
   __device__ __forceinline__ static void run(C2* v) {
     C2 y[R2][R1];
     SFor<0, R2>::run([&](auto n2c) {
@@ -167,25 +135,9 @@ template <int R1, int R2, bool INV> struct DftSplit2 {
       for (int n1 = 0; n1 < R1; ++n1) y[n2][n1] = v[R2 * n1 + n2];
       Dft2<R1, INV>::run(y[n2]);
       SFor<1, R1>::run([&](auto k1c) {
-        constexpr int k1 = decltype(k1c)::value, RR = R1 * R2;
         if constexpr (n2 != 0) {
-          if constexpr (16 % RR == 0) {
-            y[n2][k1] = mul_w16_2<(16 / RR) * ((n2 * k1) % RR), INV>(y[n2][k1]);
-          } else {
-            constexpr int e = (n2 * k1) % RR;
-            if constexpr (4 * e == RR) {
-              y[n2][k1] = mul_w16_2<4, INV>(y[n2][k1]);
-            } else if constexpr (2 * e == RR) {
-              y[n2][k1] = mul_w16_2<8, INV>(y[n2][k1]);
-            } else if constexpr (4 * e == 3 * RR) {
-              y[n2][k1] = mul_w16_2<12, INV>(y[n2][k1]);
-            } else if constexpr (e != 0) {
-              constexpr CxCS w = cx_root(e, RR);
-              constexpr float ch = (float)w.c, sh = (float)w.s;
-              constexpr float cl = (float)(w.c - (double)ch), sl = (float)(w.s - (double)sh);
-              y[n2][k1] = rot2<INV>(y[n2][k1], ch, cl, sh, sl);
-            }
-          }
+          constexpr int k1 = decltype(k1c)::value, RR = R1 * R2;
+          y[n2][k1] = mul_w16_2<(16 / RR) * ((n2 * k1) % RR), INV>(y[n2][k1]);
         }
       });
     });
@@ -202,8 +154,5 @@ template <int R1, int R2, bool INV> struct DftSplit2 {
 };
 template <bool INV> struct Dft2<8, INV>  : DftSplit2<4, 2, INV> {};
 template <bool INV> struct Dft2<16, INV> : DftSplit2<4, 4, INV> {};
-template <bool INV> struct Dft2<6, INV>  : DftSplit2<3, 2, INV> {};
-template <bool INV> struct Dft2<10, INV> : DftSplit2<5, 2, INV> {};
-template <bool INV> struct Dft2<12, INV> : DftSplit2<4, 3, INV> {};
 
 }  // namespace gpe

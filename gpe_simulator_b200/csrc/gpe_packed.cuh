@@ -1,8 +1,9 @@
 // gpe_packed.cuh -- the register-resident complex64 sweeps with two lines per thread
 // (packed FP32, gpe_pack.cuh), sm_100a.
 //
-// Same sweeps, splits, modes and operations as gpe_fast.cuh: a tile is 16 lines = 8 line pairs, a thread holds the values of one pair.  Against one line
-// per thread that halves the issue slots of the transforms' arithmetic, of the exchange
+// Same sweeps, splits, modes and operations as gpe_fast.cuh for n = 256 (16 x 16) and 512
+// (8 x 8 x 8): a tile is 16 lines = 8 line pairs, a thread holds 16 values of one pair in one
+// slot (n = 512: two).  Against one line per thread that halves the issue slots of the transforms' arithmetic, of the exchange
 // (one 16-byte access moves (re a, re b, im a, im b)) and, in y/x tiles, of the loads and
 // stores from HBM; twiddles and table values are read once for both lines.  The twiddles
 // are copied into shared memory by cp.async (through L1 they missed: with most of it taken
@@ -14,20 +15,18 @@
 namespace gpe {
 
 template <int N> struct PackCfg {
-  static constexpr int L = FastCfg<N, float>::L, LP = L / 2;
-  static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+  static_assert(N == 256 || N == 512, "sides whose twiddles d_twp holds");
   static constexpr bool THREE = N == 512;
-  static constexpr int P1 = LP * N1, P2 = THREE ? P1 : LP * N2;
-  // 16 values per line and thread from n = 128 (powers of two), one slot per phase below
-  static constexpr int T = (N == 128 || N == 256 || N == 512) ? LP * N / 16 : cdiv(P1 > P2 ? P1 : P2, 32) * 32;
-  static constexpr int Q1 = cdiv(P1, T), Q2 = cdiv(P2, T);
-  static constexpr int V = Q1 * N2 > Q2 * N1 ? Q1 * N2 : Q2 * N1;
+  static constexpr int L = FastCfg<N, float>::L, LP = L / 2;
+  static constexpr int LANES = Split<N>::N1, VALS = Split<N>::N2;   // of a pair, in every layout
+  static constexpr int V = 16;                                      // values per line and thread
+  static constexpr int T = LP * N / V, Q = LP * LANES / T;          // threads, slots
+  static_assert(Q * T == LP * LANES && Q * VALS == V, "no partial slots");
   // exchange buffer (16-byte elements)
-  static constexpr int EX = THREE ? LP * N : LP * (N + (N1 > N2 ? N1 : N2));
+  static constexpr int EX = THREE ? LP * N : LP * (N + LANES);
   static constexpr size_t EXB = (size_t)EX * 16;
-  // twiddles of the split (N1 lanes, N2 values), then of (N2, N1) when that differs (n = 512:
-  // the 64 second-phase ones)
-  static constexpr int TW = N + (THREE ? 64 : N1 == N2 ? 0 : N);
+  // twiddles of the (first) split, n = 512: then the 64 second-phase ones
+  static constexpr int TW = N + (THREE ? 64 : 0);
   // tables of a z sweep: reduction scratch, vz, c1, c2, c12; of an x sweep: kx, kyz, kx2, kyz2
   static constexpr size_t ZB = 32 * 16 + (size_t)(N + 3 * L) * 4, XB = (size_t)(N + L) * 24;
 };
@@ -46,10 +45,6 @@ template <int N, int AX> __device__ __forceinline__ void pack_slot(int gs, int p
     lane = gs / LP;
   }
 }
-template <int N, int LANES, int SLOTS> __device__ __forceinline__ bool pack_ok(int s) {
-  constexpr int LP = PackCfg<N>::LP, T = PackCfg<N>::T;
-  return !(SLOTS * T > LP * LANES) || (int)threadIdx.x + s * T < LP * LANES;
-}
 
 // 16 bytes from global to shared memory, asynchronously
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -67,48 +62,37 @@ __device__ __forceinline__ C2 ex_load(const ulonglong2* p) {
   return v;
 }
 
-// fft_2phase of gpe_fast.cuh on line pairs; tw: this split's twiddles, [k2*A + lane].
-template <int N, int A, int B, int AX, int QA, int QB, int V, bool INV, bool TAIL>
-__device__ __forceinline__ void pack_2phase(C2 (&v)[V], ulonglong2* ex, const float4* tw) {
-  constexpr int LP = PackCfg<N>::LP, T = PackCfg<N>::T;
-  static_assert(QA * B <= V && QB * A <= V, "register array too small");
-  constexpr bool WARP_LOCAL = AX == FZ && A == B && QA == 1 && QB == 1 && 32 % A == 0 && LP * A == T;
+// fft_2phase of gpe_fast.cuh on line pairs (n = 256); tw: the split's twiddles, [k2*16 + lane].
+template <int N, int AX, bool INV, bool TAIL>
+__device__ __forceinline__ void pack_2phase(C2 (&v)[PackCfg<N>::V], ulonglong2* ex, const float4* tw) {
+  constexpr int LP = PackCfg<N>::LP, A = 16;
+  static_assert(N == A * A && PackCfg<N>::Q == 1, "two-phase layout");
+  constexpr bool WARP_LOCAL = AX == FZ && LP * A == PackCfg<N>::T;
+  int lp, lane;
+  pack_slot<N, AX>(threadIdx.x, A, lp, lane);
+  Dft2<A, INV>::run(v);
 #pragma unroll
-  for (int s = 0; s < QA; ++s) {
-    if (!pack_ok<N, A, QA>(s)) break;
-    int lp, lane;
-    pack_slot<N, AX>(threadIdx.x + s * T, A, lp, lane);
-    C2* x = v + s * B;
-    Dft2<B, INV>::run(x);
+  for (int k2 = 1; k2 < A; ++k2) v[k2] = tw2<INV>(v[k2], tw[k2 * A + lane]);
 #pragma unroll
-    for (int k2 = 1; k2 < B; ++k2) x[k2] = tw2<INV>(x[k2], tw[k2 * A + lane]);
-#pragma unroll
-    for (int k2 = 0; k2 < B; ++k2)
-      ex_store(ex + (AX == FZ ? (lp * B + k2) * (A + 1) + lane : (k2 * A + lane) * LP + lp), x[k2]);
-  }
+  for (int k2 = 0; k2 < A; ++k2)
+    ex_store(ex + (AX == FZ ? (lp * A + k2) * (A + 1) + lane : (k2 * A + lane) * LP + lp), v[k2]);
   if (WARP_LOCAL) __syncwarp(); else __syncthreads();
+  // (the slot's lane is the second phase's k2)
 #pragma unroll
-  for (int s = 0; s < QB; ++s) {
-    if (!pack_ok<N, B, QB>(s)) break;
-    int lp, k2;
-    pack_slot<N, AX>(threadIdx.x + s * T, B, lp, k2);
-    C2* x = v + s * A;
-#pragma unroll
-    for (int n1 = 0; n1 < A; ++n1)
-      x[n1] = ex_load(ex + (AX == FZ ? (lp * B + k2) * (A + 1) + n1 : (k2 * A + n1) * LP + lp));
-    Dft2<A, INV>::run(x);
-  }
+  for (int n1 = 0; n1 < A; ++n1)
+    v[n1] = ex_load(ex + (AX == FZ ? (lp * A + lane) * (A + 1) + n1 : (lane * A + n1) * LP + lp));
+  Dft2<A, INV>::run(v);
   if (TAIL) {
     if (WARP_LOCAL) __syncwarp(); else __syncthreads();
   }
 }
 
 // fft_3phase of gpe_fast.cuh on line pairs (n = 512).
-template <int N, int AX, int Q, int V, bool INV, bool TAIL>
-__device__ __forceinline__ void pack_3phase(C2 (&v)[V], ulonglong2* ex, const float4* twa, const float4* twb) {
-  constexpr int LP = PackCfg<N>::LP, T = PackCfg<N>::T;
+template <int N, int AX, bool INV, bool TAIL>
+__device__ __forceinline__ void pack_3phase(C2 (&v)[PackCfg<N>::V], ulonglong2* ex, const float4* twa, const float4* twb) {
+  constexpr int LP = PackCfg<N>::LP, T = PackCfg<N>::T, Q = PackCfg<N>::Q;
   constexpr int RD = 8, A = 64;
-  static_assert(N == RD * RD * RD && Q * RD <= V && Q * T == LP * A, "three-phase layout");
+  static_assert(N == RD * RD * RD, "three-phase layout");
   constexpr bool WARP_LOCAL = AX == FZ && T == 32 * LP;
   auto e1 = [](int lp, int k3, int p) { return AX == FZ ? (lp * RD + k3) * A + p : (k3 * A + p) * LP + lp; };
   auto e2 = [](int lp, int k3, int k1, int p1) {
@@ -197,15 +181,14 @@ __device__ __forceinline__ float2 half_one(float2 x, float V, float g, float bet
 
 // half_all of gpe_fast.cuh on pairs: layout LANES x VALS, element m = lane + LANES*a of
 // lines 2 lp, 2 lp + 1.
-template <int N, int LANES, int VALS, int SLOTS, int V_, bool REAL, bool ARR, bool TWO>
-__device__ __forceinline__ void pack_half(C2 (&v)[V_], const FastTile<N, FZ, float>& tl, const Phys& ph,
+template <int N, bool REAL, bool ARR, bool TWO>
+__device__ __forceinline__ void pack_half(C2 (&v)[PackCfg<N>::V], const FastTile<N, FZ, float>& tl, const Phys& ph,
                                           const FastTables<float>& tb, const float* ctab, float beta, float h) {
-  constexpr int T = PackCfg<N>::T;
+  constexpr int T = PackCfg<N>::T, LANES = PackCfg<N>::LANES, VALS = PackCfg<N>::VALS, SLOTS = PackCfg<N>::Q;
   static_assert(SLOTS * VALS <= 32, "pending mask");
   unsigned pend = 0;
 #pragma unroll
   for (int s = 0; s < SLOTS; ++s) {
-    if (!pack_ok<N, LANES, SLOTS>(s)) break;
     int lp, lane;
     pack_slot<N, FZ>(threadIdx.x + s * T, LANES, lp, lane);
     const float2 c = *(const float2*)(ctab + 2 * lp);
@@ -257,46 +240,46 @@ __device__ __forceinline__ void pack_half(C2 (&v)[V_], const FastTile<N, FZ, flo
     }
     }
   }
-  if (ARR || !__any_sync(0xffffffffu, pend != 0)) return;
+  if constexpr (!ARR) {
+    if (!__any_sync(0xffffffffu, pend != 0)) return;
 #pragma unroll
-  for (int s = 0; s < SLOTS; ++s) {
-    if (!pack_ok<N, LANES, SLOTS>(s)) break;
-    int lp, lane;
-    pack_slot<N, FZ>(threadIdx.x + s * T, LANES, lp, lane);
-    const float2 c = *(const float2*)(ctab + 2 * lp);
+    for (int s = 0; s < SLOTS; ++s) {
+      int lp, lane;
+      pack_slot<N, FZ>(threadIdx.x + s * T, LANES, lp, lane);
+      const float2 c = *(const float2*)(ctab + 2 * lp);
 #pragma unroll
-    for (int a = 0; a < VALS; ++a) {
-      const int e = s * VALS + a;
-      if (!((pend >> e) & 1)) continue;
-      const float2 x = unpack(v[e].x), y = unpack(v[e].y);
-      const float vz = tb.vz[lane + LANES * a];
-      const float2 r0 = half_one<REAL, false, TWO>(make_float2(x.x, y.x), vz + c.x, 0.0f, beta, h);
-      const float2 r1 = half_one<REAL, false, TWO>(make_float2(x.y, y.y), vz + c.y, 0.0f, beta, h);
-      v[e] = c2(f2(r0.x, r1.x), f2(r0.y, r1.y));
+      for (int a = 0; a < VALS; ++a) {
+        const int e = s * VALS + a;
+        if (!((pend >> e) & 1)) continue;
+        const float2 x = unpack(v[e].x), y = unpack(v[e].y);
+        const float vz = tb.vz[lane + LANES * a];
+        const float2 r0 = half_one<REAL, false, TWO>(make_float2(x.x, y.x), vz + c.x, 0.0f, beta, h);
+        const float2 r1 = half_one<REAL, false, TWO>(make_float2(x.y, y.y), vz + c.y, 0.0f, beta, h);
+        v[e] = c2(f2(r0.x, r1.x), f2(r0.y, r1.y));
+      }
     }
   }
 }
 
-template <int N, int LANES, int VALS, int SLOTS, int V_>
-__device__ __forceinline__ void pack_half_dispatch(C2 (&v)[V_], const FastTile<N, FZ, float>& tl, const Phys& ph,
+template <int N>
+__device__ __forceinline__ void pack_half_dispatch(C2 (&v)[PackCfg<N>::V], const FastTile<N, FZ, float>& tl, const Phys& ph,
                                                    const FastTables<float>& tb) {
   const float beta = (float)ph.beta, h = (float)(ph.dt * 0.5);
   const bool arr = ph.vre != nullptr || ph.vim != nullptr;
   if (ph.kind == 1) {
-    if (arr) pack_half<N, LANES, VALS, SLOTS, V_, true, true, false>(v, tl, ph, tb, tb.c1, beta, h);
-    else pack_half<N, LANES, VALS, SLOTS, V_, true, false, false>(v, tl, ph, tb, tb.c1, beta, h);
+    if (arr) pack_half<N, true, true, false>(v, tl, ph, tb, tb.c1, beta, h);
+    else pack_half<N, true, false, false>(v, tl, ph, tb, tb.c1, beta, h);
   } else {
-    if (arr) pack_half<N, LANES, VALS, SLOTS, V_, false, true, false>(v, tl, ph, tb, tb.c1, beta, h);
-    else pack_half<N, LANES, VALS, SLOTS, V_, false, false, false>(v, tl, ph, tb, tb.c1, beta, h);
+    if (arr) pack_half<N, false, true, false>(v, tl, ph, tb, tb.c1, beta, h);
+    else pack_half<N, false, false, false>(v, tl, ph, tb, tb.c1, beta, h);
   }
 }
 
-template <int N, int LANES, int VALS, int SLOTS, int V_, bool REAL, bool CUT>
-__device__ __forceinline__ void pack_kin(C2 (&v)[V_], const Phys& ph, const FastTables<float>& tb) {
-  constexpr int T = PackCfg<N>::T;
+template <int N, bool REAL, bool CUT>
+__device__ __forceinline__ void pack_kin(C2 (&v)[PackCfg<N>::V], const Phys& ph, const FastTables<float>& tb) {
+  constexpr int T = PackCfg<N>::T, LANES = PackCfg<N>::LANES, VALS = PackCfg<N>::VALS, SLOTS = PackCfg<N>::Q;
 #pragma unroll
   for (int s = 0; s < SLOTS; ++s) {
-    if (!pack_ok<N, LANES, SLOTS>(s)) break;
     int lp, lane;
     pack_slot<N, FX>(threadIdx.x + s * T, LANES, lp, lane);
 #pragma unroll
@@ -312,13 +295,12 @@ __device__ __forceinline__ void pack_kin(C2 (&v)[V_], const Phys& ph, const Fast
 
 // ---------------------------------------------------------------- loads and stores
 // (past L1, which holds the twiddles) vec: y/x rows by 16-byte accesses (psi aligned to 16 bytes), else one line at a time
-template <int N, int AX, int LANES, int VALS, int SLOTS, int V_>
-__device__ __forceinline__ void pack_load(C2 (&v)[V_], const FastTile<N, AX, float>& tl,
+template <int N, int AX>
+__device__ __forceinline__ void pack_load(C2 (&v)[PackCfg<N>::V], const FastTile<N, AX, float>& tl,
                                           const float2* __restrict__ src, bool vec) {
-  constexpr int T = PackCfg<N>::T;
+  constexpr int T = PackCfg<N>::T, LANES = PackCfg<N>::LANES, VALS = PackCfg<N>::VALS, SLOTS = PackCfg<N>::Q;
 #pragma unroll
   for (int s = 0; s < SLOTS; ++s) {
-    if (!pack_ok<N, LANES, SLOTS>(s)) break;
     int lp, lane;
     pack_slot<N, AX>(threadIdx.x + s * T, LANES, lp, lane);
     const float2* p = src + tl.gidx(2 * lp, lane);
@@ -339,13 +321,12 @@ __device__ __forceinline__ void pack_load(C2 (&v)[V_], const FastTile<N, AX, flo
   }
 }
 
-template <int N, int AX, int LANES, int VALS, int SLOTS, int V_>
-__device__ __forceinline__ void pack_store(const C2 (&v)[V_], const FastTile<N, AX, float>& tl,
+template <int N, int AX>
+__device__ __forceinline__ void pack_store(const C2 (&v)[PackCfg<N>::V], const FastTile<N, AX, float>& tl,
                                            float2* __restrict__ dst, bool vec) {
-  constexpr int T = PackCfg<N>::T;
+  constexpr int T = PackCfg<N>::T, LANES = PackCfg<N>::LANES, VALS = PackCfg<N>::VALS, SLOTS = PackCfg<N>::Q;
 #pragma unroll
   for (int s = 0; s < SLOTS; ++s) {
-    if (!pack_ok<N, LANES, SLOTS>(s)) break;
     int lp, lane;
     pack_slot<N, AX>(threadIdx.x + s * T, LANES, lp, lane);
     float2* p = dst + tl.gidx(2 * lp, lane);
@@ -367,11 +348,8 @@ __device__ __forceinline__ void pack_store(const C2 (&v)[V_], const FastTile<N, 
 template <int N, int AX, int MODE>
 __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const FastOps& op, int tile, int ntiles) {
   constexpr int L = PackCfg<N>::L;
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  constexpr int V_ = PackCfg<N>::V, S1 = PackCfg<N>::Q1, S2 = PackCfg<N>::Q2;
   constexpr bool ZM = MODE == FM_Z1 || MODE == FM_Z2 || MODE == FM_Z21;
   constexpr bool THREE = PackCfg<N>::THREE;
-  constexpr int LM = THREE ? N1 : N2, VM = THREE ? N2 : N1, SM = THREE ? S1 : S2;
   constexpr bool TWO_FFT = MODE == FM_Z21 || MODE == FM_XKIN;
   griddep_launch_dependents();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -388,8 +366,6 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
   tb.c1 = tb.vz + N;
   tb.c2 = tb.c1 + L;
   tb.c12 = tb.c2 + L;
-  const float4* t1 = tw;
-  const float4* t2 = N1 == N2 ? t1 : t1 + N;
   // (plan constants: copied past the registers, in flight with the tile's loads)
   for (int q = threadIdx.x; q < PackCfg<N>::TW; q += PackCfg<N>::T) cp_async16(tw + q, (const float4*)sw.twp + q);
   const FastTile<N, AX, float> tl(tile);
@@ -397,27 +373,28 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
   float sc_mul = 1.0f;
   if (MODE == FM_Z1 && op.scale) sc_mul = (float)__ldcg(sw.scale + 1);
   const bool vec = op.vec != 0;
-  C2 v[V_];
-  pack_load<N, AX, N1, N2, S1>(v, tl, (const float2*)sw.src, vec);
+  constexpr int V = PackCfg<N>::V;
+  C2 v[V];
+  pack_load<N, AX>(v, tl, (const float2*)sw.src, vec);
   if (op.pf > 0) {
     const int next = op.rev ? tile - op.pf : tile + op.pf;
     if (next >= 0 && next < ntiles) fast_prefetch_l2<N, AX, float, PackCfg<N>::T>(FastTile<N, AX, float>(next), sw.src);
   }
-  if (ZM) z_tables<N, float, PackCfg<N>::T>(ph, sw, tl.a0, tb, MODE == FM_Z21, MODE == FM_Z21);
+  if (ZM) z_tables<N, float, PackCfg<N>::T>(ph, sw, tl.a0, tb, MODE == FM_Z21);
   if (MODE == FM_XKIN) x_tables<N, float, PackCfg<N>::T>(ph, tl.a0, tl.b0, tb);
   cp_async_wait();
   __syncthreads();   // twiddles and tables visible
   if constexpr (MODE == FM_Z1) {
     if (op.scale) {
 #pragma unroll
-      for (int e = 0; e < V_; ++e) v[e] = c2(v[e].x * f2(sc_mul), v[e].y * f2(sc_mul));
+      for (int e = 0; e < V; ++e) v[e] = c2(v[e].x * f2(sc_mul), v[e].y * f2(sc_mul));
     }
-    pack_half_dispatch<N, N1, N2, S1>(v, tl, ph, tb);
+    pack_half_dispatch<N>(v, tl, ph, tb);
   }
   auto first = [&](auto inv) {
     constexpr bool INV = decltype(inv)::value;
-    if constexpr (THREE) pack_3phase<N, AX, S1, V_, INV, TWO_FFT>(v, ex, t1, t2);
-    else pack_2phase<N, N1, N2, AX, S1, S2, V_, INV, TWO_FFT>(v, ex, t1);
+    if constexpr (THREE) pack_3phase<N, AX, INV, TWO_FFT>(v, ex, tw, tw + N);
+    else pack_2phase<N, AX, INV, TWO_FFT>(v, ex, tw);
   };
   using std::integral_constant;
   if constexpr (MODE == FM_Z2 || MODE == FM_Z21) {
@@ -432,36 +409,30 @@ __device__ __forceinline__ void pack_body(const Phys& ph, const Sweep& sw, const
     if constexpr (MODE == FM_Z21) {
       const float h = (float)(ph.dt * 0.5), b2 = (float)(2.0 * ph.beta) * h;
       if (ph.vre == nullptr && ph.vim == nullptr)
-        pack_half<N, LM, VM, SM, V_, true, false, true>(v, tl, ph, tb, tb.c12, b2, h);
+        pack_half<N, true, false, true>(v, tl, ph, tb, tb.c12, b2, h);
       else
-        pack_half<N, LM, VM, SM, V_, true, true, true>(v, tl, ph, tb, tb.c12, b2, h);
+        pack_half<N, true, true, true>(v, tl, ph, tb, tb.c12, b2, h);
     } else if (ph.kind == 1) {
-      if (ph.kcut) pack_kin<N, LM, VM, SM, V_, true, true>(v, ph, tb);
-      else pack_kin<N, LM, VM, SM, V_, true, false>(v, ph, tb);
+      if (ph.kcut) pack_kin<N, true, true>(v, ph, tb);
+      else pack_kin<N, true, false>(v, ph, tb);
     } else {
-      pack_kin<N, LM, VM, SM, V_, false, false>(v, ph, tb);
+      pack_kin<N, false, false>(v, ph, tb);
     }
     constexpr bool INV = MODE == FM_XKIN;
-    if constexpr (THREE) pack_3phase<N, AX, S1, V_, INV, false>(v, ex, t1, t2);
-    else pack_2phase<N, N2, N1, AX, S2, S1, V_, INV, false>(v, ex, t2);
-    pack_store<N, AX, N1, N2, S1>(v, tl, (float2*)sw.dst, vec);
+    if constexpr (THREE) pack_3phase<N, AX, INV, false>(v, ex, tw, tw + N);
+    else pack_2phase<N, AX, INV, false>(v, ex, tw);
+    pack_store<N, AX>(v, tl, (float2*)sw.dst, vec);
   } else {
-    if constexpr (MODE == FM_Z2) pack_half_dispatch<N, LM, VM, SM>(v, tl, ph, tb);
-    if (MODE == FM_PLAIN && op.invm) {
-      const F2 f = f2((float)ph.inv_m);
-#pragma unroll
-      for (int e = 0; e < V_; ++e) v[e] = c2(v[e].x * f, v[e].y * f);
-    }
-    pack_store<N, AX, LM, VM, SM>(v, tl, (float2*)sw.dst, vec);
+    if constexpr (MODE == FM_Z2) pack_half_dispatch<N>(v, tl, ph, tb);
+    pack_store<N, AX>(v, tl, (float2*)sw.dst, vec);
     if (MODE == FM_Z2 && op.norm) {
       // a thread's values of a line summed in plain FP64 (fixed order), then compensated
       Acc a[1];
 #pragma unroll
-      for (int s = 0; s < SM; ++s) {
-        if (!pack_ok<N, LM, SM>(s)) break;
+      for (int s = 0; s < PackCfg<N>::Q; ++s) {
         double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-        for (int e = s * VM; e < (s + 1) * VM; ++e) {
+        for (int e = s * PackCfg<N>::VALS; e < (s + 1) * PackCfg<N>::VALS; ++e) {
           const float2 x = unpack(v[e].x), y = unpack(v[e].y);
           s0 = fma((double)x.x, (double)x.x, fma((double)y.x, (double)y.x, s0));
           s1 = fma((double)x.y, (double)x.y, fma((double)y.y, (double)y.y, s1));

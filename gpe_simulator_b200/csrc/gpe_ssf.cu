@@ -359,17 +359,6 @@ __global__ void k_build_static(int n, const double* x, const double* prog, int l
 
 // Sum per-block diagnostic partials in a fixed order: out[0..3] = sums of pa
 // columns 0..2 and pb column 3 (the shell bins out[4 + b] come from k_finish_hist).
-// Angular momentum: the sums of the x and y sweeps' partials (column 3) into out[0], out[1].
-__global__ void k_finish_lz(const double* px, int nx, const double* py, int ny, double* out) {
-  __shared__ Acc sh[32 * 2];
-  Acc a[2];
-  for (int b = threadIdx.x; b < nx; b += blockDim.x) a[0].add(px[(long long)b * 4 + 3]);
-  for (int b = threadIdx.x; b < ny; b += blockDim.x) a[1].add(py[(long long)b * 4 + 3]);
-  block_merge<2>(a, sh);
-  if (threadIdx.x == 0)
-    for (int v = 0; v < 2; ++v) out[v] = a[v].value();
-}
-
 __global__ void k_finish_diag(const double* pa, int na, const double* pb, int nb, double* out) {
   __shared__ Acc sh[32 * 4];
   Acc a[4];
@@ -382,6 +371,17 @@ __global__ void k_finish_diag(const double* pa, int na, const double* pb, int nb
   block_merge<4>(a, sh);
   if (threadIdx.x == 0)
     for (int v = 0; v < 4; ++v) out[v] = a[v].value();
+}
+
+// Angular momentum: the sums of the x and y sweeps' partials (column 3) into out[0], out[1].
+__global__ void k_finish_lz(const double* px, int nx, const double* py, int ny, double* out) {
+  __shared__ Acc sh[32 * 2];
+  Acc a[2];
+  for (int b = threadIdx.x; b < nx; b += blockDim.x) a[0].add(px[(long long)b * 4 + 3]);
+  for (int b = threadIdx.x; b < ny; b += blockDim.x) a[1].add(py[(long long)b * 4 + 3]);
+  block_merge<2>(a, sh);
+  if (threadIdx.x == 0)
+    for (int v = 0; v < 2; ++v) out[v] = a[v].value();
 }
 
 // k-space sums of a spectrum passed in by the caller (no transform): sum k^2 |f|^2
