@@ -1342,19 +1342,24 @@ int ensure_hist(gpe_plan* p) {
 
 // The least double kk >= 0 of every shell b, floor(sqrt(kk)/w + 0.5) >= b: the expression never
 // decreases with kk (each of its operations rounds monotonically), so the boundary is found
-// by bisection over the doubles, which order as their bits.
+// by bisection over the doubles, which order as their bits, from a few hundred of them
+// around ((b - 1/2) w)^2 (the whole range between two shells took 2.8 ms for 5000 bins).
 std::vector<double> shell_starts(double w, int nbins) {
   std::vector<double> t(nbins, 0.0);
   for (int b = 1; b < nbins; ++b) {
-    double lo_d = t[b - 1], hi_d = (b + 1.0) * w * ((b + 1.0) * w) * 2.0;
-    long long lo, hi;   // the shell of lo is below b (or lo = 0), that of hi is not
+    auto in = [&](double x) { return std::floor(std::sqrt(x) / w + 0.5) >= b; };
+    const double at = (b - 0.5) * w * ((b - 0.5) * w);
+    double lo_d = std::max(t[b - 1], at * (1.0 - 1e-13)), hi_d = at * (1.0 + 1e-13);
+    if (in(lo_d)) lo_d = t[b - 1];
+    if (!in(hi_d)) hi_d = (b + 1.0) * w * ((b + 1.0) * w) * 2.0;
+    long long lo, hi;   // the shell of lo is below b (or lo is the last shell's start), that of hi is not
     memcpy(&lo, &lo_d, 8);
     memcpy(&hi, &hi_d, 8);
     while (lo < hi) {
       const long long mid = lo + (hi - lo) / 2;
       double x;
       memcpy(&x, &mid, 8);
-      if (std::floor(std::sqrt(x) / w + 0.5) >= b) hi = mid;
+      if (in(x)) hi = mid;
       else lo = mid + 1;
     }
     memcpy(&t[b], &hi, 8);
