@@ -181,7 +181,8 @@ __device__ __forceinline__ void slot(int gs, int per, int& l, int& lane) {
 // One forward FFT of every line of the tile, A = lanes in phase 1 (values A-strided),
 // B = values per lane in phase 1.  In: v[s][b] = x[lane_s + A*b] of line l_s (phase-1
 // slots).  Out: v[s][a] = X[lane_s + B*a] (phase-2 slots with B lanes per line).
-template <int N, int A, int B, int AX, typename R, int QA, int QB, int V, bool ASYNC_NEXT = false, bool TAIL = true>
+template <int N, int A, int B, int AX, typename R, int QA, int QB, int V, bool ASYNC_NEXT = false, bool TAIL = true,
+          bool NAMED = false>
 __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename Cx<R>::T* ex,
                                            const typename TwE<R>::T* tw) {
   // In: QA slots of (A lanes, B values), slot s holding x[lane + A*b] in v[s*B + b].
@@ -196,8 +197,8 @@ __device__ __forceinline__ void fft_2phase(typename Cx<R>::T (&v)[V], typename C
   constexpr int L = FastCfg<N, R>::L;
   constexpr int T = FastCfg<N, R>::T;
   static_assert(QA * B <= V && QB * A <= V, "register array too small");
-  // (the arithmetic of the packed sweeps, gpe_packed.cuh)
-  constexpr bool NAMED = N == 256 && sizeof(R) == 4;
+  // NAMED: the arithmetic of the packed sweeps, gpe_packed.cuh (16 x 16 points).
+  static_assert(!NAMED || (A == 16 && B == 16 && sizeof(R) == 4), "packed arithmetic");
   using DftA = typename std::conditional<NAMED, DftSplit<4, 4, true>, Dft<A>>::type;
   using DftB = typename std::conditional<NAMED, DftSplit<4, 4, true>, Dft<B>>::type;
   // Z tiles with A == B lanes per line in both phases and one slot per thread:
@@ -385,7 +386,7 @@ __device__ __forceinline__ float expm1_series(float x) {
 }
 
 // complex128: the same factors in FP64, as f - 1 applied by v + v*(f - 1).  Taylor
-// series on |x| <= 1/2: sin to x^15 (first omitted term x^17/17! < 3e-20 of x), cos - 1
+// series on |x| <= 1/2: sin to x^15 (first omitted term x^17/17! < 5e-20 of x), cos - 1
 // to x^16 (x^18/18! < 7e-22), exp - 1 to x^15 (x^16/16! < 8e-19); library functions,
 // out of line, beyond.  Steps in use keep V dt/2 far inside the range; with the library
 // sincos and exp inlined per half-step, and two of them per fused z sweep, that sweep was
@@ -692,7 +693,7 @@ __device__ __forceinline__ void local_block(typename Cx<R>::T* v, const R (&V)[U
   }
 }
 
-// elements per local_block: the largest of 5, 4, 3, 2 that divides n (1: none does)
+// elements per local_block: 4 where that divides n, else 5, 3 or 2 (1: none does)
 constexpr int local_unroll(int n) { return n % 4 == 0 ? 4 : n % 5 == 0 ? 5 : n % 3 == 0 ? 3 : n % 2 == 0 ? 2 : 1; }
 
 // Phase of an element's half-step (TWO: of both), and exp(-i phase) - 1 times 1 + am; NAMED as in
@@ -765,7 +766,8 @@ __device__ __forceinline__ void half_all(typename Cx<R>::T (&v)[EPT], const Fast
     }
     return;
   }
-  constexpr bool NAMED = N == 256;
+  // (the fused z sweep at 256 is packed; here it is a stage of the plane-fused launches)
+  constexpr bool NAMED = N == 256 && TWO;
   static_assert(SLOTS * VALS <= 64, "pending mask");
   // complex64: elements whose phase exceeds the short series' range
   using Mask = typename std::conditional<(SLOTS * VALS <= 32), unsigned, unsigned long long>::type;
@@ -1142,14 +1144,15 @@ __device__ __forceinline__ void fast_body(const Phys& ph, const Sweep& sw, const
   if (MODE == FM_DIAGR) diag_real_all<N, AX, R, N1, N2, S1>(v, tl, ph, tb, cx);
   // the first transform frees the exchange buffer only when a second one follows
   constexpr bool TWO_FFT = MODE == FM_Z21 || MODE == FM_XKIN;
+  constexpr bool NAMED = N == 256 && sizeof(R) == 4 && MODE == FM_Z21;
   static_assert(!(THREE && TWO_FFT), "the fused 512-point sweeps are packed");
   if constexpr (THREE) fft_3phase<N, AX, R, S1, EPT>(v, ex, t1, t2);
-  else fft_2phase<N, N1, N2, AX, R, S1, S2, EPT, false, TWO_FFT>(v, ex, t1);
+  else fft_2phase<N, N1, N2, AX, R, S1, S2, EPT, false, TWO_FFT, NAMED>(v, ex, t1);
   if constexpr (TWO_FFT) {
     if (MODE == FM_Z21) conj_all(v);  // finish the inverse before the physics
     fast_pointwise<N, AX, R, MODE, 1, LM, VM, SM>(v, tl, ph, tb, op, cx);
     if (MODE == FM_XKIN) conj_all(v);  // start the inverse
-    fft_2phase<N, N2, N1, AX, R, S2, S1, EPT, false, false>(v, ex, t2);
+    fft_2phase<N, N2, N1, AX, R, S2, S1, EPT, false, false, NAMED>(v, ex, t2);
     if (MODE == FM_XKIN) conj_all(v);
     fast_store<N, AX, R, N1, N2, S1>(v, tl, (C*)sw.dst);
   } else {

@@ -103,7 +103,7 @@ __device__ __forceinline__ double2 tw_apply(double2 v, double2 w) { return cmul(
 // The complex64 products above with every fused operation named.  Which of two products of a
 // sum the compiler fuses differs between kernels, for the low parts once in some 1e10
 // operations visibly; kernels that promise each other the same bits although one packs
-// two lines and one does not (n = 256) use these.
+// two lines and one does not (the fused z sweep at n = 256) use these.
 __device__ __forceinline__ float2 rot_named(float2 v, float ch, float cl, float sh, float sl) {
   return make_float2(fmaf(v.x, ch, fmaf(v.y, sh, fmaf(v.x, cl, __fmul_rn(v.y, sl)))),
                      fmaf(v.y, ch, fmaf(-v.x, sh, fmaf(v.y, cl, __fmul_rn(-v.x, sl)))));

@@ -49,9 +49,11 @@ def first_two(*axes):
 
 def utility_plan(psi, x_array, k_array=None, nbins=0, pairs=None):
     """Plan without physics, for FFTs and reductions on ``psi``'s grid (``nbins``:
-    0 = the reference's shell binning, else that many uniform bins).  Plans are
-    cached by the grid's values, so repeated diagnostics on one grid create no new
-    device tables.  ``pairs``: ``first_two(x_array[, k_array])`` if already read."""
+    0 = the reference's shell binning, else that many uniform bins).  The axes are a
+    uniform grid and its ``2 pi fftfreq`` (``get_grids``): plans are cached by their
+    first two values, read at every call, so repeated diagnostics on one grid create
+    no new device tables; what else an axis holds is read when the plan is made.
+    ``pairs``: ``first_two(x_array[, k_array])`` if already read."""
     n = psi.shape[0]
     if pairs is None:
         pairs = first_two(x_array) if k_array is None else first_two(x_array, k_array)
