@@ -6,8 +6,10 @@
  * (a cudaStream_t; NULL = legacy default stream).  Every entry point returns a
  * status code (GPE_OK = 0); gpe_last_error() gives the message of the last
  * failure on the calling host thread.  A plan is not thread-safe: use one plan
- * per host thread.  All launch functions are asynchronous on `stream` unless
- * stated otherwise.
+ * per host thread.  Calls that reduce, renormalise or run path 3 use the plan's
+ * scratch: order them across streams.  Other real-time steps share nothing but the
+ * tables of a dynamic potential, on which calls wait for each other.  All launch
+ * functions are asynchronous on `stream` unless stated otherwise.
  *
  * Arrays are cubes `[x][y][z]` in C order (z fastest), complex64
  * (interleaved float re,im) or complex128 (interleaved double re,im), as in the
@@ -105,7 +107,8 @@ typedef struct gpe_desc {
     const double* static_g;  int static_g_len;
     /* time-dependent potential V(x,y,z,t) (real time only), optional */
     const double* dynamic_g; int dynamic_g_len;
-    /* momentum cutoff (real time only) */
+    /* momentum cutoff (real time only): drops modes with k^2 > k_cut^2 (those of exactly
+     * that length stay or go by the rounding of k^2, which differs between sweep paths) */
     int k_cut_enabled;        double k_cut;
     /* built-in rotating Gaussian stirring beam (real time only):
      * amp*exp(-((x-r cos th)^2+(y-r sin th)^2)/w^2),
